@@ -293,24 +293,116 @@ __global__ void __launch_bounds__(kThreads) k_diag(cplx_t<T>* __restrict__ psi, 
   }
 }
 
+// Swapping physical bit pairs in place: amplitude j moves to pi(j), pi an
+// involution on index bits. What bounds it is HBM (every amplitude that
+// moves is read and written once, as long as both accesses are coalesced):
+// a swap of a low bit with a high one scatters single amplitudes, 8 bytes
+// of a 32-byte sector. So a block moves whole tiles: the tile's bits are the
+// low `m` bits, their images under pi, and more bits up to kSwapTileBits,
+// closed under pi. Then pi maps tile t to the tile t' whose index bits are
+// swapped and element e of it to image(e), and a block reads both tiles of a
+// pair as rows of 2^m contiguous amplitudes (256 bytes), and writes each
+// from the other's copy in shared memory, in rows again. Tiles that pi
+// leaves as they are (t = t', image the identity) are not touched. The next
+// pair's loads fly while the present one is written.
+// Element e lies at e with its row bits folded into its low bits: row bit i
+// is the image of low bit i where that leaves the row, so lanes that step
+// over low bits hit distinct banks both when they write rows (low bits
+// vary) and when they read mapped elements (row bits vary). All three maps
+// of e are linear in its bits, so a thread's elements are its first one's
+// plus constants.
+// Tiles of 16 KB: with 8 KB ones a complex64 pass ran at 0.51-0.54 of the
+// copy rate (complex128, 16 KB, at 0.76-0.83).
+constexpr int kSwapTileBits = 11;  // most (complex64); 10 for complex128
+constexpr int kSwapElems = (1 << kSwapTileBits) / kThreads;
+
 struct SwapGeom {
-  uint64_t mask;  // every swapped bit
-  int32_t np;
-  uint8_t a[32], b[32];
+  uint64_t tiles;                 // 2^(n - k)
+  int32_t k, m;                   // tile bits, low bits of a row
+  int32_t np;                     // swapped pairs of tile-index bits
+  int32_t moves;                  // image is not the identity
+  uint8_t a[32], b[32];           // those pairs
+  uint8_t fixed[kSwapTileBits];   // the tile's physical bits, ascending
+  uint8_t bit[kSwapTileBits];     // physical bit of element bit i (the low m ones are 0..m-1)
+  uint8_t image[kSwapTileBits];   // element bit that element bit i moves to
+  // Element i * kThreads: its offset in the state, its place in shared
+  // memory and the place of its image.
+  uint64_t off[kSwapElems];
+  uint16_t pos[kSwapElems], from[kSwapElems];
 };
 
+__host__ __device__ __forceinline__ uint32_t swap_pos(uint32_t e, int m) {
+  return e ^ ((e >> m) & ((1u << m) - 1u));
+}
+
 template <typename T>
-__global__ void k_swap_bits(cplx_t<T>* __restrict__ psi, uint64_t len, const SwapGeom g) {
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < len; i += stride) {
-    uint64_t j = i & ~g.mask;
-    for (int p = 0; p < g.np; ++p)
-      j |= (((i >> g.a[p]) & 1) << g.b[p]) | (((i >> g.b[p]) & 1) << g.a[p]);
-    if (i < j) {
-      const cplx_t<T> t = psi[i];
-      psi[i] = psi[j];
-      psi[j] = t;
+__global__ void __launch_bounds__(kThreads) k_swap_bits(cplx_t<T>* __restrict__ psi,
+                                                        const __grid_constant__ SwapGeom g) {
+  constexpr int E = sizeof(T) == 4 ? kSwapElems : kSwapElems / 2;  // elements of a tile per thread
+  __shared__ cplx_t<T> buf[2][E * kThreads];
+  __shared__ uint8_t fixed[kSwapTileBits];
+  if (threadIdx.x < kSwapTileBits) fixed[threadIdx.x] = g.fixed[threadIdx.x];
+  __syncthreads();
+  uint64_t off = 0;
+  uint32_t x0 = 0;
+  for (int j = 0; j < g.k; ++j) {
+    off |= uint64_t((threadIdx.x >> j) & 1u) << g.bit[j];
+    x0 |= ((threadIdx.x >> j) & 1u) << g.image[j];
+  }
+  const uint32_t pos = swap_pos(threadIdx.x, g.m), from = swap_pos(x0, g.m);
+  auto live = [&](int i) { return threadIdx.x + uint32_t(i) * kThreads < (1u << g.k); };
+  auto partner = [&](uint64_t t) {
+    uint64_t t2 = t;
+    for (int p = 0; p < g.np; ++p) {
+      const uint64_t d = ((t >> g.a[p]) ^ (t >> g.b[p])) & 1u;
+      t2 ^= (d << g.a[p]) | (d << g.b[p]);
     }
+    return t2;
+  };
+  // The block's next tile from t on that moves, with its partner.
+  auto next = [&](uint64_t& t, uint64_t& t2) {
+    for (; t < g.tiles; t += gridDim.x) {
+      t2 = partner(t);
+      if (t2 > t || (t2 == t && g.moves)) return true;
+    }
+    return false;
+  };
+  cplx_t<T> x[E], y[E];
+  cplx_t<T>*p1 = psi, *p2 = psi;  // this thread's first element of the two tiles
+  auto load = [&](uint64_t t, uint64_t t2) {
+    p1 = psi + (insert_zeros(t, fixed, g.k) + off);
+    p2 = psi + (insert_zeros(t2, fixed, g.k) + off);
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (live(i)) x[i] = p1[g.off[i]];
+    if (t2 != t)
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+        if (live(i)) y[i] = p2[g.off[i]];
+  };
+  uint64_t t = blockIdx.x, t2 = 0;
+  bool more = next(t, t2);
+  if (more) load(t, t2);
+  while (more) {
+    cplx_t<T>*w1 = p1, *w2 = p2;
+    const bool two = w2 != w1;
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (live(i)) {
+        buf[0][pos ^ g.pos[i]] = x[i];
+        if (two) buf[1][pos ^ g.pos[i]] = y[i];
+      }
+    __syncthreads();
+    t += gridDim.x;
+    more = next(t, t2);
+    if (more) load(t, t2);
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (live(i)) {
+        w1[g.off[i]] = buf[two ? 1 : 0][from ^ g.from[i]];
+        if (two) w2[g.off[i]] = buf[0][from ^ g.from[i]];
+      }
+    __syncthreads();
   }
 }
 
@@ -577,17 +669,90 @@ void launch_plain_gate(StateImpl& s, const PlainGate& g, const void* matrices) {
 
 void launch_swap_bits(StateImpl& s, const std::vector<std::pair<uint32_t, uint32_t>>& pairs) {
   if (pairs.empty()) return;
+  std::vector<uint32_t> pi(s.n);
+  for (uint32_t q = 0; q < s.n; ++q) pi[q] = q;
+  for (auto& pr : pairs) std::swap(pi[pr.first], pi[pr.second]);
   SwapGeom g{};
-  g.np = int(pairs.size());
-  for (size_t p = 0; p < pairs.size(); ++p) {
-    g.a[p] = uint8_t(pairs[p].first);
-    g.b[p] = uint8_t(pairs[p].second);
-    g.mask |= (uint64_t(1) << pairs[p].first) | (uint64_t(1) << pairs[p].second);
+  // 256-byte rows, 16 KB tiles.
+  const uint32_t m = std::min<uint32_t>(s.bits == 32 ? 5 : 4, s.n);
+  const uint32_t most = std::min<uint32_t>(s.bits == 32 ? kSwapTileBits : kSwapTileBits - 1, s.n);
+  // Element bits: the low bits, each one's image outside them next to it
+  // (row bit i for low bit i as far as that goes), then more bits or pairs.
+  std::vector<uint32_t> bits;
+  std::vector<bool> in(s.n, false);
+  auto add = [&](uint32_t q) {
+    if (!in[q]) bits.push_back(q);
+    in[q] = true;
+  };
+  for (uint32_t q = 0; q < m; ++q) add(q);
+  std::vector<uint32_t> rows(m, ~0u), more;
+  size_t count = m;
+  for (uint32_t q = 0; q < m; ++q)
+    if (pi[q] >= m) {
+      rows[q] = pi[q];
+      in[pi[q]] = true;
+      ++count;
+    }
+  for (uint32_t q = m; q < s.n; ++q) {
+    if (in[q]) continue;
+    const uint32_t need = pi[q] == q ? 1 : 2;
+    if (count + need > most) continue;
+    more.push_back(q);
+    in[q] = true;
+    if (need == 2) {
+      more.push_back(pi[q]);
+      in[pi[q]] = true;
+    }
+    count += need;
   }
+  size_t next = 0;
+  for (uint32_t q = 0; q < m; ++q) {
+    if (rows[q] != ~0u)
+      bits.push_back(rows[q]);
+    else if (next < more.size())
+      bits.push_back(more[next++]);
+  }
+  while (next < more.size()) bits.push_back(more[next++]);
+  // A gap (a low bit whose image stays low, and no bit to fill it) would
+  // only cost bank conflicts: the order of the row bits is free.
+  g.k = int(bits.size());
+  g.m = int(m);
+  g.tiles = uint64_t(1) << (s.n - bits.size());
+  std::vector<uint32_t> sorted(bits);
+  std::sort(sorted.begin(), sorted.end());
+  for (size_t i = 0; i < bits.size(); ++i) {
+    g.fixed[i] = uint8_t(sorted[i]);
+    g.bit[i] = uint8_t(bits[i]);
+    g.image[i] = uint8_t(std::find(bits.begin(), bits.end(), pi[bits[i]]) - bits.begin());
+    if (pi[bits[i]] != bits[i]) g.moves = 1;
+  }
+  for (uint32_t i = 0; i < uint32_t(kSwapElems) && i * kThreads < (1u << g.k); ++i) {
+    uint32_t image = 0;
+    for (int j = 0; j < g.k; ++j)
+      if ((i * kThreads >> j) & 1u) {
+        g.off[i] |= uint64_t(1) << g.bit[j];
+        image |= 1u << g.image[j];
+      }
+    g.pos[i] = uint16_t(swap_pos(i * kThreads, g.m));
+    g.from[i] = uint16_t(swap_pos(image, g.m));
+  }
+  // Tile-index bit of a physical bit outside the tile.
+  auto outer = [&](uint32_t q) {
+    uint32_t o = q;
+    for (uint32_t b : bits) o -= b < q ? 1 : 0;
+    return uint8_t(o);
+  };
+  for (auto& pr : pairs)
+    if (!in[pr.first]) {
+      g.a[g.np] = outer(pr.first);
+      g.b[g.np] = outer(pr.second);
+      ++g.np;
+    }
+  const unsigned grid = unsigned(std::min<uint64_t>(g.tiles, uint64_t(s.sms) * 16));
   if (s.bits == 32)
-    k_swap_bits<float><<<grid_for(s, s.size()), kThreads, 0, s.stream>>>(static_cast<float2*>(s.amp), s.size(), g);
+    k_swap_bits<float><<<grid, kThreads, 0, s.stream>>>(static_cast<float2*>(s.amp), g);
   else
-    k_swap_bits<double><<<grid_for(s, s.size()), kThreads, 0, s.stream>>>(static_cast<double2*>(s.amp), s.size(), g);
+    k_swap_bits<double><<<grid, kThreads, 0, s.stream>>>(static_cast<double2*>(s.amp), g);
   QVDG_LAUNCH_CHECK();
 }
 

@@ -787,32 +787,35 @@ DeviceUpload upload_program(StateImpl& s, const Program& p, DeviceScratch& dst) 
 }
 
 // Bring the state to the layout the program's passes use: free on a
-// |0...0> state, otherwise swap passes of disjoint physical bit pairs.
+// |0...0> state, otherwise at most two passes of disjoint bit swaps.
 static void relabel_to(StateImpl& s, const std::vector<uint32_t>& layout) {
   if (layout == s.layout) return;
   if (s.zero_state) {
     s.layout = layout;
     return;
   }
-  while (s.layout != layout) {
-    std::vector<std::pair<uint32_t, uint32_t>> pairs;
-    uint64_t used = 0;
-    for (uint32_t q = 0; q < s.n; ++q) {
-      const uint32_t a = s.layout[q], b = layout[q];
-      const uint64_t m = (uint64_t(1) << a) | (uint64_t(1) << b);
-      if (a == b || (used & m)) continue;
-      used |= m;
-      pairs.push_back({a, b});
+  // Any permutation of the bits is two passes of disjoint swaps: along each
+  // cycle c_0 -> c_1 -> ... (c_i: a bit, c_i+1: where it belongs), first
+  // c_i <-> c_-i, then c_i <-> c_1-i.
+  std::vector<uint32_t> to(s.n);  // present position -> position in `layout`
+  for (uint32_t q = 0; q < s.n; ++q) to[s.layout[q]] = layout[q];
+  std::vector<std::pair<uint32_t, uint32_t>> pairs[2];
+  std::vector<bool> seen(s.n, false);
+  for (uint32_t p = 0; p < s.n; ++p) {
+    std::vector<uint32_t> cycle;
+    for (uint32_t x = p; !seen[x]; x = to[x]) {
+      seen[x] = true;
+      cycle.push_back(x);
     }
-    launch_swap_bits(s, pairs);
-    for (auto& q : s.layout)
-      for (auto& pr : pairs) {
-        if (q == pr.first)
-          q = pr.second;
-        else if (q == pr.second)
-          q = pr.first;
-      }
+    const size_t k = cycle.size();
+    for (size_t i = 0; i < k; ++i) {
+      const size_t j0 = (k - i) % k, j1 = (k + 1 - i) % k;
+      if (i < j0) pairs[0].push_back({cycle[i], cycle[j0]});
+      if (i < j1) pairs[1].push_back({cycle[i], cycle[j1]});
+    }
   }
+  for (auto& pass : pairs) launch_swap_bits(s, pass);
+  s.layout = layout;
 }
 
 void run_program(StateImpl& s, const Program& p, const DeviceUpload& dev, qvdg_stats* stats) {

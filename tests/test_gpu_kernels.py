@@ -4,7 +4,7 @@ the C ABI), every precision, plain and staged paths."""
 import numpy as np
 import pytest
 
-from conftest import max_distance, random_diagonal, random_qubits, random_state, random_unitary
+from conftest import device_physical, max_distance, random_diagonal, random_qubits, random_state, random_unitary
 from qevedo_simulator_b200 import DeviceState, Op, options
 
 pytestmark = pytest.mark.gpu
@@ -537,3 +537,28 @@ def test_low_qubit_gates_by_warp_shuffles(oracle, bits):
                 st.set_amplitudes(initial)
                 st.apply(m, qubits, controls)
                 assert max_distance(st.amplitudes(), expected) < TOL[bits], (n, qubits, controls)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 9, 10, 11, 12, 13, 16])
+def test_swap_passes_move_every_amplitude(bits, n):
+    """In-place swaps of disjoint bit pairs, low with low, low with high and
+    high with high bits, on states below, at and above a swap tile: the
+    buffer holds the permuted amplitudes and their logical order stays."""
+    rng = np.random.default_rng(100 * n + bits)
+    psi = random_state(rng, n)
+    if bits == 32:
+        psi = psi.astype(np.complex64).astype(np.complex128)
+    picks = [rng.permutation(n)[:2 * int(rng.integers(1, n // 2 + 1))].reshape(-1, 2) for _ in range(4)]
+    picks += [np.array(p) for p in ([[0, n - 1]], [[n - 1, n - 2]], [[i, n - 1 - i] for i in range(n // 2)])]
+    with DeviceState(n, bits) as st:
+        for pairs in picks:
+            st.set_amplitudes(psi)
+            st.swap_physical([tuple(int(x) for x in p) for p in pairs])
+            index = np.arange(1 << n)
+            moved = index.copy()
+            for a, b in pairs:
+                d = ((index >> a) ^ (index >> b)) & 1
+                moved ^= (d << a) | (d << b)
+            assert np.array_equal(device_physical(st), psi[moved])
+            assert np.array_equal(st.amplitudes(), psi)
