@@ -37,6 +37,21 @@ struct PlainGate {
   size_t tc_offset = 0;      // tensor: byte offset of its bf16 matrices in the tensor-core blob
 };
 
+// Diagonal gates that one pass applies, in order, on physical bits.
+constexpr int kDiagRunGates = 8;
+constexpr int kDiagRunTargets = 10;  // QVDG_MAX_DIAGONAL_QUBITS
+// Entries of all its gates' tables together (32 KB of shared memory).
+constexpr uint32_t diag_run_entries(int bits) { return bits == 32 ? 4096u : 2048u; }
+struct DiagRun {
+  int32_t count = 0;
+  uint32_t entries = 0;                               // of all tables
+  uint32_t matrix[kDiagRunGates] = {};                // element offset (complex) of each diagonal in the upload
+  uint16_t table[kDiagRunGates] = {};                 // its place among the pass's tables
+  uint8_t k[kDiagRunGates] = {};
+  uint8_t targets[kDiagRunGates][kDiagRunTargets] = {};  // diagonal index bit j = targets[j]
+  uint64_t control_mask[kDiagRunGates] = {}, control_value[kDiagRunGates] = {};
+};
+
 struct StateImpl {
   uint32_t n = 0;
   int bits = 32;
@@ -74,6 +89,11 @@ struct StateImpl {
 // Launch one plain gate pass; `matrices` is the device copy of the upload
 // (complex in the state's precision).
 void launch_plain_gate(StateImpl& s, const PlainGate& g, const void* matrices);
+// Whether diagonal `g` fits beside the gates of `run`, and adding it.
+bool diag_run_fits(const DiagRun& run, const PlainGate& g, int bits);
+void diag_run_add(DiagRun& run, const PlainGate& g);
+// One pass applying the gates of `run` in order.
+void launch_diag_run(StateImpl& s, const DiagRun& run, const void* matrices);
 // Exchange physical bit pairs in one pass.
 void launch_swap_bits(StateImpl& s, const std::vector<std::pair<uint32_t, uint32_t>>& pairs);
 // |0...0>.

@@ -293,6 +293,108 @@ __global__ void __launch_bounds__(kThreads) k_diag(cplx_t<T>* __restrict__ psi, 
   }
 }
 
+// Several diagonal gates in one pass, each amplitude multiplied by their
+// factors in order (the same products and roundings as one pass per gate).
+// HBM bounds a diagonal pass, so gates that share one cost little more than
+// one of them, as long as finding each gate's factor stays cheap: the bits
+// of an amplitude's index that a gate reads are gathered into its table
+// index by parts, from the thread's low bits (once), from the vector's place
+// in the block's tile (constants) and from the tile's number (through byte
+// tables in shared memory), each part holding all eight gates' indices as
+// 16-bit fields of one 16-byte word. A thread moves 16-byte vectors, four
+// in flight.
+constexpr int kRunUnroll = 4;
+constexpr int kRunTileBits = 10;  // vectors of a block's tile: kThreads * kRunUnroll
+
+__device__ __forceinline__ uint4 or4(const uint4& a, const uint4& b) {
+  return make_uint4(a.x | b.x, a.y | b.y, a.z | b.z, a.w | b.w);
+}
+__device__ __forceinline__ uint32_t field16(const uint4& v, int o) {
+  const uint32_t w = o < 2 ? v.x : (o < 4 ? v.y : (o < 6 ? v.z : v.w));
+  return (o & 1) ? w >> 16 : w & 0xffffu;
+}
+
+// All gates' table indices that the set bits of `x`, standing `shift` bits
+// up in an amplitude's index, give.
+__device__ __forceinline__ uint4 run_index(const DiagRun& g, uint64_t x, int shift) {
+  uint32_t w[4] = {0, 0, 0, 0};
+  const uint64_t i = x << shift;
+#pragma unroll
+  for (int o = 0; o < kDiagRunGates; ++o) {
+    if (o >= g.count) break;
+    uint32_t d = 0;
+    for (int j = 0; j < g.k[o]; ++j) d |= uint32_t((i >> g.targets[o][j]) & 1u) << j;
+    w[o >> 1] |= d << (16 * (o & 1));
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_diag_run(cplx_t<T>* __restrict__ psi, uint64_t vectors, int pieces,
+                                                       const __grid_constant__ DiagRun g,
+                                                       const cplx_t<T>* __restrict__ mats) {
+  constexpr int V = sizeof(T) == 4 ? 2 : 1;       // amplitudes of a vector
+  constexpr int kLow = sizeof(T) == 4 ? 1 : 0;    // index bits inside one
+  constexpr int kTile = kLow + kRunTileBits;      // index bits inside a tile
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx_t<T>* tables = reinterpret_cast<cplx_t<T>*>(smem_raw);
+  uint4* high = reinterpret_cast<uint4*>(smem_raw + ((size_t(g.entries) * sizeof(cplx_t<T>) + 15) & ~size_t(15)));
+  for (int o = 0; o < g.count; ++o)
+    for (int i = threadIdx.x; i < (1 << g.k[o]); i += kThreads) tables[g.table[o] + i] = mats[g.matrix[o] + i];
+  for (int p = 0; p < pieces; ++p) high[p * 256 + threadIdx.x] = run_index(g, threadIdx.x, kTile + 8 * p);
+  const uint4 low = run_index(g, threadIdx.x, kLow);
+  uint4 place[kRunUnroll];
+#pragma unroll
+  for (int u = 0; u < kRunUnroll; ++u) place[u] = run_index(g, uint64_t(u), kLow + 8);
+  uint4 odd = make_uint4(0, 0, 0, 0);  // index bit 0 (complex64: the vector's second amplitude)
+  if constexpr (V == 2) odd = run_index(g, 1, 0);
+  __syncthreads();
+  const uint64_t tiles = (vectors + (1u << kRunTileBits) - 1) >> kRunTileBits;
+  for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const uint64_t v0 = (t << kRunTileBits) + threadIdx.x;
+    float4 raw[kRunUnroll];
+#pragma unroll
+    for (int u = 0; u < kRunUnroll; ++u)
+      if (v0 + u * kThreads < vectors) raw[u] = reinterpret_cast<const float4*>(psi)[v0 + u * kThreads];
+    uint4 base = low;
+    for (int p = 0; p < pieces; ++p) base = or4(base, high[p * 256 + ((t >> (8 * p)) & 255)]);
+#pragma unroll
+    for (int u = 0; u < kRunUnroll; ++u) {
+      const uint64_t v = v0 + u * kThreads;
+      if (v >= vectors) break;
+      const uint4 index = or4(base, place[u]);
+      cplx_t<T> a[V];
+      if constexpr (V == 2) {
+        a[0] = make_float2(raw[u].x, raw[u].y);
+        a[V - 1] = make_float2(raw[u].z, raw[u].w);
+      } else {
+        a[0] = *reinterpret_cast<const cplx_t<T>*>(&raw[u]);
+      }
+#pragma unroll
+      for (int o = 0; o < kDiagRunGates; ++o) {
+        if (o >= g.count) break;
+        const uint32_t d = field16(index, o), second = V == 2 ? field16(odd, o) : 0u;
+        const cplx_t<T>* table = tables + g.table[o];
+        const cplx_t<T> f0 = table[d];
+        cplx_t<T> f1 = f0;
+        if (V == 2 && second) f1 = table[d | second];
+        if (g.control_mask[o]) {
+          const uint64_t i = v << kLow;
+          if ((i & g.control_mask[o]) == g.control_value[o]) a[0] = cmul<T>(f0, a[0]);
+          if (V == 2 && ((i | 1) & g.control_mask[o]) == g.control_value[o]) a[V - 1] = cmul<T>(f1, a[V - 1]);
+        } else {
+          a[0] = cmul<T>(f0, a[0]);
+          if (V == 2) a[V - 1] = cmul<T>(f1, a[V - 1]);
+        }
+      }
+      if constexpr (V == 2)
+        reinterpret_cast<float4*>(psi)[v] = make_float4(a[0].x, a[0].y, a[V - 1].x, a[V - 1].y);
+      else
+        psi[v] = a[0];
+    }
+  }
+}
+
 // Swapping physical bit pairs in place: amplitude j moves to pi(j), pi an
 // involution on index bits. What bounds it is HBM (every amplitude that
 // moves is read and written once, as long as both accesses are coalesced):
@@ -665,6 +767,41 @@ void launch_plain_gate(StateImpl& s, const PlainGate& g, const void* matrices) {
     plain_gate<float>(s, g, matrices);
   else
     plain_gate<double>(s, g, matrices);
+}
+
+bool diag_run_fits(const DiagRun& run, const PlainGate& g, int bits) {
+  return run.count < kDiagRunGates && g.targets.size() <= size_t(kDiagRunTargets) &&
+         run.entries + (1u << g.targets.size()) <= diag_run_entries(bits) &&
+         g.matrix_offset + (size_t(1) << g.targets.size()) <= ~uint32_t(0);
+}
+
+void diag_run_add(DiagRun& run, const PlainGate& g) {
+  const int o = run.count++;
+  run.matrix[o] = uint32_t(g.matrix_offset);
+  run.table[o] = uint16_t(run.entries);
+  run.k[o] = uint8_t(g.targets.size());
+  for (size_t j = 0; j < g.targets.size(); ++j) run.targets[o][j] = uint8_t(g.targets[j]);
+  for (auto& c : g.controls) {
+    run.control_mask[o] |= uint64_t(1) << c.first;
+    if (c.second) run.control_value[o] |= uint64_t(1) << c.first;
+  }
+  run.entries += 1u << g.targets.size();
+}
+
+void launch_diag_run(StateImpl& s, const DiagRun& run, const void* matrices) {
+  const uint64_t vectors = s.amp_bytes / 16;  // a state has at least one (n >= 1)
+  const int index_bits = int(s.n) - (s.bits == 32 ? 1 : 0) - kRunTileBits;  // of the tile's number
+  const int pieces = index_bits > 0 ? (index_bits + 7) / 8 : 0;
+  const size_t smem = ((size_t(run.entries) * s.elem_bytes() + 15) & ~size_t(15)) + size_t(pieces) * 256 * 16;
+  const uint64_t tiles = (vectors + (uint64_t(1) << kRunTileBits) - 1) >> kRunTileBits;
+  const unsigned grid = unsigned(std::min<uint64_t>(tiles, uint64_t(s.sms) * 8));
+  if (s.bits == 32)
+    k_diag_run<float><<<grid, kThreads, smem, s.stream>>>(static_cast<float2*>(s.amp), vectors, pieces, run,
+                                                          static_cast<const float2*>(matrices));
+  else
+    k_diag_run<double><<<grid, kThreads, smem, s.stream>>>(static_cast<double2*>(s.amp), vectors, pieces, run,
+                                                           static_cast<const double2*>(matrices));
+  QVDG_LAUNCH_CHECK();
 }
 
 void launch_swap_bits(StateImpl& s, const std::vector<std::pair<uint32_t, uint32_t>>& pairs) {

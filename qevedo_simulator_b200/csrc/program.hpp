@@ -2,6 +2,7 @@
 // their gate programs, built on the host once and uploaded to the device.
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "engine.hpp"
@@ -24,6 +25,13 @@ struct Target {
 // kind of pass, its gates by type and width, where they sit, tile shape.
 constexpr int kPassFeatures = 32;
 
+// What a run launches after its zero-start prefix: pass `pass`, or the
+// diagonal passes of `diag` as one pass over the state.
+struct ProgramStep {
+  size_t pass = 0;
+  std::shared_ptr<const DiagRun> diag;
+};
+
 struct Program {
   Target target;                      // the state the program starts from (layout included)
   std::vector<uint32_t> run_layout;   // the layout its passes use, when it relabels first (else empty)
@@ -40,6 +48,11 @@ struct Program {
   // controls that must be 0 and move only 2^-c of the state.
   std::vector<LoweredPass> zero_passes;
   std::vector<double> zero_pass_bytes;
+  // passes[zero_passes.size()..] as launches, in order, and the bytes that
+  // shared diagonal passes save. `passes` and `features` keep one entry per
+  // fused op, and a run that times its passes launches them one by one.
+  std::vector<ProgramStep> steps;
+  double shared_bytes = 0.0;
 };
 
 void pass_features(const Target& t, const PlannedPass& p, const LoweredPass& lp, const StageUpload& up, float* f);

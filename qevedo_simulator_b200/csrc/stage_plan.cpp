@@ -391,6 +391,49 @@ bool zero_start_layout(const std::vector<PlannedPass>& passes, uint32_t n, bool 
   return layout != given;
 }
 
+// Diagonal passes commute with one another and with passes on other qubits:
+// each waits, past the passes that share no qubit with it, for others to
+// share one pass over the state with (the 28-qubit QFT at fusion 6: 27
+// diagonal passes become 9). Gates with controls move 2^-c of the state when
+// they run alone, so they share only where that moves less.
+void share_diagonal_passes(Program& prog, const std::vector<uint64_t>& touches) {
+  std::vector<size_t> waiting;
+  auto run = std::make_shared<DiagRun>();
+  auto flush = [&] {
+    double alone = 0.0, whole = 0.0;
+    for (size_t i : waiting) {
+      alone += prog.pass_bytes[i];
+      whole = std::max(whole, prog.pass_bytes[i] * double(uint64_t(1) << prog.passes[i].plain.controls.size()));
+    }
+    if (waiting.size() > 1 && alone > 1.25 * whole) {
+      prog.steps.push_back({waiting[0], run});
+      prog.shared_bytes += alone - whole;
+    } else {
+      for (size_t i : waiting) prog.steps.push_back({i, nullptr});
+    }
+    waiting.clear();
+    run = std::make_shared<DiagRun>();
+  };
+  for (size_t i = prog.zero_passes.size(); i < prog.passes.size(); ++i) {
+    const LoweredPass& lp = prog.passes[i];
+    if (!lp.staged && !lp.block && !lp.pair && lp.plain.diagonal) {
+      if (!diag_run_fits(*run, lp.plain, prog.target.bits)) flush();
+      if (diag_run_fits(*run, lp.plain, prog.target.bits)) {
+        diag_run_add(*run, lp.plain);
+        waiting.push_back(i);
+      } else {
+        prog.steps.push_back({i, nullptr});
+      }
+      continue;
+    }
+    bool held = lp.staged;
+    for (size_t w : waiting) held = held || (touches[w] & touches[i]);
+    if (held) flush();
+    prog.steps.push_back({i, nullptr});
+  }
+  flush();
+}
+
 }  // namespace
 
 Program build_program(const Target& t, const std::vector<HOp>& ops, const qvdg_options& opt,
@@ -674,9 +717,12 @@ Program build_program(const Target& t, const std::vector<HOp>& ops, const qvdg_o
     if (opt.staged) throw Error(QVDG_ERR_INVALID, "fused ops exist for plain plans only");
     for (size_t i : order) fused->insert(fused->end(), passes[i].ops.begin(), passes[i].ops.end());
   }
+  std::vector<uint64_t> touches;  // logical qubits of each of prog.passes
   for (size_t k = 0; k < order.size(); ++k) {
     const size_t pi = order[k];
     const PlannedPass& p = passes[pi];
+    touches.push_back(pass_qubits(p));
+    if (pair_next[k]) touches.back() |= pass_qubits(passes[order[k + 1]]);
     if (pair_next[k]) {
       // Two fused 6-qubit gates in one pass: both blobs in the upload, the
       // pass described by its first gate and the pair geometry.
@@ -757,6 +803,7 @@ Program build_program(const Target& t, const std::vector<HOp>& ops, const qvdg_o
     prog.zero_passes.push_back(lower_pass(tt, v, prog.cfg, prog.upload, tc ? &vb : nullptr));
     prog.zero_pass_bytes.push_back(2.0 * state_bytes / double(uint64_t(1) << v.ops[0].controls.size()));
   }
+  share_diagonal_passes(prog, touches);
   return prog;
 }
 
@@ -834,11 +881,21 @@ void run_program(StateImpl& s, const Program& p, const DeviceUpload& dev, qvdg_s
   // The passes' layout (a relabel pass is timed with them).
   relabel_to(s, p.run_layout.empty() ? p.target.layout : p.run_layout);
   s.zero_state = false;
-  for (size_t i = 0; i < p.passes.size(); ++i) {
-    if (timing) QVDG_CUDA(cudaEventRecord(s.pass_events[i], s.stream));
-    launch_pass(s, pass(i), dev);
+  if (timing) {
+    for (size_t i = 0; i < p.passes.size(); ++i) {
+      QVDG_CUDA(cudaEventRecord(s.pass_events[i], s.stream));
+      launch_pass(s, pass(i), dev);
+    }
+    QVDG_CUDA(cudaEventRecord(s.pass_events[p.passes.size()], s.stream));
+  } else {
+    for (size_t i = 0; i < p.zero_passes.size(); ++i) launch_pass(s, pass(i), dev);
+    for (const ProgramStep& step : p.steps) {
+      if (step.diag)
+        launch_diag_run(s, *step.diag, dev.mats);
+      else
+        launch_pass(s, p.passes[step.pass], dev);
+    }
   }
-  if (timing) QVDG_CUDA(cudaEventRecord(s.pass_events[p.passes.size()], s.stream));
   QVDG_CUDA(cudaEventRecord(s.ev_stop, s.stream));
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
   bool tensor = false;
@@ -872,7 +929,7 @@ void run_program(StateImpl& s, const Program& p, const DeviceUpload& dev, qvdg_s
     for (size_t i = 0; i < zero; ++i) s.pass_bytes[i] = p.zero_pass_bytes[i];
   }
   if (stats) {
-    double bytes = p.bytes;
+    double bytes = p.bytes - (timing ? 0.0 : p.shared_bytes);
     for (size_t i = 0; i < zero; ++i) bytes += p.zero_pass_bytes[i] - p.pass_bytes[i];
     stats->kernels += p.kernels;
     stats->passes += p.passes.size();

@@ -562,3 +562,42 @@ def test_swap_passes_move_every_amplitude(bits, n):
                 moved ^= (d << a) | (d << b)
             assert np.array_equal(device_physical(st), psi[moved])
             assert np.array_equal(st.amplitudes(), psi)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [1, 2, 5, 10, 11, 12, 13, 18, 20])
+def test_shared_diagonal_passes_equal_separate_ones(oracle, bits, n):
+    """Diagonals (with and without controls), up to the widest and more than
+    one pass holds, applied together: bit for bit what one pass per gate
+    gives (a run that times its passes) where nothing stands between them.
+    Between dense gates, where a diagonal also moves past those on other
+    qubits, the same state up to rounding."""
+    rng = np.random.default_rng(7 * n + bits)
+    ops = []
+    for i in range(40):
+        if i % 9 == 8:
+            ops.append(Op(random_qubits(rng, n, 1), [], random_unitary(rng, 1)))
+            continue
+        k = min(n, int(rng.integers(1, 5)) if i % 5 else 10)
+        c = int(rng.integers(0, min(4, n - k + 1))) if i % 2 else 0
+        qs = random_qubits(rng, n, k + c)
+        ops.append(Op(qs[:k], [(q, bool(rng.integers(0, 2))) for q in qs[k:]], random_diagonal(rng, k)))
+    psi = random_state(rng, n)
+    diagonals = [op for op in ops if np.count_nonzero(op.matrix) <= op.matrix.shape[0]]
+    for program in (diagonals, ops):
+        got = []
+        with DeviceState(n, bits) as st:
+            for timed in (False, True):
+                st.set_amplitudes(psi)
+                st.set_pass_timing(timed)
+                stats = st.apply_ops(program, options(1, staged=False))
+                got.append((st.amplitudes(), stats))
+            assert len(st.pass_times()[0]) == stats["passes"]
+        if program is diagonals:
+            assert np.array_equal(got[0][0], got[1][0])
+        assert max_distance(got[0][0], got[1][0]) < {32: 1e-5, 64: 1e-11}[bits]
+        if n >= 10:
+            assert got[0][1]["bytes"] < got[1][1]["bytes"]
+        if n <= 13:
+            expected = oracle.naive_statevector(program, n, initial=psi)
+            assert max_distance(got[0][0], expected) < {32: 1e-5, 64: 1e-11}[bits]
