@@ -59,86 +59,168 @@ __device__ double block_sum(double v, double* red) {
   return t;
 }
 
+// The amplitudes of a 16-byte vector: two of complex64, one of complex128.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_sumsq(const cplx_t<T>* __restrict__ psi, uint64_t len,
+constexpr int kPerVec = sizeof(T) == 4 ? 2 : 1;
+
+template <typename T>
+__device__ __forceinline__ void unpack(const float4& v, cplx_t<T>* a) {
+  if constexpr (sizeof(T) == 4) {
+    a[0] = make_float2(v.x, v.y);
+    a[1] = make_float2(v.z, v.w);
+  } else {
+    a[0] = *reinterpret_cast<const double2*>(&v);
+  }
+}
+
+// Vectors a thread of a whole-state reduction has in flight. These passes
+// read the state once (HBM bounds them); with one 8-byte load in flight per
+// thread they ran at half the copy rate.
+constexpr int kReduceUnroll = 4;
+
+// Sum of |a|^2 over the vectors (of a state of at least one vector) whose
+// index has bit `bit` set, or over all of them (bit < 0); with `odd`, over
+// each vector's second amplitude alone.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_sumsq(const float4* __restrict__ psi, uint64_t count, int bit, int odd,
                                                     double* __restrict__ partials) {
   __shared__ double red[32];
   double acc = 0.0;
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < len; i += stride) {
-    const cplx_t<T> a = psi[i];
-    acc += double(a.x) * double(a.x) + double(a.y) * double(a.y);
+  const uint64_t step = uint64_t(gridDim.x) * kThreads;
+  const uint64_t low = bit < 0 ? 0 : (uint64_t(1) << bit) - 1;
+  auto at = [&](uint64_t i) { return bit < 0 ? i : (((i & ~low) << 1) | (uint64_t(1) << bit) | (i & low)); };
+  for (uint64_t i = uint64_t(blockIdx.x) * kThreads + threadIdx.x; i < count; i += step * kReduceUnroll) {
+    float4 v[kReduceUnroll];
+#pragma unroll
+    for (int u = 0; u < kReduceUnroll; ++u)
+      if (i + u * step < count) v[u] = __ldcs(psi + at(i + u * step));
+#pragma unroll
+    for (int u = 0; u < kReduceUnroll; ++u) {
+      if (i + u * step >= count) break;
+      cplx_t<T> a[kPerVec<T>];
+      unpack<T>(v[u], a);
+#pragma unroll
+      for (int e = 0; e < kPerVec<T>; ++e)
+        if (e == 1 || !odd) acc += prob<T>(a[e]);
+    }
   }
   const double t = block_sum(acc, red);
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
-// Sums `count` vectors of `width` doubles (vector i at partials + i*width)
-// into out[0..width), each component in index order.
-__global__ void k_sum_columns(const double* __restrict__ partials, int count, int width, double* __restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= width) return;
+// Sums `count` vectors of `width` doubles (vector i at partials + i*width),
+// one block per component in a fixed order, into out[0..width): device or
+// mapped host memory. A single thread per component took longer than the
+// reduction before it on states that fit in L2.
+__global__ void __launch_bounds__(kThreads) k_sum_columns(const double* __restrict__ partials, int count, int width,
+                                                          double* __restrict__ out) {
+  __shared__ double red[32];
   double t = 0.0;
-  for (int i = 0; i < count; ++i) t += partials[size_t(i) * width + j];
-  out[j] = t;
+  for (int i = threadIdx.x; i < count; i += kThreads) t += partials[size_t(i) * width + blockIdx.x];
+  t = block_sum(t, red);
+  if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 // Per-bit probabilities. A segment is 1024 consecutive amplitudes: bits 0-1
-// inside a thread (4 elements), bits 2-9 from the thread index. Each block
-// takes `per_block` consecutive segments (a power of two), so the low
-// log2(per_block) segment bits vary inside the block and the others are fixed
-// by the block index. Each block writes P(bit = 1) for every bit, then the
-// total, to partials[block * (n + 1) + ...].
-constexpr int kMaxVarBits = 16;
+// inside a thread (4 elements), bits 2-9 from the thread index; a group is
+// 2^var_bits consecutive segments, and blocks take groups in turn, so that
+// the grid need not be a power of two and fills the SMs evenly. A thread
+// keeps one sum per varying segment bit of the group (kSegmentBits at most);
+// the group's sum goes to its index bits in lane b of each warp for bit b.
+// Each block writes P(bit = 1) for every bit, then the total, to
+// partials[block * (n + 1) + ...]. `aligned`: psi lies on a 16-byte boundary
+// (a caller's own complex64 buffer may not).
+constexpr int kSegmentBits = 6;
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_bit_probs(const cplx_t<T>* __restrict__ psi, int n,
-                                                        uint64_t per_block, int var_bits,
-                                                        double* __restrict__ partials) {
-  __shared__ double red[32];
+__global__ void __launch_bounds__(kThreads, 4) k_bit_probs(const cplx_t<T>* __restrict__ psi, int n, uint64_t groups,
+                                                           int var_bits, bool aligned,
+                                                           double* __restrict__ partials) {
+  constexpr int kVecs = 4 / kPerVec<T>;  // vectors of a thread's 4 amplitudes
+  constexpr int kWarps = kThreads / 32;
+  __shared__ double own[kWarps][10 + kSegmentBits];  // bits 0..9 and the segment bits
+  __shared__ double index[kWarps][32];               // the group index bits
+  __shared__ double totals[kWarps];
   const uint64_t len = uint64_t(1) << n;
-  double tot = 0.0, lo0 = 0.0, lo1 = 0.0;
-  double hv[kMaxVarBits];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double tot = 0.0, lo0 = 0.0, lo1 = 0.0, hacc = 0.0;
+  double hv[kSegmentBits];
 #pragma unroll
-  for (int b = 0; b < kMaxVarBits; ++b) hv[b] = 0.0;
-  for (uint64_t i = 0; i < per_block; ++i) {
-    const uint64_t first = ((uint64_t(blockIdx.x) * per_block + i) << 10) + uint64_t(threadIdx.x) * 4;
-    double st = 0.0;
+  for (int b = 0; b < kSegmentBits; ++b) hv[b] = 0.0;
+  for (uint64_t g = blockIdx.x; g < groups; g += gridDim.x) {
+    double sum = 0.0;
+#pragma unroll 2
+    for (uint32_t i = 0; i < (1u << var_bits); ++i) {
+      const uint64_t first = (((g << var_bits) + i) << 10) + uint64_t(threadIdx.x) * 4;
+      double p[4];
+      if (aligned && first + 4 <= len) {
+        float4 v[kVecs];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (first + e < len) {
-        const double p = prob<T>(psi[first + e]);
-        st += p;
-        if (e & 1) lo0 += p;
-        if (e & 2) lo1 += p;
+        for (int e = 0; e < kVecs; ++e) v[e] = reinterpret_cast<const float4*>(psi + first)[e];
+#pragma unroll
+        for (int e = 0; e < kVecs; ++e) {
+          cplx_t<T> a[kPerVec<T>];
+          unpack<T>(v[e], a);
+#pragma unroll
+          for (int f = 0; f < kPerVec<T>; ++f) p[e * kPerVec<T> + f] = prob<T>(a[f]);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[e] = first + e < len ? prob<T>(psi[first + e]) : 0.0;
       }
-    }
-    tot += st;
+      lo0 += p[1] + p[3];
+      lo1 += p[2] + p[3];
+      const double st = (p[0] + p[1]) + (p[2] + p[3]);
+      sum += st;
 #pragma unroll
-    for (int b = 0; b < kMaxVarBits; ++b)
-      if ((i >> b) & 1) hv[b] += st;
+      for (int b = 0; b < kSegmentBits; ++b)
+        if ((i >> b) & 1) hv[b] += st;
+    }
+    tot += sum;
+    double w = sum;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if ((g >> lane) & 1) hacc += w;
   }
+  auto put = [&](int bit, double v) {
+    const double s = warp_sum(v);
+    if (lane == 0) own[warp][bit] = s;
+  };
+  put(0, lo0);
+  put(1, lo1);
+#pragma unroll
+  for (int b = 2; b < 10; ++b) put(b, ((threadIdx.x >> (b - 2)) & 1) ? tot : 0.0);
+#pragma unroll
+  for (int b = 0; b < kSegmentBits; ++b) put(10 + b, hv[b]);
+  const double t = warp_sum(tot);
+  if (lane == 0) totals[warp] = t;
+  index[warp][lane] = hacc;
+  __syncthreads();
   double* out = partials + size_t(blockIdx.x) * (n + 1);
-  for (int bit = 0; bit < n; ++bit) {
-    double v = 0.0;
-    if (bit == 0) {
-      v = lo0;
-    } else if (bit == 1) {
-      v = lo1;
-    } else if (bit < 10) {
-      v = ((threadIdx.x >> (bit - 2)) & 1) ? tot : 0.0;
-    } else if (bit < 10 + var_bits) {
-#pragma unroll
-      for (int b = 0; b < kMaxVarBits; ++b)
-        if (b == bit - 10) v = hv[b];
-    } else {
-      v = ((uint64_t(blockIdx.x) >> (bit - 10 - var_bits)) & 1) ? tot : 0.0;
-    }
-    const double s = block_sum(v, red);
-    if (threadIdx.x == 0) out[bit] = s;
+  for (int bit = threadIdx.x; bit <= n; bit += kThreads) {
+    double s = 0.0;
+    for (int w = 0; w < kWarps; ++w)
+      s += bit == n ? totals[w] : (bit < 10 + var_bits ? own[w][bit] : index[w][bit - 10 - var_bits]);
+    out[bit] = s;
   }
-  const double s = block_sum(tot, red);
-  if (threadIdx.x == 0) out[n] = s;
+}
+
+// The shape of a k_bit_probs launch on at most `most` blocks: groups of up
+// to 2^kSegmentBits segments, smaller ones where the state would not give
+// every block several.
+struct BitProbsShape {
+  uint64_t groups;
+  int var_bits;
+  unsigned blocks;
+};
+BitProbsShape bit_probs_shape(uint32_t n, uint64_t most) {
+  const int seg_bits = n > 10 ? int(n) - 10 : 0;
+  BitProbsShape s{};
+  s.var_bits = std::min(seg_bits, kSegmentBits);
+  while (s.var_bits > 0 && (uint64_t(1) << (seg_bits - s.var_bits)) < 4 * most) --s.var_bits;
+  s.groups = uint64_t(1) << (seg_bits - s.var_bits);
+  s.blocks = unsigned(std::min(s.groups, most));
+  return s;
 }
 
 template <typename T>
@@ -541,16 +623,24 @@ __global__ void __launch_bounds__(kThreads) k_max_diff(const cplx_t<TA>* __restr
 
 unsigned blocks_for(uint64_t items, int threads) { return unsigned(std::max<uint64_t>(1, (items + threads - 1) / threads)); }
 
+// Sum of |a|^2 over the amplitudes with physical bit `bit` set (bit < 0: all
+// of them). One host synchronisation; the sum comes back through mapped
+// pinned memory.
 template <typename T>
-double norm_t(StateImpl& s) {
-  const unsigned blocks = unsigned(umin64(uint64_t(s.sms) * 8, std::max<uint64_t>(1, s.size() / kThreads)));
-  double* d = static_cast<double*>(s.work.get((blocks + 1) * sizeof(double)));
-  k_sumsq<T><<<blocks, kThreads, 0, s.stream>>>(static_cast<const cplx_t<T>*>(s.amp), s.size(), d);
-  QVDG_LAUNCH_CHECK();
-  k_sum_columns<<<1, 32, 0, s.stream>>>(d, int(blocks), 1, d + blocks);
-  QVDG_LAUNCH_CHECK();
+double sumsq_t(StateImpl& s, int bit) {
   double* h = static_cast<double*>(s.host.get(sizeof(double)));
-  QVDG_CUDA(cudaMemcpyAsync(h, d + blocks, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
+  // Bits inside a vector: every vector, complex64's second amplitudes.
+  const int shift = kPerVec<T> == 2 ? 1 : 0;
+  const bool odd = bit >= 0 && bit < shift;
+  const int vec_bit = bit < shift ? -1 : bit - shift;
+  const uint64_t count = (s.amp_bytes / 16) >> (vec_bit < 0 ? 0 : 1);
+  const unsigned blocks = unsigned(std::max<uint64_t>(
+      1, umin64(uint64_t(s.sms) * 8, (count + kThreads * kReduceUnroll - 1) / (kThreads * kReduceUnroll))));
+  double* d = static_cast<double*>(s.work.get(blocks * sizeof(double)));
+  k_sumsq<T><<<blocks, kThreads, 0, s.stream>>>(static_cast<const float4*>(s.amp), count, vec_bit, odd ? 1 : 0, d);
+  QVDG_LAUNCH_CHECK();
+  k_sum_columns<<<1, kThreads, 0, s.stream>>>(d, int(blocks), 1, h);
+  QVDG_LAUNCH_CHECK();
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
   return *h;
 }
@@ -558,23 +648,15 @@ double norm_t(StateImpl& s) {
 template <typename T>
 void bit_probs_t(StateImpl& s, std::vector<double>& p1, double& total) {
   const int n = int(s.n);
-  const uint64_t segments = (s.size() + 1023) >> 10;  // a power of two
-  uint64_t blocks = 1;
-  while (blocks * 2 <= segments && blocks * 2 <= uint64_t(s.sms) * 4) blocks *= 2;
-  while (segments / blocks > (uint64_t(1) << kMaxVarBits)) blocks *= 2;
-  const uint64_t per_block = segments / blocks;
-  int var_bits = 0;
-  while ((uint64_t(1) << var_bits) < per_block) ++var_bits;
+  const BitProbsShape shape = bit_probs_shape(s.n, uint64_t(s.sms) * 4);
   const size_t width = size_t(n) + 1;
-  double* d = static_cast<double*>(s.work.get((size_t(blocks) + 1) * width * sizeof(double)));
-  k_bit_probs<T><<<unsigned(blocks), kThreads, 0, s.stream>>>(static_cast<const cplx_t<T>*>(s.amp), n, per_block,
-                                                              var_bits, d);
-  QVDG_LAUNCH_CHECK();
-  double* sum = d + size_t(blocks) * width;
-  k_sum_columns<<<blocks_for(width, 64), 64, 0, s.stream>>>(d, int(blocks), int(width), sum);
-  QVDG_LAUNCH_CHECK();
+  double* d = static_cast<double*>(s.work.get(size_t(shape.blocks) * width * sizeof(double)));
   double* h = static_cast<double*>(s.host.get(width * sizeof(double)));
-  QVDG_CUDA(cudaMemcpyAsync(h, sum, width * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
+  k_bit_probs<T><<<shape.blocks, kThreads, 0, s.stream>>>(static_cast<const cplx_t<T>*>(s.amp), n, shape.groups,
+                                                          shape.var_bits, true, d);
+  QVDG_LAUNCH_CHECK();
+  k_sum_columns<<<unsigned(width), kThreads, 0, s.stream>>>(d, int(shape.blocks), int(width), h);
+  QVDG_LAUNCH_CHECK();
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
   p1.assign(h, h + n);
   total = h[n];
@@ -763,49 +845,86 @@ size_t counts_t(StateImpl& s, size_t shots, const double* uniforms_host, const M
 
 // <psi|P|psi> for a Pauli string with X/Y on the bits of x, Z/Y on the bits of
 // z (physical): P|j> = i^nY (-1)^popc(j & z) |j ^ x>, so the value is
-// i^nY * sum_j conj(psi[j ^ x]) psi[j] (-1)^popc(j & z). Per-block partial
-// sums (re, im) in double precision, summed in order.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_pauli(const cplx_t<T>* __restrict__ psi, uint64_t len, uint64_t x,
-                                                    uint64_t z, double* __restrict__ partials) {
+// i^nY * sum_j conj(psi[j ^ x]) psi[j] (-1)^popc(j & z). The terms of j and
+// j ^ x are complex conjugates up to the sign (-1)^nY, so the sum is real
+// (nY even) or imaginary (nY odd), and one of the two terms gives both. Each
+// pair of amplitudes is then read once: j runs over the vectors whose x has
+// its top bit clear, with the partner vector beside it (HBM bounds the pass;
+// reading every amplitude twice and summing both parts of both terms took
+// 0.42 ms at 27 qubits in complex64, whose 1 GiB takes 0.16 ms).
+// Per-block sums in double precision, summed in a fixed order.
+// kPairs: x reaches beyond a vector (partner vectors at v ^ xv); otherwise
+// x is 0 or, in complex64, 1 (both amplitudes of a pair in one vector).
+template <typename T, bool kPairs>
+__global__ void __launch_bounds__(kThreads) k_pauli(const float4* __restrict__ psi, uint64_t count, uint64_t x,
+                                                    uint64_t z, int top, int imaginary,
+                                                    double* __restrict__ partials) {
+  constexpr int V = kPerVec<T>;
   __shared__ double red[32];
-  double re = 0.0, im = 0.0;
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < len; j += stride) {
-    const cplx_t<T> a = psi[j], b = psi[j ^ x];
-    // conj(b) * a
-    const double pr = double(b.x) * double(a.x) + double(b.y) * double(a.y);
-    const double pi = double(b.x) * double(a.y) - double(b.y) * double(a.x);
-    const double sgn = (__popcll(j & z) & 1) ? -1.0 : 1.0;
-    re += sgn * pr;
-    im += sgn * pi;
+  double acc = 0.0;
+  const uint64_t step = uint64_t(gridDim.x) * kThreads;
+  const uint64_t low = kPairs ? (uint64_t(1) << top) - 1 : 0;
+  const uint64_t xv = x / V;  // x on vector indices
+  auto at = [&](uint64_t i) { return kPairs ? (((i & ~low) << 1) | (i & low)) : i; };
+  // Sign of amplitude j, from its vector's sign and its place in it.
+  const double second = (V == 2 && (z & 1)) ? -1.0 : 1.0;
+  for (uint64_t i = uint64_t(blockIdx.x) * kThreads + threadIdx.x; i < count; i += step * kReduceUnroll) {
+    float4 u[kReduceUnroll], w[kReduceUnroll];
+#pragma unroll
+    for (int k = 0; k < kReduceUnroll; ++k)
+      if (i + k * step < count) {
+        const uint64_t v = at(i + k * step);
+        u[k] = __ldcs(psi + v);
+        if (kPairs) w[k] = __ldcs(psi + (v ^ xv));
+      }
+#pragma unroll
+    for (int k = 0; k < kReduceUnroll; ++k) {
+      if (i + k * step >= count) break;
+      const uint64_t v = at(i + k * step);
+      cplx_t<T> a[V], b[V];
+      unpack<T>(u[k], a);
+      unpack<T>(kPairs ? w[k] : u[k], b);
+      double t = 0.0;
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        // The partner of amplitude e: place e ^ (x & 1) of the other vector.
+        const cplx_t<T> c = (V == 2 && (x & 1)) ? b[V - 1 - e] : b[e];
+        // conj(c) * a, its real or imaginary part
+        const double p = imaginary ? double(c.x) * double(a[e].y) - double(c.y) * double(a[e].x)
+                                   : double(c.x) * double(a[e].x) + double(c.y) * double(a[e].y);
+        t += e == 1 ? second * p : p;
+      }
+      acc += (__popcll((v * V) & z) & 1) ? -t : t;
+    }
   }
-  const double tr = block_sum(re, red);
-  __syncthreads();
-  const double ti = block_sum(im, red);
-  if (threadIdx.x == 0) {
-    partials[2 * blockIdx.x] = tr;
-    partials[2 * blockIdx.x + 1] = ti;
-  }
+  const double t = block_sum(acc, red);
+  if (threadIdx.x == 0) partials[blockIdx.x] = kPairs ? 2.0 * t : t;
 }
 
 template <typename T>
 double pauli_t(StateImpl& s, uint64_t x, uint64_t z, int ny) {
-  const unsigned blocks = unsigned(umin64(uint64_t(s.sms) * 8, std::max<uint64_t>(1, s.size() / kThreads)));
-  double* d = static_cast<double*>(s.work.get((2 * size_t(blocks) + 2) * sizeof(double)));
-  k_pauli<T><<<blocks, kThreads, 0, s.stream>>>(static_cast<const cplx_t<T>*>(s.amp), s.size(), x, z, d);
+  const uint64_t xv = x / kPerVec<T>;
+  const int top = xv ? 63 - __builtin_clzll(xv) : 0;
+  const uint64_t count = (s.amp_bytes / 16) >> (xv ? 1 : 0);
+  const unsigned blocks = unsigned(std::max<uint64_t>(
+      1, umin64(uint64_t(s.sms) * 8, (count + kThreads * kReduceUnroll - 1) / (kThreads * kReduceUnroll))));
+  double* d = static_cast<double*>(s.work.get(blocks * sizeof(double)));
+  double* h = static_cast<double*>(s.host.get(sizeof(double)));
+  const float4* psi = static_cast<const float4*>(s.amp);
+  if (xv)
+    k_pauli<T, true><<<blocks, kThreads, 0, s.stream>>>(psi, count, x, z, top, ny & 1, d);
+  else
+    k_pauli<T, false><<<blocks, kThreads, 0, s.stream>>>(psi, count, x, z, top, ny & 1, d);
   QVDG_LAUNCH_CHECK();
-  k_sum_columns<<<1, 32, 0, s.stream>>>(d, int(blocks), 2, d + 2 * blocks);
+  k_sum_columns<<<1, kThreads, 0, s.stream>>>(d, int(blocks), 1, h);
   QVDG_LAUNCH_CHECK();
-  double* h = static_cast<double*>(s.host.get(2 * sizeof(double)));
-  QVDG_CUDA(cudaMemcpyAsync(h, d + 2 * blocks, 2 * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
-  const double re = h[0], im = h[1];
+  const double sum = *h;  // i^nY times it is the value
   switch (ny & 3) {
-    case 0: return re;
-    case 1: return -im;
-    case 2: return -re;
-    default: return im;
+    case 0: return sum;
+    case 1: return -sum;
+    case 2: return -sum;
+    default: return sum;
   }
 }
 
@@ -843,7 +962,7 @@ double max_abs_diff(StateImpl& a, StateImpl& b) {
   return m;
 }
 
-double norm_sqr(StateImpl& s) { return s.bits == 32 ? norm_t<float>(s) : norm_t<double>(s); }
+double norm_sqr(StateImpl& s) { return s.bits == 32 ? sumsq_t<float>(s, -1) : sumsq_t<double>(s, -1); }
 
 void bit_probabilities(StateImpl& s, std::vector<double>& p1, double& total) {
   if (s.bits == 32)
@@ -853,10 +972,7 @@ void bit_probabilities(StateImpl& s, std::vector<double>& p1, double& total) {
 }
 
 double probability_one(StateImpl& s, uint32_t physical_bit) {
-  std::vector<double> p1;
-  double total;
-  bit_probabilities(s, p1, total);
-  return p1[physical_bit];
+  return s.bits == 32 ? sumsq_t<float>(s, int(physical_bit)) : sumsq_t<double>(s, int(physical_bit));
 }
 
 void probabilities(StateImpl& s, double* out_host) {
@@ -936,20 +1052,14 @@ void bit_probs_noalloc_t(const void* amplitudes, uint32_t n, cudaStream_t stream
   double* d = noalloc_scratch(device);
   int sms = 0;
   QVDG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const uint64_t segments = ((uint64_t(1) << n) + 1023) >> 10;
-  uint64_t blocks = 1;
-  while (blocks * 2 <= segments && blocks * 2 <= uint64_t(sms) * 4 && blocks * 2 <= kNoAllocMaxBlocks) blocks *= 2;
-  while (segments / blocks > (uint64_t(1) << kMaxVarBits)) blocks *= 2;
-  if (blocks > kNoAllocMaxBlocks) throw Error(QVDG_ERR_UNSUPPORTED, "state too large for the no-allocation scratch");
-  const uint64_t per_block = segments / blocks;
-  int var_bits = 0;
-  while ((uint64_t(1) << var_bits) < per_block) ++var_bits;
+  const BitProbsShape shape = bit_probs_shape(n, umin64(uint64_t(sms) * 4, kNoAllocMaxBlocks));
   const size_t width = size_t(n) + 1;
-  k_bit_probs<T><<<unsigned(blocks), kThreads, 0, stream>>>(static_cast<const cplx_t<T>*>(amplitudes), int(n),
-                                                            per_block, var_bits, d);
+  k_bit_probs<T><<<shape.blocks, kThreads, 0, stream>>>(static_cast<const cplx_t<T>*>(amplitudes), int(n),
+                                                        shape.groups, shape.var_bits,
+                                                        reinterpret_cast<uintptr_t>(amplitudes) % 16 == 0, d);
   QVDG_LAUNCH_CHECK();
-  double* sum = d + size_t(blocks) * width;
-  k_sum_columns<<<blocks_for(width, 64), 64, 0, stream>>>(d, int(blocks), int(width), sum);
+  double* sum = d + size_t(shape.blocks) * width;
+  k_sum_columns<<<unsigned(width), kThreads, 0, stream>>>(d, int(shape.blocks), int(width), sum);
   QVDG_LAUNCH_CHECK();
   QVDG_CUDA(cudaMemcpyAsync(p1, sum, n * sizeof(double), cudaMemcpyDeviceToHost, stream));
   QVDG_CUDA(cudaMemcpyAsync(total, sum + n, sizeof(double), cudaMemcpyDeviceToHost, stream));
