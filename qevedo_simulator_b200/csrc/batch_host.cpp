@@ -4,7 +4,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <complex>
 #include <chrono>
 #include <cstring>
 #include <numeric>
@@ -21,12 +20,14 @@ struct qvdg_batch {
   std::vector<qvdg::BatchCircuit> circuits;
   uint64_t num_matrices = 0, outputs = 0;
   uint32_t max_qubits = 0;
-  void* dev = nullptr;      // circuits | order | sample order | gates | out | queue
-  void* slots = nullptr;    // per-CTA states of wide circuits
-  size_t slot_bytes = 0;
-  double* host_out = nullptr;  // pinned
+  void* dev = nullptr;      // circuits | gates | matrices | out
+  double* matrices = nullptr;  // in dev: the complex128 matrices last given
+  // Work of the chosen shape, and of the autotuner's sample: tasks | wide | queue.
+  void* work = nullptr;
+  void* slots = nullptr;    // states of wide circuits
+  void* partials = nullptr;
+  double* host_out = nullptr;  // pinned: the outputs, then the status word
   qvdg::BatchLaunch launch;    // the chosen shape, whole batch
-  qvdg::BatchLaunch sample;    // the autotuner's sample
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<uint32_t> tune_tiles, tune_threads;
@@ -40,7 +41,8 @@ namespace {
 
 constexpr int kTileMin = 12, kTileMax = 14;
 constexpr int kMaxCtasPerSm = 4;
-constexpr size_t kSlotBudget = size_t(24) << 30;
+constexpr size_t kSlotBudget = size_t(8) << 30;  // of wide circuits' states at a time
+constexpr uint32_t kMaxDepth = 5;                // layers of an A and B pass (their tables fit kMaxSteps groups)
 
 void require(bool ok, const std::string& message) {
   if (!ok) throw Error(QVDG_ERR_INVALID, message);
@@ -53,104 +55,125 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // r >= 1 low ones) to fit, n <= 2(L - 1) - 1.
 bool shape_fits(uint32_t max_qubits, int L) { return max_qubits <= uint32_t(L) || max_qubits <= uint32_t(2 * L - 3); }
 
-uint64_t slot_elems_for(uint32_t max_qubits, int L) {
-  return max_qubits > uint32_t(L) ? (uint64_t(1) << max_qubits) : 0;
-}
-
-// Persistent CTAs for a shape: all resident CTAs (at most kMaxCtasPerSm per
-// SM), fewer when the per-CTA slots of wide circuits would exceed the budget.
+// Persistent CTAs for a shape: all resident CTAs (at most kMaxCtasPerSm per SM).
 int ctas_for(const qvdg_batch* b, int threads, int L) {
-  const int occ = batch_kernel_occupancy(threads, L);
-  if (occ <= 0) return 0;
-  int ctas = b->sms * std::min(occ, kMaxCtasPerSm);
-  const uint64_t slot = slot_elems_for(b->max_qubits, L) * sizeof(float2);
-  if (slot > 0) ctas = int(std::min<uint64_t>(uint64_t(ctas), std::max<uint64_t>(1, kSlotBudget / slot)));
-  return ctas;
+  return b->sms * std::min(batch_kernel_occupancy(threads, L), kMaxCtasPerSm);
 }
 
-// U = diag(p0, p1) R diag(q0, q1) with R real and unit p, q: rows with one
-// common phase (q = 1) or columns with one (p = 1) when possible, otherwise
-// p0 = 1 and the rest from U's entries (all four nonzero for a unitary that
-// is neither diagonal nor anti-diagonal). False when U has no such form.
-bool decompose(const double* m, float2* rec, bool& left, bool& right) {
-  using Cd = std::complex<double>;
-  const Cd u[4] = {{m[0], m[1]}, {m[2], m[3]}, {m[4], m[5]}, {m[6], m[7]}};
-  auto unit = [](Cd c) { return c / std::abs(c); };
-  const double tol = 1e-9;
-  double r[4];
-  Cd p[2] = {1.0, 1.0}, q[2] = {1.0, 1.0};
-  auto real_of = [&](Cd c, double& out) {
-    if (std::abs(c.imag()) > tol) return false;
-    out = c.real();
-    return true;
-  };
-  auto rows = [&]() {
-    for (int i = 0; i < 2; ++i) {
-      const int k = std::abs(u[2 * i]) >= std::abs(u[2 * i + 1]) ? 0 : 1;
-      if (std::abs(u[2 * i + k]) == 0.0) return false;
-      p[i] = unit(u[2 * i + k]);
-      if (!real_of(u[2 * i] / p[i], r[2 * i]) || !real_of(u[2 * i + 1] / p[i], r[2 * i + 1])) return false;
+// The work of a set of circuits on tiles of L qubits, in the order CTAs take
+// it: waves of wide circuits, as many as there are slots, each wave pass by
+// pass; then the circuits that fit a tile.
+struct Work {
+  std::vector<BatchWide> wide;
+  std::vector<uint32_t> wide_of;  // per circuit
+  std::vector<BatchTask> tasks;
+  uint64_t partials = 0;          // doubles
+};
+
+constexpr uint64_t kPartialRow = 16;  // doubles per tile
+
+// Wide circuits run on tiles of 13 qubits (the largest tile leaves two of
+// them per CTA, so that copies fly under the computation), or the tile's own
+// 12. Pass B keeps 2^r contiguous amplitudes: 64 bytes, or a 32-byte sector
+// where that lets an A and B pass take a layer more.
+void wide_shape(uint32_t n, int L, BatchWide& w) {
+  w.tile_bits = std::min(L, 13);
+  w.low = 2 * w.tile_bits - 3 - int(n) >= 2 ? 3 : 2;
+  w.high = int(n) - (w.tile_bits - w.low);
+  w.layers = std::min<uint32_t>(uint32_t(w.tile_bits - w.high) + 1, kMaxDepth);
+  w.tiles = uint32_t(1) << (n - uint32_t(w.tile_bits));
+}
+
+size_t wide_count(const std::vector<BatchCircuit>& circuits, const std::vector<uint32_t>& order, int L) {
+  size_t k = 0;
+  for (uint32_t i : order) k += circuits[i].num_qubits > uint32_t(L);
+  return k;
+}
+
+Work plan_work(const std::vector<BatchCircuit>& circuits, const std::vector<uint32_t>& order, int L, int ctas,
+               size_t slots, uint64_t slot_elems) {
+  Work w;
+  w.wide_of.assign(circuits.size(), 0);
+  std::vector<uint32_t> wide;  // circuits, largest first as in `order`
+  uint64_t pass_tiles = 0;
+  for (uint32_t i : order)
+    if (circuits[i].num_qubits > uint32_t(L)) {
+      BatchWide x{};
+      const uint32_t k = uint32_t(wide.size());
+      wide_shape(circuits[i].num_qubits, L, x);
+      x.phases = 2 * ((circuits[i].num_layers + x.layers - 1) / x.layers);
+      x.slot = (k % slots) * slot_elems;
+      x.previous = k >= slots ? int32_t(k - slots) : -1;
+      x.partials = w.partials;
+      w.partials += uint64_t(x.tiles) * kPartialRow;
+      w.wide_of[i] = k;
+      w.wide.push_back(x);
+      wide.push_back(i);
+      if (k < slots) pass_tiles += x.tiles;
     }
-    q[0] = q[1] = 1.0;
-    return true;
-  };
-  auto cols = [&]() {
-    for (int j = 0; j < 2; ++j) {
-      const int k = std::abs(u[j]) >= std::abs(u[2 + j]) ? 0 : 1;
-      if (std::abs(u[2 * k + j]) == 0.0) return false;
-      q[j] = unit(u[2 * k + j]);
-      if (!real_of(u[j] / q[j], r[j]) || !real_of(u[2 + j] / q[j], r[2 + j])) return false;
-    }
-    p[0] = p[1] = 1.0;
-    return true;
-  };
-  auto general = [&]() {
-    for (const Cd& c : u)
-      if (std::abs(c) == 0.0) return false;
-    p[0] = 1.0;
-    q[0] = unit(u[0]);
-    q[1] = unit(u[1]);
-    p[1] = unit(u[2] / q[0]);
-    for (int i = 0; i < 2; ++i)
-      for (int j = 0; j < 2; ++j)
-        if (!real_of(u[2 * i + j] / (p[i] * q[j]), r[2 * i + j])) return false;
-    return true;
-  };
-  if (!rows() && !cols() && !general()) return false;
-  for (int i = 0; i < 2; ++i)
-    for (int j = 0; j < 2; ++j)
-      if (std::abs(p[i] * r[2 * i + j] * q[j] - u[2 * i + j]) > tol) return false;
-  rec[0] = make_float2(float(r[0]), float(r[1]));
-  rec[1] = make_float2(float(r[2]), float(r[3]));
-  rec[2] = make_float2(float(p[0].real()), float(p[0].imag()));
-  rec[3] = make_float2(float(p[1].real()), float(p[1].imag()));
-  rec[4] = make_float2(float(q[0].real()), float(q[0].imag()));
-  rec[5] = make_float2(float(q[1].real()), float(q[1].imag()));
-  left = left || p[0] != Cd(1.0) || p[1] != Cd(1.0);
-  right = right || q[0] != Cd(1.0) || q[1] != Cd(1.0);
-  return true;
+  // Tiles of a task: several where that still leaves every CTA a few tasks
+  // of each pass (a task builds its gate tables once).
+  uint32_t grain = 1;
+  while (grain < 8 && pass_tiles >= uint64_t(grain) * 2 * 6 * uint64_t(ctas)) grain *= 2;
+  for (size_t first = 0; first < wide.size(); first += slots) {
+    const size_t end = std::min(wide.size(), first + slots);
+    uint32_t phases = 0;
+    for (size_t k = first; k < end; ++k) phases = std::max(phases, w.wide[k].phases);
+    for (uint32_t p = 0; p <= phases; ++p)
+      for (size_t k = first; k < end; ++k) {
+        const BatchWide& x = w.wide[k];
+        if (p > x.phases) continue;
+        if (p == x.phases || p == 0) {
+          w.tasks.push_back({wide[k], p, 0, 1});
+          continue;
+        }
+        const uint32_t g = std::min(grain, x.tiles);
+        for (uint32_t t = 0; t < x.tiles; t += g) w.tasks.push_back({wide[k], p, t, g});
+      }
+  }
+  for (uint32_t i : order)
+    if (circuits[i].num_qubits <= uint32_t(L)) w.tasks.push_back({i, 0, 0, 1});
+  return w;
 }
 
-// A circuit's gate records (kBatchGateSlots complex64 per matrix) and its
-// form: phased when every matrix decomposes, else the generic matrices.
-uint32_t encode_gates(const double* src, size_t num_matrices, float2* dst) {
-  bool left = false, right = false, phased = true;
-  for (size_t i = 0; i < num_matrices && phased; ++i)
-    phased = decompose(src + 8 * i, dst + kBatchGateSlots * i, left, right);
-  if (phased) return kBatchPhased | (left ? kBatchLeft : 0u) | (right ? kBatchRight : 0u);
-  for (size_t i = 0; i < num_matrices; ++i)
-    for (int k = 0; k < kBatchGateSlots; ++k)
-      dst[kBatchGateSlots * i + k] =
-          k < 4 ? make_float2(float(src[8 * i + 2 * k]), float(src[8 * i + 2 * k + 1])) : make_float2(0.f, 0.f);
-  return 0;
-}
-
-BatchLaunch shape(const BatchLaunch& base, int L, int threads, int ctas, uint32_t max_qubits) {
+// Plans the circuits of `order` on a shape and puts their work on the device
+// (an allocation of its own in *work, replacing what it held). The circuits'
+// `wide` fields follow.
+BatchLaunch shape(qvdg_batch* b, const BatchLaunch& base, const std::vector<uint32_t>& order, int L, int threads,
+                  int ctas, size_t slots, uint64_t slot_elems, void** work) {
+  const Work w = plan_work(b->circuits, order, L, ctas, std::max<size_t>(slots, 1), slot_elems);
+  require(w.tasks.size() < (size_t(1) << 31), "the batch has too many tiles");
   BatchLaunch l = base;
   l.tile_qubits = L;
   l.threads = threads;
   l.ctas = ctas;
-  l.slot_elems = slot_elems_for(max_qubits, L);
+  l.count = uint32_t(w.tasks.size());
+  const size_t o_tasks = 0;
+  const size_t o_wide = align256(o_tasks + w.tasks.size() * sizeof(BatchTask));
+  const size_t o_queue = align256(o_wide + std::max<size_t>(w.wide.size(), 1) * sizeof(BatchWide));
+  const size_t queue_bytes = 256 + std::max<size_t>(w.wide.size(), 1) * sizeof(uint32_t);
+  QVDG_CUDA(cudaStreamSynchronize(b->stream));
+  if (*work) cudaFree(*work);
+  *work = nullptr;
+  QVDG_CUDA(cudaMalloc(work, o_queue + queue_bytes));
+  char* d = static_cast<char*>(*work);
+  QVDG_CUDA(cudaMemcpyAsync(d + o_tasks, w.tasks.data(), w.tasks.size() * sizeof(BatchTask), cudaMemcpyHostToDevice,
+                            b->stream));
+  if (!w.wide.empty())
+    QVDG_CUDA(cudaMemcpyAsync(d + o_wide, w.wide.data(), w.wide.size() * sizeof(BatchWide), cudaMemcpyHostToDevice,
+                              b->stream));
+  for (uint32_t i : order) b->circuits[i].wide = w.wide_of[i];
+  QVDG_CUDA(cudaMemcpyAsync(const_cast<BatchCircuit*>(l.circuits), b->circuits.data(),
+                            b->circuits.size() * sizeof(BatchCircuit), cudaMemcpyHostToDevice, b->stream));
+  // The circuits' forms are written with their records.
+  launch_batch_encode(l, b->matrices, uint32_t(b->circuits.size()), b->stream);
+  QVDG_CUDA(cudaStreamSynchronize(b->stream));  // the host copies go out of scope
+  l.tasks = reinterpret_cast<const BatchTask*>(d + o_tasks);
+  l.wide = reinterpret_cast<const BatchWide*>(d + o_wide);
+  l.queue = reinterpret_cast<uint32_t*>(d + o_queue);
+  l.status = reinterpret_cast<int*>(d + o_queue + 128);
+  l.done = reinterpret_cast<uint32_t*>(d + o_queue + 256);
+  l.queue_bytes = queue_bytes;
   return l;
 }
 
@@ -169,7 +192,9 @@ void release(qvdg_batch* b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
   if (b->dev) cudaFree(b->dev);
+  if (b->work) cudaFree(b->work);
   if (b->slots) cudaFree(b->slots);
+  if (b->partials) cudaFree(b->partials);
   if (b->host_out) cudaFreeHost(b->host_out);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
@@ -208,10 +233,11 @@ qvdg_batch* batch_create(const qvdg_layered_circuit* circuits, size_t count, con
       b->max_qubits = std::max(b->max_qubits, c.num_qubits);
     }
     if (want_tile) require(shape_fits(b->max_qubits, int(want_tile)), "tile_qubits too small for the widest circuit");
-    std::vector<float2> gates(b->num_matrices * kBatchGateSlots);
+    std::vector<double> matrices(b->num_matrices * 8);
     for (size_t i = 0; i < count; ++i)
-      b->circuits[i].form = encode_gates(circuits[i].gates, size_t(circuits[i].num_layers) * circuits[i].num_qubits,
-                                         gates.data() + kBatchGateSlots * b->circuits[i].gates);
+      if (circuits[i].num_layers)
+        std::memcpy(matrices.data() + 8 * b->circuits[i].gates, circuits[i].gates,
+                    size_t(circuits[i].num_layers) * circuits[i].num_qubits * 8 * sizeof(double));
     // Largest first: an atomic counter then hands out work longest-first.
     std::vector<uint32_t> order(count);
     std::iota(order.begin(), order.end(), 0u);
@@ -230,31 +256,22 @@ qvdg_batch* batch_create(const qvdg_layered_circuit* circuits, size_t count, con
     QVDG_CUDA(cudaEventCreate(&b->ev0));
     QVDG_CUDA(cudaEventCreate(&b->ev1));
     const size_t o_circ = 0;
-    const size_t o_order = align256(o_circ + count * sizeof(BatchCircuit));
-    const size_t o_sample = align256(o_order + count * sizeof(uint32_t));
-    const size_t o_gates = align256(o_sample + sample.size() * sizeof(uint32_t));
-    const size_t o_out = align256(o_gates + std::max<size_t>(gates.size(), 1) * sizeof(float2));
-    const size_t o_queue = align256(o_out + b->outputs * sizeof(double));
-    const size_t total = o_queue + 256;
+    const size_t o_gates = align256(o_circ + count * sizeof(BatchCircuit));
+    const size_t o_mats = align256(o_gates + std::max<size_t>(b->num_matrices, 1) * kBatchGateSlots * sizeof(float2));
+    const size_t o_out = align256(o_mats + std::max<size_t>(matrices.size(), 1) * sizeof(double));
+    const size_t total = o_out + b->outputs * sizeof(double);
     QVDG_CUDA(cudaMalloc(&b->dev, total));
     char* base = static_cast<char*>(b->dev);
-    QVDG_CUDA(cudaMemcpy(base + o_circ, b->circuits.data(), count * sizeof(BatchCircuit), cudaMemcpyHostToDevice));
-    QVDG_CUDA(cudaMemcpy(base + o_order, order.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    QVDG_CUDA(cudaMemcpy(base + o_sample, sample.data(), sample.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    if (!gates.empty())
-      QVDG_CUDA(cudaMemcpy(base + o_gates, gates.data(), gates.size() * sizeof(float2), cudaMemcpyHostToDevice));
-    QVDG_CUDA(cudaMallocHost(&b->host_out, std::max<uint64_t>(b->outputs, 1) * sizeof(double)));
+    b->matrices = reinterpret_cast<double*>(base + o_mats);
+    if (!matrices.empty())
+      QVDG_CUDA(cudaMemcpyAsync(b->matrices, matrices.data(), matrices.size() * sizeof(double),
+                                cudaMemcpyHostToDevice, b->stream));
+    QVDG_CUDA(cudaMallocHost(&b->host_out, (b->outputs + 1) * sizeof(double)));
 
     BatchLaunch whole;
     whole.circuits = reinterpret_cast<const BatchCircuit*>(base + o_circ);
-    whole.order = reinterpret_cast<const uint32_t*>(base + o_order);
-    whole.count = uint32_t(count);
     whole.gates = reinterpret_cast<const float2*>(base + o_gates);
     whole.out = reinterpret_cast<double*>(base + o_out);
-    whole.queue = reinterpret_cast<uint32_t*>(base + o_queue);
-    BatchLaunch samp = whole;
-    samp.order = reinterpret_cast<const uint32_t*>(base + o_sample);
-    samp.count = uint32_t(sample.size());
 
     // Candidate shapes.
     struct Shape {
@@ -270,22 +287,34 @@ qvdg_batch* batch_create(const qvdg_layered_circuit* circuits, size_t count, con
         if (ctas > 0) shapes.push_back({L, t, ctas});
       }
     if (shapes.empty()) throw Error(QVDG_ERR_UNSUPPORTED, "no tile shape can run this batch on this device");
-    size_t slot_need = 0;
-    for (const Shape& s : shapes)
-      slot_need = std::max<size_t>(slot_need, size_t(s.ctas) * slot_elems_for(b->max_qubits, s.L) * sizeof(float2));
-    if (slot_need) {
-      QVDG_CUDA(cudaMalloc(&b->slots, slot_need));
-      b->slot_bytes = slot_need;
+    // Slots for as many wide circuits as the budget holds, at least one, and
+    // fewer where the device has less memory; the last pass's sums per tile.
+    const uint64_t slot_elems = uint64_t(1) << b->max_qubits;
+    size_t slots = 0, partials = 0;
+    for (const Shape& s : shapes) {
+      slots = std::max(slots, wide_count(b->circuits, order, s.L));
+      partials = std::max<size_t>(partials, plan_work(b->circuits, order, s.L, s.ctas, 1, slot_elems).partials);
+    }
+    if (slots) {
+      slots = std::min<size_t>(slots, std::max<size_t>(1, kSlotBudget / (slot_elems * sizeof(float2))));
+      while (cudaMalloc(&b->slots, slots * slot_elems * sizeof(float2)) != cudaSuccess) {
+        cudaGetLastError();
+        b->slots = nullptr;
+        if (slots == 1) throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate the batch's device memory");
+        slots /= 2;
+      }
+      QVDG_CUDA(cudaMalloc(&b->partials, std::max<size_t>(partials, 1) * sizeof(double)));
     }
     whole.slots = static_cast<float2*>(b->slots);
-    samp.slots = whole.slots;
+    whole.partials = static_cast<double*>(b->partials);
 
     Shape best = shapes[0];
     if (shapes.size() > 1) {
       const auto t0 = std::chrono::steady_clock::now();
       double best_s = 1e300;
       for (const Shape& s : shapes) {
-        const double sec = time_launch(b, shape(samp, s.L, s.threads, s.ctas, b->max_qubits));
+        const double sec =
+            time_launch(b, shape(b, whole, sample, s.L, s.threads, s.ctas, slots, slot_elems, &b->work));
         b->tune_tiles.push_back(uint32_t(s.L));
         b->tune_threads.push_back(uint32_t(s.threads));
         b->tune_seconds.push_back(sec);
@@ -296,13 +325,14 @@ qvdg_batch* batch_create(const qvdg_layered_circuit* circuits, size_t count, con
       }
       b->tune_host_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     }
-    b->launch = shape(whole, best.L, best.threads, best.ctas, b->max_qubits);
-    b->sample = shape(samp, best.L, best.threads, best.ctas, b->max_qubits);
+    b->launch = shape(b, whole, order, best.L, best.threads, best.ctas, slots, slot_elems, &b->work);
 
     // Capture: reset the counter, the persistent launch, results to pinned host memory.
     QVDG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     launch_batch(b->launch, b->stream);
     QVDG_CUDA(cudaMemcpyAsync(b->host_out, b->launch.out, b->outputs * sizeof(double), cudaMemcpyDeviceToHost,
+                              b->stream));
+    QVDG_CUDA(cudaMemcpyAsync(b->host_out + b->outputs, b->launch.status, sizeof(int), cudaMemcpyDeviceToHost,
                               b->stream));
     QVDG_CUDA(cudaStreamEndCapture(b->stream, &b->graph));
     QVDG_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
@@ -334,16 +364,12 @@ void batch_set_gates(qvdg_batch* b, const double* gates, size_t num_matrices) {
   require(num_matrices == b->num_matrices, "expected " + std::to_string(b->num_matrices) + " matrices");
   require(gates != nullptr || num_matrices == 0, "null gates");
   if (num_matrices == 0) return;
-  // Each circuit's records and form (the form follows the new matrices).
-  std::vector<float2> g(num_matrices * kBatchGateSlots);
-  for (BatchCircuit& c : b->circuits)
-    c.form = encode_gates(gates + 8 * c.gates, size_t(c.num_layers) * c.num_qubits, g.data() + kBatchGateSlots * c.gates);
+  // The records and forms follow the new matrices, on the device (encoding
+  // them on the host took most of a call that sets and runs a batch).
   QVDG_CUDA(cudaSetDevice(b->device));
+  QVDG_CUDA(cudaMemcpyAsync(b->matrices, gates, num_matrices * 8 * sizeof(double), cudaMemcpyHostToDevice, b->stream));
+  launch_batch_encode(b->launch, b->matrices, uint32_t(b->circuits.size()), b->stream);
   QVDG_CUDA(cudaStreamSynchronize(b->stream));
-  QVDG_CUDA(cudaMemcpy(const_cast<float2*>(b->launch.gates), g.data(), g.size() * sizeof(float2),
-                       cudaMemcpyHostToDevice));
-  QVDG_CUDA(cudaMemcpy(const_cast<BatchCircuit*>(b->launch.circuits), b->circuits.data(),
-                       b->circuits.size() * sizeof(BatchCircuit), cudaMemcpyHostToDevice));
 }
 
 void batch_run(qvdg_batch* b, double* expect_z, size_t count, double* seconds) {
@@ -359,6 +385,9 @@ void batch_run(qvdg_batch* b, double* expect_z, size_t count, double* seconds) {
   QVDG_CUDA(cudaGetLastError());
   float ms = 0.f;
   QVDG_CUDA(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
+  int gave_up = 0;
+  std::memcpy(&gave_up, b->host_out + b->outputs, sizeof(int));
+  if (gave_up) throw Error(QVDG_ERR_TIMEOUT, "a task of the batch gave up waiting for the tiles it reads");
   if (seconds) *seconds = ms * 1e-3;
   std::memcpy(expect_z, b->host_out, b->outputs * sizeof(double));
 }
