@@ -210,13 +210,38 @@ void apply_program(StateImpl& s, const std::vector<HOp>& ops, const qvdg_options
   if (stats) stats->settings = chosen;
 }
 
-// One op as a single plain pass (StateVector::apply, src/state.rs:181-198).
+// One op as a single plain pass (StateVector::apply, src/state.rs:181-198),
+// without the planner: its matrix through the pinned staging buffer, one
+// launch, one synchronisation (planning, timing events and their reads took
+// two thirds of a small state's 42 us). A state still |0...0> goes through
+// the planner, whose zero-start pass moves little of it.
 void apply_single(StateImpl& s, const HOp& op) {
-  qvdg_options opt;
-  qvdg_default_options(&opt);
-  opt.staged = 0;
-  opt.max_fused_qubits = 1;
-  apply_program(s, {op}, opt, nullptr);
+  if (s.zero_state) {
+    qvdg_options opt;
+    qvdg_default_options(&opt);
+    opt.staged = 0;
+    opt.max_fused_qubits = 1;
+    apply_program(s, {op}, opt, nullptr);
+    return;
+  }
+  Program prog;
+  prog.target = target_of(s);
+  PlannedPass pass;
+  pass.staged = false;
+  pass.ops.push_back(op);
+  const LoweredPass lp = lower_pass(prog.target, pass, prog.cfg, prog.upload);
+  const DeviceUpload dev = upload_program(s, prog, s.work);
+  launch_pass(s, lp, dev);
+  QVDG_CUDA(cudaStreamSynchronize(s.stream));
+}
+
+// src/measure.rs:68-87. A state still |0...0> reads 0 with certainty and
+// stays as it is.
+int measure_qubit(StateImpl& s, uint32_t qubit, double uniform, bool reset) {
+  require(qubit < s.n, "qubit out of range");
+  if (s.zero_state && !(uniform < 0.0)) return 0;
+  s.zero_state = false;
+  return measure(s, s.layout[qubit], uniform, reset);
 }
 
 }  // namespace
@@ -418,35 +443,13 @@ qvdg_status qvdg_probabilities(const qvdg_state* st, double* out, size_t count) 
 
 qvdg_status qvdg_measure(qvdg_state* st, uint32_t qubit, double uniform, int32_t* outcome) {
   return guarded([&] {
-    StateImpl& s = impl(st);
-    require(qubit < s.n, "qubit out of range");
-    // src/measure.rs:68-80
-    const double p1 = std::min(std::max(probability_one(s, s.layout[qubit]), 0.0), 1.0);
-    const bool one = uniform < p1;
-    const double p = one ? p1 : 1.0 - p1;
-    const C keep{1.0 / std::sqrt(p), 0.0}, zero{0.0, 0.0};
-    HOp op;
-    op.targets = {qubit};
-    op.matrix = HMatrix::diagonal(one ? std::vector<C>{zero, keep} : std::vector<C>{keep, zero});
-    op.diagonal = true;
-    apply_single(s, op);
-    if (outcome) *outcome = one ? 1 : 0;
+    const int one = measure_qubit(impl(st), qubit, uniform, false);
+    if (outcome) *outcome = one;
   });
 }
 
 qvdg_status qvdg_reset(qvdg_state* st, uint32_t qubit, double uniform) {
-  int32_t outcome = 0;
-  qvdg_status rc = qvdg_measure(st, qubit, uniform, &outcome);
-  if (rc != QVDG_OK || !outcome) return rc;
-  return guarded([&] {
-    StateImpl& s = impl(st);
-    HOp x;
-    x.targets = {qubit};
-    x.matrix = HMatrix(2);
-    x.matrix.at(0, 1) = {1.0, 0.0};
-    x.matrix.at(1, 0) = {1.0, 0.0};
-    apply_single(s, x);
-  });
+  return guarded([&] { measure_qubit(impl(st), qubit, uniform, true); });
 }
 
 qvdg_status qvdg_sample_unordered(const qvdg_state* st, size_t shots, const double* uniforms, uint64_t* out,

@@ -107,6 +107,9 @@ void launch_scale(StateImpl& s, double factor);
 // ---- measure.cu
 double norm_sqr(StateImpl& s);
 double probability_one(StateImpl& s, uint32_t physical_bit);
+// Measures the bit with the caller's uniform draw and collapses the state on
+// the outcome, which it returns; with `reset` the bit ends in |0>.
+int measure(StateImpl& s, uint32_t physical_bit, double uniform, bool reset);
 // P(bit = 1) for every physical bit, and the total.
 void bit_probabilities(StateImpl& s, std::vector<double>& p1, double& total);
 // Sample and count by classical key (clbits < 64; logical measured qubits);

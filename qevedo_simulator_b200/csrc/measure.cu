@@ -623,24 +623,83 @@ __global__ void __launch_bounds__(kThreads) k_max_diff(const cplx_t<TA>* __restr
 
 unsigned blocks_for(uint64_t items, int threads) { return unsigned(std::max<uint64_t>(1, (items + threads - 1) / threads)); }
 
-// Sum of |a|^2 over the amplitudes with physical bit `bit` set (bit < 0: all
-// of them). One host synchronisation; the sum comes back through mapped
-// pinned memory.
+// The launch of k_sumsq over the amplitudes with physical bit `bit` set
+// (bit < 0: all of them).
+struct SumShape {
+  uint64_t count;
+  int vec_bit, odd;
+  unsigned blocks;
+};
+template <typename T>
+SumShape sum_shape(const StateImpl& s, int bit) {
+  // Bits inside a vector: every vector, complex64's second amplitudes.
+  const int shift = kPerVec<T> == 2 ? 1 : 0;
+  SumShape h{};
+  h.odd = bit >= 0 && bit < shift ? 1 : 0;
+  h.vec_bit = bit < shift ? -1 : bit - shift;
+  h.count = (s.amp_bytes / 16) >> (h.vec_bit < 0 ? 0 : 1);
+  h.blocks = unsigned(std::max<uint64_t>(
+      1, umin64(uint64_t(s.sms) * 8, (h.count + kThreads * kReduceUnroll - 1) / (kThreads * kReduceUnroll))));
+  return h;
+}
+
+// Sum of |a|^2 over those amplitudes. One host synchronisation; the sum
+// comes back through mapped pinned memory.
 template <typename T>
 double sumsq_t(StateImpl& s, int bit) {
   double* h = static_cast<double*>(s.host.get(sizeof(double)));
-  // Bits inside a vector: every vector, complex64's second amplitudes.
-  const int shift = kPerVec<T> == 2 ? 1 : 0;
-  const bool odd = bit >= 0 && bit < shift;
-  const int vec_bit = bit < shift ? -1 : bit - shift;
-  const uint64_t count = (s.amp_bytes / 16) >> (vec_bit < 0 ? 0 : 1);
-  const unsigned blocks = unsigned(std::max<uint64_t>(
-      1, umin64(uint64_t(s.sms) * 8, (count + kThreads * kReduceUnroll - 1) / (kThreads * kReduceUnroll))));
-  double* d = static_cast<double*>(s.work.get(blocks * sizeof(double)));
-  k_sumsq<T><<<blocks, kThreads, 0, s.stream>>>(static_cast<const float4*>(s.amp), count, vec_bit, odd ? 1 : 0, d);
+  const SumShape shape = sum_shape<T>(s, bit);
+  double* d = static_cast<double*>(s.work.get(shape.blocks * sizeof(double)));
+  k_sumsq<T><<<shape.blocks, kThreads, 0, s.stream>>>(static_cast<const float4*>(s.amp), shape.count, shape.vec_bit,
+                                                      shape.odd, d);
   QVDG_LAUNCH_CHECK();
-  k_sum_columns<<<1, kThreads, 0, s.stream>>>(d, int(blocks), 1, h);
+  k_sum_columns<<<1, kThreads, 0, s.stream>>>(d, int(shape.blocks), 1, h);
   QVDG_LAUNCH_CHECK();
+  QVDG_CUDA(cudaStreamSynchronize(s.stream));
+  return *h;
+}
+
+// A measurement's outcome from the partial sums of P(1) (src/measure.rs:68-80)
+// and the gate that collapses the state on it, as the gate kernels read it:
+// the diagonal (keep, 0) or (0, keep), or, for a reset, the matrix that also
+// moves the kept amplitude to |0>.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_outcome(const double* __restrict__ partials, int count, double uniform,
+                                                      int reset, cplx_t<T>* __restrict__ gate,
+                                                      int* __restrict__ outcome) {
+  __shared__ double red[32];
+  double t = 0.0;
+  for (int i = threadIdx.x; i < count; i += kThreads) t += partials[i];
+  t = block_sum(t, red);
+  if (threadIdx.x) return;
+  double p1 = t < 0.0 ? 0.0 : t;
+  p1 = 1.0 < p1 ? 1.0 : p1;
+  const bool one = uniform < p1;
+  const cplx_t<T> keep = make_c<T>(T(1.0 / sqrt(one ? p1 : 1.0 - p1)), T(0)), zero = make_c<T>(T(0), T(0));
+  gate[0] = one ? zero : keep;
+  gate[1] = one ? keep : zero;
+  if (reset) gate[2] = gate[3] = zero;
+  *outcome = one ? 1 : 0;
+}
+
+// P(1) of the bit, the outcome and the collapse as three launches and one
+// synchronisation.
+template <typename T>
+int measure_t(StateImpl& s, uint32_t bit, double uniform, bool reset) {
+  int* h = static_cast<int*>(s.host.get(sizeof(int)));
+  const SumShape shape = sum_shape<T>(s, int(bit));
+  char* w = static_cast<char*>(s.work.get(256 + shape.blocks * sizeof(double)));
+  cplx_t<T>* gate = reinterpret_cast<cplx_t<T>*>(w);
+  double* d = reinterpret_cast<double*>(w + 256);
+  k_sumsq<T><<<shape.blocks, kThreads, 0, s.stream>>>(static_cast<const float4*>(s.amp), shape.count, shape.vec_bit,
+                                                      shape.odd, d);
+  QVDG_LAUNCH_CHECK();
+  k_outcome<T><<<1, kThreads, 0, s.stream>>>(d, int(shape.blocks), uniform, reset ? 1 : 0, gate, h);
+  QVDG_LAUNCH_CHECK();
+  PlainGate g;
+  g.diagonal = !reset;
+  g.targets = {bit};
+  launch_plain_gate(s, g, gate);
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
   return *h;
 }
@@ -973,6 +1032,11 @@ void bit_probabilities(StateImpl& s, std::vector<double>& p1, double& total) {
 
 double probability_one(StateImpl& s, uint32_t physical_bit) {
   return s.bits == 32 ? sumsq_t<float>(s, int(physical_bit)) : sumsq_t<double>(s, int(physical_bit));
+}
+
+int measure(StateImpl& s, uint32_t physical_bit, double uniform, bool reset) {
+  return s.bits == 32 ? measure_t<float>(s, physical_bit, uniform, reset)
+                      : measure_t<double>(s, physical_bit, uniform, reset);
 }
 
 void probabilities(StateImpl& s, double* out_host) {
