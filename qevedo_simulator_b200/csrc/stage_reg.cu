@@ -15,9 +15,13 @@
 // FMAs per amplitude (real and RX-type matrices take the cheaper forms), a
 // +-1 diagonal (CZ and the like) only toggles sign bits.
 //
-// Tiles are double-buffered: the next tile's 16-byte cp.async copies are in
-// flight while the current one is computed, and a finished tile is stored
-// from shared memory straight to HBM.
+// A tile's 16-byte cp.async copies and its stores back to HBM are covered by
+// another CTA's computation: two CTAs per SM, one tile buffer each. What
+// bounds the kernel is the latency of each gate's chain (its record, then
+// its matrix, then the arithmetic), so warps count for more than a second
+// buffer: one CTA with two buffers left a complex128 stage 8 warps per SM.
+// Only a pass whose gate data leave no room for a second CTA keeps two
+// buffers, the next tile's copies in flight while the current is computed.
 
 #include <cuda_runtime.h>
 
@@ -51,19 +55,17 @@ struct RegPassHdr {
   uint16_t pair;        // g[0] == 0: registers j, j^1 are one 16-byte slot (complex64)
   uint32_t first_gate;  // index of the pass's first gate
   uint32_t pad;
-  uint16_t off[16];     // tile element offset of register j (j deposited over g)
 };
-static_assert(sizeof(RegPassHdr) == 48, "header layout");
+static_assert(sizeof(RegPassHdr) == 16, "header layout");
 
 // Dispatch codes of the register kernel (one switch per gate).
 enum : uint16_t {
   kOpDense1 = 0,         // + 4 * spec + target register bit (16 codes), no register controls
   kOpDense1Masked = 16,  // any matrix, register controls
-  kOpDense2 = 17,        // + index of (t0, t1) in (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
-  kOpDense2Masked = 23,
-  kOpSign2 = 24,
-  kOpSign = 25,
-  kOpPhase = 26,
+  kOpDense2 = 17,
+  kOpSign2 = 18,
+  kOpSign = 19,
+  kOpPhase = 20,
 };
 
 struct RegGate {
@@ -173,37 +175,30 @@ __device__ __forceinline__ void apply1_bit(cplx_t<T> (&a)[16], int tb, const cpl
   }
 }
 
-// Dense 2-qubit gate on register bits B0 < B1 (matrix bit 0 <-> B0).
-template <typename T, int B0, int B1, bool MASKED>
-__device__ __forceinline__ void apply2(cplx_t<T> (&a)[16], const cplx_t<T>* m, uint32_t pmask) {
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    if (j & ((1 << B0) | (1 << B1))) continue;
-    const int i[4] = {j, j | (1 << B0), j | (1 << B1), j | (1 << B0) | (1 << B1)};
-    cplx_t<T> x[4] = {a[i[0]], a[i[1]], a[i[2]], a[i[3]]};
-    cplx_t<T> y[4];
+// Dense 2-qubit gate on the subcube at `place` in the tile, on the register
+// bits whose byte distances are b0 and b1 (the others c0 and c1), for the
+// groups active in `groups` (bit k: the others' values). It works on the
+// thread's own subcube in shared memory, one group at a time: six pairs of
+// target bits as code on the registers would take more of them than two CTAs
+// per SM leave.
+template <typename T>
+__device__ __noinline__ void apply2(unsigned char* tile, uint32_t place, uint32_t b0, uint32_t b1, uint32_t c0,
+                                    uint32_t c1, uint32_t groups, const cplx_t<T>* m) {
+#pragma unroll 1
+  for (uint32_t k = 0; k < 4; ++k) {
+    if (!((groups >> k) & 1u)) continue;
+    const uint32_t o = place ^ ((k & 1u) ? c0 : 0u) ^ ((k & 2u) ? c1 : 0u);
+    cplx_t<T>* p[4] = {reinterpret_cast<cplx_t<T>*>(tile + o), reinterpret_cast<cplx_t<T>*>(tile + (o ^ b0)),
+                       reinterpret_cast<cplx_t<T>*>(tile + (o ^ b1)),
+                       reinterpret_cast<cplx_t<T>*>(tile + (o ^ b0 ^ b1))};
+    const cplx_t<T> x[4] = {*p[0], *p[1], *p[2], *p[3]};
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       cplx_t<T> acc = make_c<T>(T(0), T(0));
 #pragma unroll
       for (int c = 0; c < 4; ++c) cmac<T>(acc, m[r * 4 + c], x[c]);
-      y[r] = acc;
+      *p[r] = acc;
     }
-    const bool on = !MASKED || ((pmask >> j) & 1u);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) a[i[r]] = on ? y[r] : x[r];
-  }
-}
-
-template <typename T, bool MASKED>
-__device__ __forceinline__ void apply2_any(cplx_t<T> (&a)[16], const RegGate& g, const cplx_t<T>* m) {
-  switch (g.t0 * 4 + g.t1) {
-    case 1: apply2<T, 0, 1, MASKED>(a, m, g.pmask); break;
-    case 2: apply2<T, 0, 2, MASKED>(a, m, g.pmask); break;
-    case 3: apply2<T, 0, 3, MASKED>(a, m, g.pmask); break;
-    case 6: apply2<T, 1, 2, MASKED>(a, m, g.pmask); break;
-    case 7: apply2<T, 1, 3, MASKED>(a, m, g.pmask); break;
-    default: apply2<T, 2, 3, MASKED>(a, m, g.pmask); break;
   }
 }
 
@@ -231,6 +226,10 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
                                   const unsigned char* blob, int L, uint64_t tile_base) {
   using C2 = cplx_t<T>;
   const uint32_t nsub = 1u << (L - 4);
+  uint32_t bit[4];  // byte distance (swizzled) of each register bit
+#pragma unroll
+  for (int i = 0; i < 4; ++i) bit[i] = reg_swz(1u << h.g[i]) * uint32_t(sizeof(C2));
+  const uint32_t first = h.first_gate, last = first + h.num_gates;
   for (uint32_t s = threadIdx.x; s < nsub; s += blockDim.x) {
     uint32_t eb = s;
 #pragma unroll
@@ -238,31 +237,59 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
       const uint32_t p = h.g[i];
       eb = ((eb >> p) << (p + 1)) | (eb & ((1u << p) - 1u));
     }
+    // Register j at the subcube's place XOR the places of j's bits (the
+    // swizzle is XOR-linear).
+    unsigned char* const bytes = reinterpret_cast<unsigned char*>(tile);
+    const uint32_t place = reg_swz(eb) * uint32_t(sizeof(C2));
+    auto at = [&](int j) {
+      uint32_t o = place;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if ((j >> i) & 1) o ^= bit[i];
+      return bytes + o;
+    };
     C2 a[16];
-    if (sizeof(C2) == 8 && h.pair) {
+    auto fetch = [&] {
+      if (sizeof(C2) == 8 && h.pair) {
 #pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        const float4 v = *reinterpret_cast<const float4*>(tile + reg_swz(eb | h.off[j]));
-        a[j] = make_c<T>(T(v.x), T(v.y));
-        a[j + 1] = make_c<T>(T(v.z), T(v.w));
+        for (int j = 0; j < 16; j += 2) {
+          const float4 v = *reinterpret_cast<const float4*>(at(j));
+          a[j] = make_c<T>(T(v.x), T(v.y));
+          a[j + 1] = make_c<T>(T(v.z), T(v.w));
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) a[j] = *reinterpret_cast<const C2*>(at(j));
       }
-    } else {
+    };
+    auto save = [&] {
+      if (sizeof(C2) == 8 && h.pair) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) a[j] = tile[reg_swz(eb | h.off[j])];
-    }
+        for (int j = 0; j < 16; j += 2)
+          *reinterpret_cast<float4*>(at(j)) =
+              make_float4(float(a[j].x), float(a[j].y), float(a[j + 1].x), float(a[j + 1].y));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) *reinterpret_cast<C2*>(at(j)) = a[j];
+      }
+    };
+    fetch();
     // Bits a sign gate reads outside the registers: the tile's global bits
     // and the subcube's tile bits (at 48 and up).
     const uint64_t where = tile_base | (uint64_t(eb) << 48);
-    for (uint32_t gi = h.first_gate; gi < h.first_gate + h.num_gates; ++gi) {
+    // The next gate's record is read while the present one is applied.
+    uint4 ahead = *reinterpret_cast<const uint4*>(&gates[first]);
+    for (uint32_t gi = first; gi < last; ++gi) {
       const RegGate& g = gates[gi];
-      const uint4 hot = *reinterpret_cast<const uint4*>(&g);
+      const uint4 hot = ahead;
+      ahead = *reinterpret_cast<const uint4*>(&gates[gi + 1 < last ? gi + 1 : gi]);
       const uint32_t op = hot.x & 0xffffu, pmask = hot.x >> 16;
       const uint32_t t0 = hot.y & 0xffu, t1 = (hot.y >> 8) & 0xffu;
       if ((hot.y >> 16) & 0xffu)
         if ((tile_base & g.gcm) != g.gcv || (eb & g.lcm) != g.lcv) continue;
       const unsigned char* data = blob + hot.z;
       const C2* m = reinterpret_cast<const C2*>(data);
-      switch (op >= kOpSign2 ? op : (op >= kOpDense2 ? 1u : 0u)) {
+      switch (op >= kOpSign2 ? op : (op == kOpDense2 ? 1u : 0u)) {
         case 0:  // dense 1-qubit
           if (op == kOpDense1Masked) {
             apply1_bit<T, kSpecGeneral, true>(a, int(t0), m, pmask);
@@ -277,14 +304,17 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
           }
           break;
         case 1: {  // dense 2-qubit
-          RegGate gg;
-          gg.t0 = uint8_t(t0);
-          gg.t1 = uint8_t(t1);
-          gg.pmask = uint16_t(pmask);
-          if (op == kOpDense2Masked)
-            apply2_any<T, true>(a, gg, m);
-          else
-            apply2_any<T, false>(a, gg, m);
+          save();
+          // The register bits that are not targets, and the groups (by their
+          // values) that are active.
+          const uint32_t rest = 15u & ~((1u << t0) | (1u << t1));
+          const uint32_t r0 = __ffs(rest) - 1u, r1 = 31u - __clz(rest);
+          uint32_t groups = 0;
+          for (uint32_t k = 0; k < 4; ++k)
+            groups |= ((pmask >> (((k & 1u) << r0) | ((k >> 1) << r1))) & 1u) << k;
+          auto dist = [&](uint32_t i) { return i == 0 ? bit[0] : (i == 1 ? bit[1] : (i == 2 ? bit[2] : bit[3])); };
+          apply2<T>(bytes, place, dist(t0), dist(t1), dist(r0), dist(r1), groups, m);
+          fetch();
           break;
         }
         case kOpSign2: {
@@ -306,15 +336,7 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
         }
       }
     }
-    if (sizeof(C2) == 8 && h.pair) {
-#pragma unroll
-      for (int j = 0; j < 16; j += 2)
-        *reinterpret_cast<float4*>(tile + reg_swz(eb | h.off[j])) =
-            make_float4(float(a[j].x), float(a[j].y), float(a[j + 1].x), float(a[j + 1].y));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) tile[reg_swz(eb | h.off[j])] = a[j];
-    }
+    save();
   }
   __syncthreads();
 }
@@ -327,8 +349,9 @@ constexpr int reg_threads() {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(reg_threads<T>(), 1)
-    k_stage_reg(cplx_t<T>* __restrict__ psi, const TileGeom geo, const unsigned char* __restrict__ blob_all) {
+__global__ void __launch_bounds__(reg_threads<T>(), 2)
+    k_stage_reg(cplx_t<T>* __restrict__ psi, const TileGeom geo, const unsigned char* __restrict__ blob_all,
+                int buffers) {
   using C2 = cplx_t<T>;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint8_t tile_bits[48];
@@ -336,8 +359,8 @@ __global__ void __launch_bounds__(reg_threads<T>(), 1)
   const int tid = threadIdx.x;
   const int L = geo.L, B = geo.B;
   const uint32_t n_el = 1u << L;
-  C2* const buf0 = reinterpret_cast<C2*>(smem);  // tiles at buf0 and buf0 + n_el
-  unsigned char* blob = smem + 2 * sizeof(C2) * n_el;
+  C2* const buf0 = reinterpret_cast<C2*>(smem);  // tiles at buf0 (and buf0 + n_el)
+  unsigned char* blob = smem + size_t(buffers) * sizeof(C2) * n_el;
 
   for (int i = tid; i < 48; i += blockDim.x) tile_bits[i] = geo.tile_bits[i];
   {
@@ -379,13 +402,20 @@ __global__ void __launch_bounds__(reg_threads<T>(), 1)
 
   uint64_t t = blockIdx.x;
   int cur = 0;
-  if (t < geo.num_tiles) issue(t, buf0);
+  const int other = buffers - 1;  // 0: one buffer
+  if (t < geo.num_tiles && other) issue(t, buf0);
   cp_async_commit();
   for (; t < geo.num_tiles; t += gridDim.x) {
     const uint64_t next = t + gridDim.x;
-    if (next < geo.num_tiles) issue(next, buf0 + (cur ^ 1) * n_el);
-    cp_async_commit();
-    cp_async_wait1();
+    if (!other) {
+      issue(t, buf0);
+      cp_async_commit();
+      cp_async_wait0();
+    } else {
+      if (next < geo.num_tiles) issue(next, buf0 + (cur ^ 1) * n_el);
+      cp_async_commit();
+      cp_async_wait1();
+    }
     __syncthreads();
     C2* tile = buf0 + cur * n_el;
     const uint64_t base = insert_zeros(t, tile_bits, L);
@@ -395,7 +425,7 @@ __global__ void __launch_bounds__(reg_threads<T>(), 1)
       *reinterpret_cast<uint4*>(psi + phys(base, e)) = *reinterpret_cast<const uint4*>(tile + reg_swz(e));
     }
     __syncthreads();
-    cur ^= 1;
+    cur ^= other;
   }
   cp_async_wait0();
 }
@@ -575,12 +605,6 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
         reg_of[b] = gi++;
       }
     h.pair = h.g[0] == 0 ? 1 : 0;
-    for (uint32_t j = 0; j < 16; ++j) {
-      uint32_t o = 0;
-      for (int i = 0; i < 4; ++i)
-        if ((j >> i) & 1u) o |= 1u << h.g[i];
-      h.off[j] = uint16_t(o);
-    }
     h.first_gate = uint32_t(gates.size());
     h.num_gates = uint16_t(ps.ops.size());
     std::memcpy(blob.data() + pi * sizeof(RegPassHdr), &h, sizeof(h));
@@ -692,8 +716,7 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
       if (g.kind == kRegDense1)
         g.op = g.pmask == 0xffffu ? uint16_t(kOpDense1 + 4 * g.spec + g.t0) : uint16_t(kOpDense1Masked);
       else if (g.kind == kRegDense2)
-        g.op = g.pmask == 0xffffu ? uint16_t(kOpDense2 + (g.t0 == 0 ? g.t1 - 1 : (g.t0 == 1 ? g.t1 + 1 : 5)))
-                                  : uint16_t(kOpDense2Masked);
+        g.op = kOpDense2;
       else if (g.kind == kRegSign2)
         g.op = kOpSign2;
       else if (g.kind == kRegSign)
@@ -704,7 +727,7 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
       fixes.push_back(fx);
     }
   }
-  const size_t gates_off = blob.size();  // a multiple of 48, so of 16
+  const size_t gates_off = blob.size();  // a multiple of 16
   const size_t data_base = gates_off + gates.size() * sizeof(RegGate);
   for (const Fix& fx : fixes) {
     gates[fx.gate].data = uint32_t(data_base + fx.data_off);
@@ -729,27 +752,27 @@ size_t register_blob_budget() { return kRegBlobBudget; }
 
 void launch_stage_reg(StateImpl& s, const LoweredPass& lp, const DeviceUpload& dev) {
   const size_t tile_bytes = (s.bits == 32 ? 8 : 16) << lp.geo.L;
-  const size_t smem = 2 * tile_bytes + lp.geo.tc_bytes;
+  // Two CTAs per SM where they fit beside each other (227 KB of shared
+  // memory, a few hundred bytes of each CTA static, 1 KB reserved).
+  const int buffers = tile_bytes + lp.geo.tc_bytes + 2048 <= 227 * 1024 / 2 ? 1 : 2;
+  const size_t smem = buffers * tile_bytes + lp.geo.tc_bytes;
   // One thread per register subcube, at least one full warp (the set-up
   // loops are strided, so any count works).
   const int cap = s.bits == 32 ? reg_threads<float>() : reg_threads<double>();
   const int threads = std::max(32, std::min(cap, 1 << (lp.geo.L - 4)));
-  const uint64_t grid = std::min<uint64_t>(lp.geo.num_tiles, uint64_t(s.sms));
-  if (s.bits == 32) {
-    static size_t configured = 0;
+  const uint64_t grid = std::min<uint64_t>(lp.geo.num_tiles, uint64_t(s.sms) * (buffers == 1 ? 2 : 1));
+  auto launch = [&](auto* psi, auto kernel, size_t& configured) {
     if (smem > configured) {
-      QVDG_CUDA(cudaFuncSetAttribute(k_stage_reg<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      QVDG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
       configured = smem;
     }
-    k_stage_reg<float><<<unsigned(grid), threads, smem, s.stream>>>(static_cast<float2*>(s.amp), lp.geo, dev.tc);
-  } else {
-    static size_t configured = 0;
-    if (smem > configured) {
-      QVDG_CUDA(cudaFuncSetAttribute(k_stage_reg<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-      configured = smem;
-    }
-    k_stage_reg<double><<<unsigned(grid), threads, smem, s.stream>>>(static_cast<double2*>(s.amp), lp.geo, dev.tc);
-  }
+    kernel<<<unsigned(grid), threads, smem, s.stream>>>(psi, lp.geo, dev.tc, buffers);
+  };
+  static size_t configured[2] = {0, 0};
+  if (s.bits == 32)
+    launch(static_cast<float2*>(s.amp), k_stage_reg<float>, configured[0]);
+  else
+    launch(static_cast<double2*>(s.amp), k_stage_reg<double>, configured[1]);
   QVDG_LAUNCH_CHECK();
 }
 
