@@ -654,7 +654,9 @@ qvdg_status qvdg_sample_counts(const qvdg_state* st, size_t shots, const double*
       require(measure_qubits[i] < s.n, "measured qubit out of range");
       require(measure_clbits[i] < 64, "classical bits beyond 63 are not supported by device counting");
     }
-    for (size_t i = 0; i < shots; ++i) require(uniforms[i] >= 0.0 && uniforms[i] < 1.0, "uniforms must be in [0, 1)");
+    bool in_range = true;  // checked in one go: a message per shot took longer than the sampling
+    for (size_t i = 0; i < shots; ++i) in_range &= uniforms[i] >= 0.0 && uniforms[i] < 1.0;
+    require(in_range, "uniforms must be in [0, 1)");
     std::vector<uint64_t> k, c;
     sample_counts(s, shots, uniforms, measure_qubits, measure_clbits, num_measures, k, c);
     if (num_keys) *num_keys = k.size();

@@ -132,8 +132,10 @@ double max_abs_diff(StateImpl& a, StateImpl& b);
 
 // ---- sort.cu
 // Ascending stable LSD radix sort of `count` 64-bit keys in place (`tmp` has
-// room for `count` keys). `work` provides temporary device memory.
-void radix_sort_u64(uint64_t* keys, uint64_t* tmp, size_t count, DeviceScratch& work, cudaStream_t stream);
+// room for `count` keys), all below 2^bits. `work` provides temporary device
+// memory.
+void radix_sort_u64(uint64_t* keys, uint64_t* tmp, size_t count, DeviceScratch& work, cudaStream_t stream,
+                    int bits = 64);
 
 // ---- mlp.cu (learned cost model network)
 qvdg_mlp* mlp_create(uint32_t inputs, uint32_t hidden, uint64_t seed);

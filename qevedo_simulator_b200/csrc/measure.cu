@@ -11,11 +11,11 @@
 //     src/measure.rs:13 and src/simd.rs:71-97), in physical index order;
 //   - p = re*re + im*im in f64 without contraction (__dmul_rn/__dadd_rn);
 //   - each chunk sum is one sequential left fold in index order (one lane
-//     owns a chunk; a warp streams 32 chunks' data through shared memory);
+//     owns a chunk);
 //   - the chunk prefix is sequential; targets = u * total are sorted in f64
 //     total order; bounds are partition points of the prefix;
-//   - the walk adds nonzero p in index order from prefix[chunk] and emits an
-//     index while target < cumulative, pads with the last nonzero index.
+//   - the walk adds p in index order from prefix[chunk] and emits the first
+//     index whose running sum exceeds the target, or the last nonzero index.
 
 #include <cuda_runtime.h>
 
@@ -239,32 +239,13 @@ __global__ void k_probs(const cplx_t<T>* __restrict__ psi, double* __restrict__ 
 }
 
 // ---------------------------------------------------------------- sampler
-// Pass 1: sequential f64 sum of p over each chunk (src/measure.rs:110-118).
-// A warp owns 32 consecutive chunks and lane c folds chunk c, in index
-// order. The chunks stream through shared memory in windows of 256 bytes
-// per chunk, copied with cp.async (16 bytes a lane, lanes 0-15 on one chunk
-// and 16-31 on the next) kSumStages - 1 windows ahead of the fold, so each
-// warp keeps 16 KB of loads in flight. Rows are padded by 16 bytes: the
-// fold's 16-byte reads (one row per lane) then hit distinct banks.
-constexpr int kSumStages = 3;
-constexpr int kSumWindow = 256;             // bytes per chunk per window
-constexpr int kSumRow = kSumWindow + 16;    // padded row in shared memory
-constexpr int kSumStageBytes = 32 * kSumRow;
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                   static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
-               "l"(gmem)
-               : "memory");
+__device__ __forceinline__ void cp_async16_s(uint32_t smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ void cp_async16_s(uint32_t smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
 }
 
 // prob<T> in fewer instructions: for a complex64 amplitude re*re and im*im
@@ -280,96 +261,128 @@ __device__ __forceinline__ double prob_fast(const cplx_t<T>& a) {
   }
 }
 
-// p of the amplitudes of one 16-byte read, in index order.
+// Sequential f64 folds of p over chunks, in index order: each chunk's sum
+// from +0 (src/measure.rs:110-118), or, with `checkpoints`, the running sum
+// from prefix[chunk] of the chunks listed in `active`, written down after
+// every kCheckpoint amplitudes (the walk of src/measure.rs:134-167 without
+// its emissions).
+//
+// The order of the additions is fixed (bit-exactness), so a chunk's chain of
+// 32768 (complex64) dependent additions, 8.4 cycles each, bounds a state of
+// few chunks (0.15 ms) and HBM one of many. Warp 0 does nothing but the
+// chains, lane c folding chunk c of the block's kFoldChunks; the other warps
+// turn amplitudes into probabilities beside it (the f32 to f64 conversions,
+// 16 a cycle and SM, took twice the chain's time when the folding lanes did
+// them: 0.63 ms for the sums of 26 qubits). Amplitudes come in windows of 512
+// bytes a chunk, copied with cp.async kFoldStages - 1 windows ahead;
+// probabilities go through two buffers, rows padded by 16 bytes so that the
+// chains' 16-byte reads (one row per lane) hit distinct banks. One block
+// barrier a window. Past the state's end the windows hold zeros: adding +0
+// changes nothing.
+constexpr int kFoldChunks = 16;
+constexpr int kFoldWarps = 5;    // the chains' and four that convert
+constexpr int kFoldStages = 4;
+constexpr int kFoldWindow = 512;  // bytes per chunk per window
+constexpr int kCheckpoint = 256;  // amplitudes
+
 template <typename T>
-__device__ __forceinline__ void probs16(const float4& v, double* p) {
-  if constexpr (sizeof(T) == 4) {
-    p[0] = prob_fast<float>(make_float2(v.x, v.y));
-    p[1] = prob_fast<float>(make_float2(v.z, v.w));
-  } else {
-    p[0] = prob<double>(*reinterpret_cast<const double2*>(&v));
-  }
+constexpr int fold_smem() {
+  constexpr int amps = kFoldWindow / int(sizeof(cplx_t<T>));
+  return kFoldStages * kFoldChunks * kFoldWindow + 2 * kFoldChunks * (amps * 8 + 16);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(32) k_chunk_sums(const cplx_t<T>* __restrict__ psi, uint64_t len,
-                                                   uint64_t chunk_len, uint64_t nchunks,
-                                                   double* __restrict__ sums) {
-  constexpr int kAmp = int(sizeof(cplx_t<T>));  // 8 or 16 bytes
-  constexpr int kPerWin = kSumWindow / kAmp;     // amplitudes per chunk per window
-  constexpr int kPerRead = 16 / kAmp;            // amplitudes per 16-byte read
-  __shared__ __align__(16) unsigned char sbuf[kSumStages][kSumStageBytes];
-  const int lane = threadIdx.x;
-  const uint64_t chunk0 = uint64_t(blockIdx.x) * 32;
-  if (chunk0 >= nchunks) return;
-  const int live = int(umin64(32, nchunks - chunk0));
-  // Windows of the warp's first chunk (no later chunk is longer).
-  const uint64_t windows = (umin64(chunk_len, len - chunk0 * chunk_len) + kPerWin - 1) / kPerWin;
-  const unsigned char* src0 = reinterpret_cast<const unsigned char*>(psi);
-  const int half = lane >> 4, sub = lane & 15;
-  // Every chunk of the warp whole (all but a state shorter than one chunk):
-  // a lane's copies are then one pointer and one shared address apart.
-  const bool whole = (chunk0 + uint64_t(live)) * chunk_len <= len;
-  const unsigned char* lane_src = src0 + (chunk0 + uint64_t(half)) * chunk_len * kAmp + sub * 16;
-  const uint64_t lane_step = 2 * chunk_len * kAmp;
-  const uint32_t lane_dst = static_cast<uint32_t>(__cvta_generic_to_shared(&sbuf[0][half * kSumRow + sub * 16]));
-  auto issue = [&](uint64_t w, int stage) {
-    if (whole) {
-      const unsigned char* src = lane_src + w * kSumWindow;
-      uint32_t dst = lane_dst + uint32_t(stage) * kSumStageBytes;
-      if (live == 32) {
+__global__ void __launch_bounds__(32 * kFoldWarps) k_fold(const cplx_t<T>* __restrict__ psi, uint64_t len,
+                                                          uint64_t chunk_len, uint64_t count,
+                                                          const uint32_t* __restrict__ active,
+                                                          const double* __restrict__ prefix,
+                                                          double* __restrict__ out, int checkpoints) {
+  constexpr int kAmp = int(sizeof(cplx_t<T>));
+  constexpr int kAmps = kFoldWindow / kAmp;      // per chunk per window
+  constexpr int kRow = kAmps * 8 + 16;           // bytes of a row of probabilities
+  constexpr int kVecs = kFoldWindow / 16;        // 16-byte vectors per chunk per window
+  constexpr int kWorkers = 32 * (kFoldWarps - 1);
+  constexpr int kEach = kFoldChunks * kVecs / kWorkers;
+  extern __shared__ __align__(16) unsigned char smem[];
+  unsigned char* raw = smem;                                                // [stage][chunk][window]
+  unsigned char* rows = smem + kFoldStages * kFoldChunks * kFoldWindow;     // [2][chunk][row]
+  __shared__ uint64_t first[kFoldChunks];
+  const uint64_t item0 = uint64_t(blockIdx.x) * kFoldChunks;
+  const int live = int(umin64(kFoldChunks, count - item0));
+  if (threadIdx.x < uint32_t(kFoldChunks))
+    first[threadIdx.x] = int(threadIdx.x) < live
+                             ? (active ? uint64_t(active[item0 + threadIdx.x]) : item0 + threadIdx.x) * chunk_len
+                             : len;
+  __syncthreads();
+  const uint64_t windows = (umin64(chunk_len, len) + kAmps - 1) / kAmps;
+  const int worker = int(threadIdx.x) - 32;
+  const unsigned char* bytes = reinterpret_cast<const unsigned char*>(psi);
+  const uint64_t end_b = len * kAmp;
+  const uint32_t raw_s = static_cast<uint32_t>(__cvta_generic_to_shared(raw));
+  auto issue = [&](uint64_t w) {
+    if (w < windows)
 #pragma unroll
-        for (int r = 0; r < 16; ++r) cp_async16_s(dst + uint32_t(r) * 2 * kSumRow, src + r * lane_step);
-      } else {
-        for (int r = 0; 2 * r + half < live; ++r) cp_async16_s(dst + uint32_t(r) * 2 * kSumRow, src + r * lane_step);
+      for (int i = 0; i < kEach; ++i) {
+        const int v = worker + i * kWorkers, c = v / kVecs, o = v % kVecs;
+        const uint64_t at = (first[c] * kAmp) + w * kFoldWindow + uint64_t(o) * 16;
+        const uint32_t dst = uint32_t(int(w % kFoldStages) * kFoldChunks * kFoldWindow + v * 16);
+        if (at < end_b)
+          cp_async16_s(raw_s + dst, bytes + at);
+        else
+          *reinterpret_cast<float4*>(raw + dst) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      return;
-    }
-    for (int r = 0; r < 16; ++r) {
-      const int c = 2 * r + half;
-      if (c >= live) break;
-      const uint64_t chunk = chunk0 + c;
-      const uint64_t end_b = umin64(chunk_len, len - chunk * chunk_len) * kAmp;
-      const uint64_t off_b = w * kSumWindow + uint64_t(sub) * 16;
-      unsigned char* dst = &sbuf[stage][c * kSumRow + sub * 16];
-      const unsigned char* src = src0 + chunk * chunk_len * kAmp + off_b;
-      if (off_b + 16 <= end_b)
-        cp_async16(dst, src);
-      else if (off_b < end_b)  // one complex64 left (a state of one amplitude)
-        *reinterpret_cast<cplx_t<T>*>(dst) = *reinterpret_cast<const cplx_t<T>*>(src);
+    cp_async_commit();
+  };
+  // Window w's probabilities into its row buffer (this worker's own copies).
+  auto convert = [&](uint64_t w) {
+    cp_async_wait<kFoldStages - 2>();
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) {
+      const int v = worker + i * kWorkers, c = v / kVecs, o = v % kVecs;
+      const float4 x = *reinterpret_cast<const float4*>(raw + int(w % kFoldStages) * kFoldChunks * kFoldWindow + v * 16);
+      unsigned char* row = rows + (int(w & 1) * kFoldChunks + c) * kRow;
+      if constexpr (sizeof(T) == 4) {
+        const double p0 = prob_fast<float>(make_float2(x.x, x.y)), p1 = prob_fast<float>(make_float2(x.z, x.w));
+        *reinterpret_cast<double2*>(row + o * 16) = make_double2(p0, p1);
+      } else {
+        *reinterpret_cast<double*>(row + o * 8) = prob_fast<double>(*reinterpret_cast<const double2*>(&x));
+      }
     }
   };
-  for (int st = 0; st < kSumStages - 1; ++st) {
-    if (uint64_t(st) < windows) issue(uint64_t(st), st);
-    cp_async_commit();
-  }
+  const int lane = int(threadIdx.x);
   double s = 0.0;
-  const uint64_t my_end = lane < live ? umin64(chunk_len, len - (chunk0 + lane) * chunk_len) : 0;
-  for (uint64_t w = 0; w < windows; ++w) {
-    const uint64_t ahead = w + kSumStages - 1;
-    if (ahead < windows) issue(ahead, int(ahead % kSumStages));
-    cp_async_commit();
-    cp_async_wait<kSumStages - 1>();  // window w has landed
-    __syncwarp();
-    const uint64_t pos = w * kPerWin;
-    if (pos < my_end) {
-      const float4* row = reinterpret_cast<const float4*>(&sbuf[w % kSumStages][lane * kSumRow]);
-      const uint64_t n = umin64(kPerWin, my_end - pos);
-      if (n == uint64_t(kPerWin)) {
-        // The probabilities first (independent of the sum), then the chain.
-        double p[kPerWin];
-#pragma unroll
-        for (int j = 0; j < kPerWin / kPerRead; ++j) probs16<T>(row[j], p + j * kPerRead);
-#pragma unroll
-        for (int j = 0; j < kPerWin; ++j) s = __dadd_rn(s, p[j]);
-      } else {
-        const cplx_t<T>* amps = reinterpret_cast<const cplx_t<T>*>(row);
-        for (uint64_t j = 0; j < n; ++j) s = __dadd_rn(s, prob_fast<T>(amps[j]));
-      }
-    }
-    __syncwarp();
+  double* mine = nullptr;
+  if (worker >= 0) {
+    for (int w = 0; w < kFoldStages - 1; ++w) issue(uint64_t(w));
+    convert(0);
+  } else if (checkpoints && lane < live) {
+    s = prefix[active[item0 + lane]];
+    mine = out + (item0 + lane) * (chunk_len / kCheckpoint);
   }
-  if (lane < live) sums[chunk0 + lane] = s;
+  __syncthreads();
+  for (uint64_t w = 0; w < windows; ++w) {
+    if (worker >= 0) {
+      issue(w + kFoldStages - 1);
+      if (w + 1 < windows) convert(w + 1);
+    } else if (lane < kFoldChunks) {
+      const double2* row = reinterpret_cast<const double2*>(rows + (int(w & 1) * kFoldChunks + lane) * kRow);
+#pragma unroll
+      for (int j = 0; j < kAmps / 2; ++j) {
+        const double2 p = row[j];
+        s = __dadd_rn(s, p.x);
+        s = __dadd_rn(s, p.y);
+      }
+      if (mine && ((w + 1) * kAmps) % kCheckpoint == 0) mine[(w + 1) * kAmps / kCheckpoint - 1] = s;
+    }
+    __syncthreads();
+  }
+  if (worker < 0 && lane < live) {
+    if (!checkpoints)
+      out[item0 + lane] = s;
+    else if ((windows * kAmps) % kCheckpoint != 0)  // a state shorter than a checkpoint
+      mine[windows * kAmps / kCheckpoint] = s;
+  }
+  cp_async_wait<0>();  // no copy outlives the kernel's shared memory
 }
 
 // prefix[0] = 0, prefix[c + 1] = prefix[c] + sums[c], sequentially
@@ -433,146 +446,78 @@ __global__ void k_bounds(const double* __restrict__ targets, size_t shots, const
   bounds[c] = lo;
 }
 
+// Chunks that hold shots, in any order, and each one's place among them.
 __global__ void k_active(const uint64_t* __restrict__ bounds, uint64_t nchunks, size_t shots,
-                         uint32_t* __restrict__ active, uint32_t* __restrict__ count) {
+                         uint32_t* __restrict__ active, uint32_t* __restrict__ place, uint32_t* __restrict__ count) {
   const uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (c >= nchunks) return;
   const uint64_t lo = bounds[c], hi = umin64(bounds[c + 1], shots);
-  if (lo < hi) active[atomicAdd(count, 1u)] = uint32_t(c);
+  if (lo < hi) {
+    const uint32_t a = atomicAdd(count, 1u);
+    active[a] = uint32_t(c);
+    place[c] = a;
+  }
 }
 
-// Pass 2: one warp per chunk that holds shots (src/measure.rs:134-167). The
-// warp streams the chunk's amplitudes through shared memory with cp.async
-// (windows of 2 KB, two ahead of the fold). For each window the lanes
-// compute the probabilities, eight each, with each block of eight's last
-// nonzero position; lane 0 then folds them in index order exactly as the
-// reference does: one sequential f64 sum from prefix[chunk], emitting an
-// index while the next target is below the running sum. Lane 0 adds eight
-// probabilities at a time and checks the target once against the eighth
-// sum: the running sum never decreases (p >= +0, and adding +0 changes
-// nothing), so a target at or above it emits nothing in those eight, and
-// only a block that emits is redone one probability at a time (the same
-// additions, so the same sums). Lane 0's work per amplitude is then one
-// addition of the chain.
-constexpr int kWalkWarps = 4;
-constexpr int kWalkStages = 3;
-constexpr int kWalkBytes = 2048;  // per window
-
+// Pass 2: the outcome of each sorted target (src/measure.rs:134-167), one
+// thread per shot. Its chunk is the one whose bounds hold the shot; the
+// reference walks that chunk from prefix[chunk] and emits the first index
+// whose running sum exceeds the target. The sums never decrease (p >= +0), so
+// the checkpoints (the same sums) tell which kCheckpoint amplitudes hold it,
+// and only those are added again, from the checkpoint before them. Targets
+// beyond the chunk's last sum get its last nonzero index. Chunks whose place
+// among the active ones is outside [a0, a1) are another launch's.
 template <typename T>
-__global__ void __launch_bounds__(32 * kWalkWarps) k_walk(const cplx_t<T>* __restrict__ psi, uint64_t len,
-                                                          uint64_t chunk_len, const uint32_t* __restrict__ active,
-                                                          const uint32_t* __restrict__ num_active,
-                                                          const double* __restrict__ prefix,
-                                                          const uint64_t* __restrict__ bounds, size_t shots,
-                                                          const double* __restrict__ targets,
-                                                          uint64_t* __restrict__ out) {
-  constexpr int kAmp = int(sizeof(cplx_t<T>));
-  constexpr int kPerWin = kWalkBytes / kAmp;  // 256 or 128 amplitudes
-  constexpr int kBlocks = kPerWin / 8;        // blocks of eight per window
-  __shared__ __align__(16) unsigned char raw[kWalkWarps][kWalkStages][kWalkBytes];
-  __shared__ __align__(16) double pw[kWalkWarps][kPerWin];
-  __shared__ int8_t last_in[kWalkWarps][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t a = blockIdx.x * kWalkWarps + warp;
-  if (a >= *num_active) return;
-  const uint64_t chunk = active[a];
-  const uint64_t base = chunk * chunk_len;
-  const uint64_t end = umin64(chunk_len, len - base);
-  const uint64_t hi = umin64(bounds[chunk + 1], shots);
-  uint64_t shot = bounds[chunk];
-  if (shot >= hi) return;  // the whole warp: no shot lands here
-  uint64_t last_nonzero = base;
-  double cumulative = prefix[chunk];
-  const uint64_t windows = (end + kPerWin - 1) / kPerWin;
-  const uint64_t end_b = end * kAmp;
-  const unsigned char* src0 = reinterpret_cast<const unsigned char*>(psi + base);
-  auto issue = [&](uint64_t w, int stage) {
-#pragma unroll
-    for (int i = 0; i < kWalkBytes / 512; ++i) {
-      const uint64_t off_b = w * kWalkBytes + uint64_t(i * 32 + lane) * 16;
-      unsigned char* dst = &raw[warp][stage][(i * 32 + lane) * 16];
-      if (off_b + 16 <= end_b)
-        cp_async16(dst, src0 + off_b);
-      else if (off_b < end_b)  // one complex64 left (a state of one amplitude)
-        *reinterpret_cast<cplx_t<T>*>(dst) = *reinterpret_cast<const cplx_t<T>*>(src0 + off_b);
-    }
-  };
-  for (int st = 0; st < kWalkStages - 1; ++st) {
-    if (uint64_t(st) < windows) issue(uint64_t(st), st);
-    cp_async_commit();
+__global__ void __launch_bounds__(kThreads) k_emit(const cplx_t<T>* __restrict__ psi, uint64_t len,
+                                                   uint64_t chunk_len, uint64_t nchunks,
+                                                   const uint32_t* __restrict__ place, uint32_t a0, uint32_t a1,
+                                                   const double* __restrict__ prefix,
+                                                   const uint64_t* __restrict__ bounds, size_t found,
+                                                   const double* __restrict__ checkpoints,
+                                                   const double* __restrict__ targets, uint64_t* __restrict__ out) {
+  const size_t shot = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (shot >= found) return;
+  if (shot < bounds[0]) {  // a negative target: in no chunk
+    out[shot] = 0;
+    return;
   }
-  for (uint64_t w = 0; w < windows; ++w) {
-    const uint64_t ahead = w + kWalkStages - 1;
-    if (ahead < windows) issue(ahead, int(ahead % kWalkStages));
-    cp_async_commit();
-    cp_async_wait<kWalkStages - 1>();  // window w has landed
-    __syncwarp();
-    const uint64_t pos = w * kPerWin;
-    const int n = int(umin64(kPerWin, end - pos));
-    // Lane b: the probabilities of block b (0 past the window's end) and the
-    // position of its last nonzero one (-1: none).
-    if (lane < kBlocks) {
-      const cplx_t<T>* amps = reinterpret_cast<const cplx_t<T>*>(&raw[warp][w % kWalkStages][0]);
-      const int j0 = lane * 8;
-      double p[8];
-      if (j0 + 8 <= n) {
-        const float4* v = reinterpret_cast<const float4*>(amps + j0);
-#pragma unroll
-        for (int r = 0; r < 8 * kAmp / 16; ++r) probs16<T>(v[r], p + r * (16 / kAmp));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) p[j] = j0 + j < n ? prob_fast<T>(amps[j0 + j]) : 0.0;
-      }
-      int last = -1;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        pw[warp][j0 + j] = p[j];
-        last = p[j] != 0.0 ? j : last;
-      }
-      last_in[warp][lane] = int8_t(last);
-    }
-    __syncwarp();
-    if (lane == 0) {
-      double next = targets[shot];  // shot < hi here
-      for (int j0 = 0; j0 < n && shot < hi; j0 += 8) {
-        double p[8];
-        const double2* v = reinterpret_cast<const double2*>(&pw[warp][j0]);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const double2 x = v[r];
-          p[2 * r] = x.x;
-          p[2 * r + 1] = x.y;
-        }
-        double c8 = cumulative;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) c8 = __dadd_rn(c8, p[j]);
-        if (!(next < c8)) {  // no emission among these eight
-          cumulative = c8;
-          const int last = last_in[warp][j0 >> 3];
-          if (last >= 0) last_nonzero = base + pos + uint64_t(j0 + last);
-          continue;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (p[j] == 0.0 || shot == hi) continue;
-          const uint64_t index = base + pos + uint64_t(j0 + j);
-          last_nonzero = index;
-          cumulative = __dadd_rn(cumulative, p[j]);
-          while (next < cumulative) {
-            out[shot++] = index;
-            if (shot == hi) break;
-            next = targets[shot];
-          }
-        }
-      }
-    }
-    const bool walking = __shfl_sync(0xffffffffu, shot < hi ? 1 : 0, 0) != 0;
-    __syncwarp();
-    if (!walking) break;
+  uint64_t lo = 0, hi = nchunks;  // bounds[lo] <= shot < bounds[hi]
+  while (hi - lo > 1) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (bounds[mid] <= shot)
+      lo = mid;
+    else
+      hi = mid;
   }
-  cp_async_wait<0>();  // no copy outlives the kernel's shared memory
-  if (lane == 0)
-    for (; shot < hi; ++shot) out[shot] = umin64(last_nonzero, len - 1);
+  const uint64_t chunk = lo;
+  const uint32_t a = place[chunk];
+  if (a < a0 || a >= a1) return;
+  const uint64_t base = chunk * chunk_len, end = umin64(chunk_len, len - base);
+  const uint64_t blocks = (end + kCheckpoint - 1) / kCheckpoint;
+  const double* sums = checkpoints + uint64_t(a - a0) * (chunk_len / kCheckpoint);
+  const double target = targets[shot];
+  uint64_t k = 0, top = blocks;  // the first block whose last sum exceeds the target
+  while (k < top) {
+    const uint64_t mid = (k + top) >> 1;
+    if (target < sums[mid])
+      top = mid;
+    else
+      k = mid + 1;
+  }
+  if (k < blocks) {
+    double s = k ? sums[k - 1] : prefix[chunk];
+    const uint64_t first = base + k * kCheckpoint, last = umin64(first + kCheckpoint, base + end);
+    for (uint64_t i = first; i < last; ++i) {
+      s = __dadd_rn(s, prob_fast<T>(psi[i]));
+      if (target < s) {
+        out[shot] = i;
+        return;
+      }
+    }
+  }
+  uint64_t i = base + end;
+  while (i > base && !(prob_fast<T>(psi[i - 1]) != 0.0)) --i;
+  out[shot] = umin64(i > base ? i - 1 : base, len - 1);
 }
 
 // Physical -> logical index through byte tables.
@@ -776,19 +721,26 @@ size_t sample_device_t(StateImpl& s, size_t shots, const double* uniforms_host, 
   const size_t o_prefix = o_sums + align(nchunks * 8);
   const size_t o_bounds = o_prefix + align((nchunks + 1) * 8);
   const size_t o_active = o_bounds + align((nchunks + 1) * 8);
-  const size_t o_count = o_active + align(nchunks * 4);
+  const size_t o_place = o_active + align(nchunks * 4);
+  const size_t o_count = o_place + align(nchunks * 4);
   const size_t o_uni = o_count + 256;
   const size_t o_keys = o_uni + align(shots * 8);
   const size_t o_tmp = o_keys + align(shots * 8);
   const size_t o_targets = o_tmp + align(shots * 8);
   const size_t o_out = o_targets + align(shots * 8);
   const size_t o_tables = o_out + align(shots * 8);
-  const size_t total_bytes = o_tables + align(size_t((s.n + 7) / 8 + 1) * 256 * 8);
+  // Checkpoints of the chunks that hold shots, at most 64 MB at a time.
+  const size_t per_chunk = size_t(chunk_len / kCheckpoint) * 8;
+  const size_t batch = std::min<size_t>(std::min<uint64_t>(nchunks, shots), (size_t(64) << 20) / per_chunk);
+  const size_t o_sumsat = o_tables + align(size_t((s.n + 7) / 8 + 1) * 256 * 8);
+  const size_t total_bytes = o_sumsat + align(batch * per_chunk);
   char* w = static_cast<char*>(s.work.get(total_bytes));
   double* sums = reinterpret_cast<double*>(w + o_sums);
   double* prefix = reinterpret_cast<double*>(w + o_prefix);
   uint64_t* bounds = reinterpret_cast<uint64_t*>(w + o_bounds);
   uint32_t* active = reinterpret_cast<uint32_t*>(w + o_active);
+  uint32_t* place = reinterpret_cast<uint32_t*>(w + o_place);
+  double* checkpoints = reinterpret_cast<double*>(w + o_sumsat);
   uint32_t* count = reinterpret_cast<uint32_t*>(w + o_count);
   double* uni = reinterpret_cast<double*>(w + o_uni);
   uint64_t* keys = reinterpret_cast<uint64_t*>(w + o_keys);
@@ -799,16 +751,17 @@ size_t sample_device_t(StateImpl& s, size_t shots, const double* uniforms_host, 
   const cplx_t<T>* psi = static_cast<const cplx_t<T>*>(s.amp);
 
   QVDG_CUDA(cudaMemcpyAsync(uni, uniforms_host, shots * 8, cudaMemcpyHostToDevice, s.stream));
-  static bool carveout = false;  // per instantiation
-  if (!carveout) {
-    // Eight one-warp blocks per SM (26 KB of shared memory each): all of the
-    // unified L1/shared storage as shared memory.
-    QVDG_CUDA(cudaFuncSetAttribute(k_chunk_sums<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   int(cudaSharedmemCarveoutMaxShared)));
-    carveout = true;
+  static bool configured = false;  // per instantiation
+  if (!configured) {
+    QVDG_CUDA(cudaFuncSetAttribute(k_fold<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, fold_smem<T>()));
+    configured = true;
   }
-  k_chunk_sums<T><<<unsigned((nchunks + 31) / 32), 32, 0, s.stream>>>(psi, len, chunk_len, nchunks, sums);
-  QVDG_LAUNCH_CHECK();
+  auto fold = [&](uint64_t items, const uint32_t* which, double* to, int at_checkpoints) {
+    k_fold<T><<<unsigned((items + kFoldChunks - 1) / kFoldChunks), 32 * kFoldWarps, fold_smem<T>(), s.stream>>>(
+        psi, len, chunk_len, items, which, prefix, to, at_checkpoints);
+    QVDG_LAUNCH_CHECK();
+  };
+  fold(nchunks, nullptr, sums, 0);
   k_prefix<<<1, 256, 0, s.stream>>>(sums, nchunks, prefix);
   QVDG_LAUNCH_CHECK();
   k_target_keys<<<blocks_for(shots, kThreads), kThreads, 0, s.stream>>>(uni, shots, prefix + nchunks, keys);
@@ -820,7 +773,7 @@ size_t sample_device_t(StateImpl& s, size_t shots, const double* uniforms_host, 
   k_bounds<<<blocks_for(nchunks + 1, kThreads), kThreads, 0, s.stream>>>(targets, shots, prefix, nchunks, bounds);
   QVDG_LAUNCH_CHECK();
   QVDG_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), s.stream));
-  k_active<<<blocks_for(nchunks, kThreads), kThreads, 0, s.stream>>>(bounds, nchunks, shots, active, count);
+  k_active<<<blocks_for(nchunks, kThreads), kThreads, 0, s.stream>>>(bounds, nchunks, shots, active, place, count);
   QVDG_LAUNCH_CHECK();
   // Shots that land in chunks: min(bounds[nchunks], shots).
   uint64_t* hb = static_cast<uint64_t*>(s.host.get(16));
@@ -830,10 +783,12 @@ size_t sample_device_t(StateImpl& s, size_t shots, const double* uniforms_host, 
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
   const size_t found = size_t(umin64(hb[0], shots));
   const uint32_t num_active = *hc;
-  if (num_active > 0) {
-    const unsigned walk_blocks = unsigned((num_active + kWalkWarps - 1) / kWalkWarps);
-    k_walk<T><<<walk_blocks, 32 * kWalkWarps, 0, s.stream>>>(psi, len, chunk_len, active, count, prefix, bounds,
-                                                            shots, targets, out);
+  for (size_t a0 = 0; a0 < num_active; a0 += batch) {
+    const size_t a1 = std::min<size_t>(num_active, a0 + batch);
+    fold(a1 - a0, active + a0, checkpoints, 1);
+    k_emit<T><<<blocks_for(found, kThreads), kThreads, 0, s.stream>>>(psi, len, chunk_len, nchunks, place, uint32_t(a0),
+                                                                     uint32_t(a1), prefix, bounds, found, checkpoints,
+                                                                     targets, out);
     QVDG_LAUNCH_CHECK();
   }
   if (!s.identity_layout() && found > 0) {
@@ -877,6 +832,67 @@ __global__ void k_outcome_keys(const uint64_t* __restrict__ out, size_t found, c
   keys[i] = k;
 }
 
+__device__ __forceinline__ bool run_head(const uint64_t* keys, size_t count, size_t i) {
+  return i < count && (i == 0 || keys[i] != keys[i - 1]);
+}
+
+// Runs of equal sorted keys that begin in each block's kThreads keys.
+__global__ void __launch_bounds__(kThreads) k_run_heads(const uint64_t* __restrict__ keys, size_t count,
+                                                        uint32_t* __restrict__ heads) {
+  const size_t i = size_t(blockIdx.x) * kThreads + threadIdx.x;
+  const int n = __syncthreads_count(run_head(keys, count, i));
+  if (threadIdx.x == 0) heads[blockIdx.x] = uint32_t(n);
+}
+
+// Exclusive prefix sums of `count` values in place, their total to *total
+// (mapped host memory); one block of 1024 threads, 1024 values at a time.
+__global__ void __launch_bounds__(1024) k_run_offsets(uint32_t* __restrict__ v, unsigned count,
+                                                      uint32_t* __restrict__ total) {
+  __shared__ uint32_t warp_sums[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t before = 0;
+  for (unsigned first = 0; first < count; first += 1024) {
+    const unsigned i = first + threadIdx.x;
+    const uint32_t x = i < count ? v[i] : 0u;
+    uint32_t run = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += y;
+    }
+    if (lane == 31) warp_sums[warp] = run;
+    __syncthreads();
+    uint32_t base = before, all = before;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) base += warp_sums[w];
+      all += warp_sums[w];
+    }
+    if (i < count) v[i] = base + run - x;
+    before = all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *total = before;
+}
+
+// Each run's key and the place of its first one, in order.
+__global__ void __launch_bounds__(kThreads) k_run_starts(const uint64_t* __restrict__ keys, size_t count,
+                                                         const uint32_t* __restrict__ offsets,
+                                                         uint64_t* __restrict__ run_keys,
+                                                         uint64_t* __restrict__ starts) {
+  __shared__ uint32_t warp_heads[kThreads / 32];
+  const size_t i = size_t(blockIdx.x) * kThreads + threadIdx.x;
+  const bool head = run_head(keys, count, i);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned mask = __ballot_sync(0xffffffffu, head);
+  if (lane == 0) warp_heads[warp] = __popc(mask);
+  __syncthreads();
+  if (!head) return;
+  uint32_t at = offsets[blockIdx.x] + __popc(mask & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) at += warp_heads[w];
+  run_keys[at] = keys[i];
+  starts[at] = i;
+}
+
 template <typename T>
 size_t counts_t(StateImpl& s, size_t shots, const double* uniforms_host, const MeasureMap& m,
                 std::vector<uint64_t>& keys_out, std::vector<uint64_t>& counts_out) {
@@ -888,17 +904,31 @@ size_t counts_t(StateImpl& s, size_t shots, const double* uniforms_host, const M
   if (found == 0) return 0;
   k_outcome_keys<<<blocks_for(found, kThreads), kThreads, 0, s.stream>>>(out, found, m, keys);
   QVDG_LAUNCH_CHECK();
-  radix_sort_u64(keys, tmp, found, s.work2, s.stream);
-  std::vector<uint64_t> sorted(found);
-  QVDG_CUDA(cudaMemcpyAsync(sorted.data(), keys, found * 8, cudaMemcpyDeviceToHost, s.stream));
+  int bits = 0;  // of a key
+  for (int j = 0; j < m.n; ++j) bits = std::max(bits, int(m.c[j]) + 1);
+  radix_sort_u64(keys, tmp, found, s.work2, s.stream, bits);
+  // The sorted keys' runs: where each begins, found on the device, so that
+  // only the distinct keys and their places come back (8 MB and a pass over
+  // them on the host for a million shots otherwise).
+  const unsigned blocks = blocks_for(found, kThreads);
+  uint32_t* heads = static_cast<uint32_t*>(s.work2.get((size_t(blocks) + 1) * sizeof(uint32_t)));
+  uint32_t* total = static_cast<uint32_t*>(s.host.get(sizeof(uint32_t)));
+  k_run_heads<<<blocks, kThreads, 0, s.stream>>>(keys, found, heads);
+  QVDG_LAUNCH_CHECK();
+  k_run_offsets<<<1, 1024, 0, s.stream>>>(heads, blocks, total);
+  QVDG_LAUNCH_CHECK();
+  // `out` (the outcomes) and `tmp` are free now.
+  k_run_starts<<<blocks, kThreads, 0, s.stream>>>(keys, found, heads, tmp, out);
+  QVDG_LAUNCH_CHECK();
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
-  for (size_t i = 0; i < found;) {
-    size_t j = i + 1;
-    while (j < found && sorted[j] == sorted[i]) ++j;
-    keys_out.push_back(sorted[i]);
-    counts_out.push_back(j - i);
-    i = j;
-  }
+  const size_t runs = *total;
+  uint64_t* h = static_cast<uint64_t*>(s.host.get(2 * runs * sizeof(uint64_t)));
+  QVDG_CUDA(cudaMemcpyAsync(h, tmp, runs * sizeof(uint64_t), cudaMemcpyDeviceToHost, s.stream));
+  QVDG_CUDA(cudaMemcpyAsync(h + runs, out, runs * sizeof(uint64_t), cudaMemcpyDeviceToHost, s.stream));
+  QVDG_CUDA(cudaStreamSynchronize(s.stream));
+  keys_out.assign(h, h + runs);
+  counts_out.resize(runs);
+  for (size_t i = 0; i < runs; ++i) counts_out[i] = (i + 1 < runs ? h[runs + i + 1] : uint64_t(found)) - h[runs + i];
   return found;
 }
 

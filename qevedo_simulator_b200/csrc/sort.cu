@@ -1,4 +1,5 @@
-// Stable LSD radix sort of 64-bit keys (8-bit digits, 8 passes).
+// Stable LSD radix sort of 64-bit keys (8-bit digits, a pass for each digit
+// in use).
 //
 // Used by the sampler to sort its targets (the reference sorts them with
 // rayon's par_sort_unstable_by(f64::total_cmp), src/measure.rs:125-126; the
@@ -96,14 +97,15 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const uint64_t* __restrict
 
 }  // namespace
 
-void radix_sort_u64(uint64_t* keys, uint64_t* tmp, size_t count, DeviceScratch& work, cudaStream_t stream) {
+void radix_sort_u64(uint64_t* keys, uint64_t* tmp, size_t count, DeviceScratch& work, cudaStream_t stream, int bits) {
   if (count <= 1) return;
+  const int end = (bits + 15) / 16 * 16;  // an even number of passes: the result is back in `keys`
   if (count > size_t(0xFFFFFFFFu)) throw Error(1, "too many keys to sort");
   const uint32_t tiles = uint32_t((count + kTile - 1) / kTile);
   uint32_t* hist = static_cast<uint32_t*>(work.get(size_t(256) * tiles * sizeof(uint32_t)));
   uint64_t* src = keys;
   uint64_t* dst = tmp;
-  for (int shift = 0; shift < 64; shift += 8) {
+  for (int shift = 0; shift < end; shift += 8) {
     k_hist<<<tiles, kThreads, 0, stream>>>(src, count, shift, hist, tiles);
     QVDG_LAUNCH_CHECK();
     k_scan<<<1, 1024, 0, stream>>>(hist, size_t(256) * tiles);
@@ -114,7 +116,6 @@ void radix_sort_u64(uint64_t* keys, uint64_t* tmp, size_t count, DeviceScratch& 
     src = dst;
     dst = t;
   }
-  // Eight passes: the sorted keys are back in `keys`.
 }
 
 }  // namespace qvdg

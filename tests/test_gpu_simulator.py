@@ -327,3 +327,41 @@ def test_run_and_statevector_on_openqasm_text():
     sv = statevector(qasm.parse(unitary))
     assert np.array_equal(statevector(unitary, threads="cores"), sv)
     assert np.array_equal(statevector(unitary, threads=2), sv)
+
+
+@pytest.mark.parametrize("shots", [1, 2, 255, 256, 257, 5000, 300000])
+@pytest.mark.parametrize("clbits", [[0], [7, 3], [15, 0], [16, 2], [63, 17, 8]])
+def test_counted_keys_equal_the_outcomes_counted_on_the_host(shots, clbits):
+    """Runs of equal keys across blocks and block groups, keys of one to
+    eight digits: the counts of the sampled outcomes themselves."""
+    rng = np.random.default_rng(shots + sum(clbits))
+    psi = rng.standard_normal(1 << 9) + 1j * rng.standard_normal(1 << 9)
+    psi[rng.random(1 << 9) < 0.3] = 0
+    uniforms = rng.random(shots)
+    measures = [(2 * i + 1, c) for i, c in enumerate(clbits)]
+    with DeviceState(9, 32) as st:
+        st.set_amplitudes(psi / np.linalg.norm(psi))
+        outcomes = st.sample_unordered(uniforms)
+        keys, counts = st.sample_counts(uniforms, measures)
+    expected = np.zeros(outcomes.size, dtype=np.uint64)
+    for q, c in measures:
+        expected |= ((outcomes >> np.uint64(q)) & np.uint64(1)) << np.uint64(c)
+    u, n = np.unique(expected, return_counts=True)
+    assert np.array_equal(keys, u) and np.array_equal(counts, n.astype(np.uint64))
+
+
+@pytest.mark.parametrize("bits, n", [(32, 15), (32, 16), (32, 19), (32, 20), (64, 14), (64, 15), (64, 18), (64, 19)])
+def test_sampler_is_bit_exact_around_blocks_of_chunks(oracle, bits, n):
+    """One chunk, two, and 16 and 17+ chunks (a block folds 16), with zeros
+    inside and at the end of chunks and shots on every chunk's last ones."""
+    rng = np.random.default_rng(n)
+    psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    psi[rng.random(1 << n) < 0.4] = 0
+    psi[-300:] = 0
+    psi /= np.linalg.norm(psi)
+    u = np.concatenate([rng.random(4000), np.linspace(0, 1, 4096, endpoint=False), [0.0, np.nextafter(1.0, 0.0)]])
+    with DeviceState(n, bits) as st:
+        st.set_amplitudes(psi)
+        held = st.amplitudes()  # in the state's own precision
+        got = st.sample_unordered(u)
+    assert np.array_equal(got, oracle.sample_from_amplitudes(held, u, bits))
