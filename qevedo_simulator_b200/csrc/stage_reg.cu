@@ -11,9 +11,14 @@
 // a mask of active register groups) and every diagonal gate that is ready
 // (a diagonal reads bits inside G per register and bits outside G from the
 // thread's subcube base). So one shared-memory round trip serves several
-// gates, and no matrix is ever multiplied out: a 1-qubit gate costs 4 to 8
-// FMAs per amplitude (real and RX-type matrices take the cheaper forms), a
-// +-1 diagonal (CZ and the like) only toggles sign bits.
+// gates, and no matrix is ever multiplied out. A 1-qubit gate whose rows'
+// larger entries lie on the diagonal and agree up to sign (rotations, H, SX,
+// the square roots of X, Y and W) is divided by them: x0 + a x1 and
+// x1 + b x0, two multiply-adds per amplitude for real or imaginary a and b,
+// four for complex ones, half of what the matrix takes. The stage's last
+// register pass multiplies by the product of the divisors, and their signs
+// join the sign flips. A +-1 diagonal (CZ and the like) only toggles sign
+// bits, consecutive ones together; a (controlled) X moves registers.
 //
 // A tile's 16-byte cp.async copies and its stores back to HBM are covered by
 // another CTA's computation: two CTAs per SM, one tile buffer each. What
@@ -26,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <complex>
 #include <cstring>
 #include <vector>
 
@@ -40,7 +46,7 @@ constexpr int kRegThreads = 512;
 constexpr size_t kRegBlobBudget = 64 * 1024;
 
 enum : uint8_t { kRegDense1 = 0, kRegDense2 = 1, kRegSign = 2, kRegPhase = 3, kRegSign2 = 4 };
-enum : uint8_t { kSpecGeneral = 0, kSpecReal = 1, kSpecRx = 2, kSpecDiagReal = 3 };
+enum : uint8_t { kFormGeneral = 0, kFormReal = 1, kFormImag = 2, kFormComplex = 3, kFormX = 4 };
 
 // Shared-memory position of tile element e: bits 1-3 XORed with bits 5-7,
 // 9-11 and 13-15 (bit 0 is kept, so element pairs 2v, 2v+1 stay one 16-byte
@@ -60,12 +66,14 @@ static_assert(sizeof(RegPassHdr) == 16, "header layout");
 
 // Dispatch codes of the register kernel (one switch per gate).
 enum : uint16_t {
-  kOpDense1 = 0,         // + 4 * spec + target register bit (16 codes), no register controls
-  kOpDense1Masked = 16,  // any matrix, register controls
-  kOpDense2 = 17,
-  kOpSign2 = 18,
-  kOpSign = 19,
-  kOpPhase = 20,
+  kOpShear = 0,    // + 4 * (form - kFormReal) + target register bit (12 codes): (a, b)
+  kOpX = 12,       // + target register bit: X where `pmask` says
+  kOpDense1 = 16,  // + target register bit: any matrix, where `pmask` says
+  kOpDense2 = 20,
+  kOpSign2 = 21,
+  kOpSign = 22,
+  kOpPhase = 23,
+  kOpScale = 24,   // multiply by a number
 };
 
 struct RegGate {
@@ -111,25 +119,12 @@ __device__ __forceinline__ cplx_t<T> mul_c(cplx_t<T> m, cplx_t<T> x) {
   return make_c<T>(fma(m.x, x.x, -m.y * x.y), fma(m.x, x.y, m.y * x.x));
 }
 
-// y = m0 * x0 + m1 * x1 for complex m (general), real m (spec real: the
-// imaginary parts are zero) or the RX form (m0 real, m1 imaginary).
-template <typename T, int SPEC>
-__device__ __forceinline__ cplx_t<T> row2(cplx_t<T> m0, cplx_t<T> m1, cplx_t<T> x0, cplx_t<T> x1) {
-  if (SPEC == kSpecReal) return make_c<T>(fma(m0.x, x0.x, m1.x * x1.x), fma(m0.x, x0.y, m1.x * x1.y));
-  if (SPEC == kSpecRx) return make_c<T>(fma(m0.x, x0.x, -m1.y * x1.y), fma(m0.x, x0.y, m1.y * x1.x));
-  if (SPEC == kSpecDiagReal)
-    return make_c<T>(fma(m0.x, x0.x, fma(m1.x, x1.x, -m1.y * x1.y)), fma(m0.x, x0.y, fma(m1.x, x1.y, m1.y * x1.x)));
-  return make_c<T>(fma(m0.x, x0.x, fma(-m0.y, x0.y, fma(m1.x, x1.x, -m1.y * x1.y))),
-                   fma(m0.x, x0.y, fma(m0.y, x0.x, fma(m1.x, x1.y, m1.y * x1.x))));
-}
-// Second rows: the RX form has an imaginary first entry and a real second;
-// the real-diagonal form a complex first entry and a real second.
-template <typename T, int SPEC>
-__device__ __forceinline__ cplx_t<T> row2b(cplx_t<T> m0, cplx_t<T> m1, cplx_t<T> x0, cplx_t<T> x1) {
-  if (SPEC == kSpecRx) return make_c<T>(fma(m1.x, x1.x, -m0.y * x0.y), fma(m1.x, x1.y, m0.y * x0.x));
-  if (SPEC == kSpecDiagReal)
-    return make_c<T>(fma(m1.x, x1.x, fma(m0.x, x0.x, -m0.y * x0.y)), fma(m1.x, x1.y, fma(m0.x, x0.y, m0.y * x0.x)));
-  return row2<T, SPEC>(m0, m1, x0, x1);
+// x + m * y for real, imaginary or complex m.
+template <typename T, int FORM>
+__device__ __forceinline__ cplx_t<T> shear(cplx_t<T> x, cplx_t<T> m, cplx_t<T> y) {
+  if (FORM == kFormReal) return make_c<T>(fma(m.x, y.x, x.x), fma(m.x, y.y, x.y));
+  if (FORM == kFormImag) return make_c<T>(fma(-m.y, y.y, x.x), fma(m.y, y.x, x.y));
+  return make_c<T>(fma(m.x, y.x, fma(-m.y, y.y, x.x)), fma(m.x, y.y, fma(m.y, y.x, x.y)));
 }
 
 // Sign flip of a complex value where `bit` is 1, on the sign bits.
@@ -145,33 +140,55 @@ __device__ __forceinline__ void flip(double2& x, uint32_t t) {
   x.y = __longlong_as_double(__double_as_longlong(x.y) ^ s);
 }
 
-template <typename T, int TB, int SPEC, bool MASKED>
-__device__ __forceinline__ void apply1(cplx_t<T> (&a)[16], const cplx_t<T>* m, uint32_t pmask) {
-  const cplx_t<T> m00 = m[0], m01 = m[1], m10 = m[2], m11 = m[3];
+template <typename T, int TB, int FORM>
+__device__ __forceinline__ void apply_shear(cplx_t<T> (&a)[16], const cplx_t<T>* m) {
+  const cplx_t<T> m0 = m[0], m1 = m[1];
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     if (j & (1 << TB)) continue;
     const cplx_t<T> x0 = a[j], x1 = a[j | (1 << TB)];
-    const cplx_t<T> y0 = row2<T, SPEC>(m00, m01, x0, x1);
-    const cplx_t<T> y1 = row2b<T, SPEC>(m10, m11, x0, x1);
-    if (MASKED) {
-      const bool on = (pmask >> j) & 1u;
-      a[j] = on ? y0 : x0;
-      a[j | (1 << TB)] = on ? y1 : x1;
-    } else {
-      a[j] = y0;
-      a[j | (1 << TB)] = y1;
-    }
+    a[j] = shear<T, FORM>(x0, m0, x1);
+    a[j | (1 << TB)] = shear<T, FORM>(x1, m1, x0);
   }
 }
 
-template <typename T, int SPEC, bool MASKED>
-__device__ __forceinline__ void apply1_bit(cplx_t<T> (&a)[16], int tb, const cplx_t<T>* m, uint32_t pmask) {
-  switch (tb) {
-    case 0: apply1<T, 0, SPEC, MASKED>(a, m, pmask); break;
-    case 1: apply1<T, 1, SPEC, MASKED>(a, m, pmask); break;
-    case 2: apply1<T, 2, SPEC, MASKED>(a, m, pmask); break;
-    default: apply1<T, 3, SPEC, MASKED>(a, m, pmask); break;
+template <typename T, int TB>
+__device__ __forceinline__ void apply_x(cplx_t<T> (&a)[16], uint32_t pmask) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (j & (1 << TB)) continue;
+    const bool on = (pmask >> j) & 1u;
+    const cplx_t<T> x0 = a[j], x1 = a[j | (1 << TB)];
+    a[j] = on ? x1 : x0;
+    a[j | (1 << TB)] = on ? x0 : x1;
+  }
+}
+
+// A matrix entry from shared memory, read where it is used (volatile: kept in
+// registers over the pairs, the entries would spill).
+__device__ __forceinline__ float2 entry(const float2* m) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(m)));
+  return v;
+}
+__device__ __forceinline__ double2 entry(const double2* m) {
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(smem_u32(m)));
+  return v;
+}
+
+template <typename T, int TB>
+__device__ __forceinline__ void apply_dense1(cplx_t<T> (&a)[16], const cplx_t<T>* m, uint32_t pmask) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (j & (1 << TB)) continue;
+    const cplx_t<T> x0 = a[j], x1 = a[j | (1 << TB)];
+    cplx_t<T> y0 = mul_c<T>(entry(m + 1), x1), y1 = mul_c<T>(entry(m + 3), x1);
+    cmac<T>(y0, entry(m), x0);
+    cmac<T>(y1, entry(m + 2), x0);
+    const bool on = (pmask >> j) & 1u;
+    a[j] = on ? y0 : x0;
+    a[j | (1 << TB)] = on ? y1 : x1;
   }
 }
 
@@ -277,6 +294,8 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
     // Bits a sign gate reads outside the registers: the tile's global bits
     // and the subcube's tile bits (at 48 and up).
     const uint64_t where = tile_base | (uint64_t(eb) << 48);
+    uint32_t flips = 0;   // registers to negate
+    bool signs = false;   // some gate has set it (the same in every thread)
     // The next gate's record is read while the present one is applied.
     uint4 ahead = *reinterpret_cast<const uint4*>(&gates[first]);
     for (uint32_t gi = first; gi < last; ++gi) {
@@ -289,21 +308,37 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
         if ((tile_base & g.gcm) != g.gcv || (eb & g.lcm) != g.lcv) continue;
       const unsigned char* data = blob + hot.z;
       const C2* m = reinterpret_cast<const C2*>(data);
-      switch (op >= kOpSign2 ? op : (op == kOpDense2 ? 1u : 0u)) {
-        case 0:  // dense 1-qubit
-          if (op == kOpDense1Masked) {
-            apply1_bit<T, kSpecGeneral, true>(a, int(t0), m, pmask);
-          } else {
-            const int tb = int(op & 3u);
-            switch ((op - kOpDense1) >> 2) {
-              case kSpecReal: apply1_bit<T, kSpecReal, false>(a, tb, m, 0); break;
-              case kSpecRx: apply1_bit<T, kSpecRx, false>(a, tb, m, 0); break;
-              case kSpecDiagReal: apply1_bit<T, kSpecDiagReal, false>(a, tb, m, 0); break;
-              default: apply1_bit<T, kSpecGeneral, false>(a, tb, m, 0); break;
-            }
-          }
-          break;
-        case 1: {  // dense 2-qubit
+      if (op < kOpSign2 && signs) {
+        // Sign flips up to here, all at once (diagonals commute with them).
+        flip_mask<T>(a, flips);
+        flips = 0;
+        signs = false;
+      }
+      switch (op) {
+#define QVDG_SHEAR(form, bit_) \
+  case kOpShear + 4 * (form - kFormReal) + bit_: apply_shear<T, bit_, form>(a, m); break;
+        QVDG_SHEAR(kFormReal, 0)
+        QVDG_SHEAR(kFormReal, 1)
+        QVDG_SHEAR(kFormReal, 2)
+        QVDG_SHEAR(kFormReal, 3)
+        QVDG_SHEAR(kFormImag, 0)
+        QVDG_SHEAR(kFormImag, 1)
+        QVDG_SHEAR(kFormImag, 2)
+        QVDG_SHEAR(kFormImag, 3)
+        QVDG_SHEAR(kFormComplex, 0)
+        QVDG_SHEAR(kFormComplex, 1)
+        QVDG_SHEAR(kFormComplex, 2)
+        QVDG_SHEAR(kFormComplex, 3)
+#undef QVDG_SHEAR
+        case kOpX + 0: apply_x<T, 0>(a, pmask); break;
+        case kOpX + 1: apply_x<T, 1>(a, pmask); break;
+        case kOpX + 2: apply_x<T, 2>(a, pmask); break;
+        case kOpX + 3: apply_x<T, 3>(a, pmask); break;
+        case kOpDense1 + 0: apply_dense1<T, 0>(a, m, pmask); break;
+        case kOpDense1 + 1: apply_dense1<T, 1>(a, m, pmask); break;
+        case kOpDense1 + 2: apply_dense1<T, 2>(a, m, pmask); break;
+        case kOpDense1 + 3: apply_dense1<T, 3>(a, m, pmask); break;
+        case kOpDense2: {
           save();
           // The register bits that are not targets, and the groups (by their
           // values) that are active.
@@ -319,23 +354,37 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
         }
         case kOpSign2: {
           const uint16_t* masks = reinterpret_cast<const uint16_t*>(data);
-          flip_mask<T>(a, masks[uint32_t((where >> t0) & 1u) | (uint32_t((where >> t1) & 1u) << 1)]);
+          flips ^= masks[uint32_t((where >> t0) & 1u) | (uint32_t((where >> t1) & 1u) << 1)];
+          signs = true;
           break;
         }
         case kOpSign: {
           const uint16_t* masks = reinterpret_cast<const uint16_t*>(data);
-          flip_mask<T>(a, masks[diag_fixed(g, eb, tile_base)]);
+          flips ^= masks[diag_fixed(g, eb, tile_base)];
+          signs = true;
           break;
         }
-        default: {  // kOpPhase
+        case kOpPhase: {
           const uint16_t* ridx = reinterpret_cast<const uint16_t*>(blob + hot.w);
           const uint32_t f = diag_fixed(g, eb, tile_base);
 #pragma unroll
           for (int j = 0; j < 16; ++j) a[j] = mul_c<T>(m[f | ridx[j]], a[j]);
           break;
         }
+        default: {  // kOpScale
+          const C2 f = m[0];
+          if (f.y == T(0)) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) a[j] = make_c<T>(f.x * a[j].x, f.x * a[j].y);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) a[j] = mul_c<T>(f, a[j]);
+          }
+          break;
+        }
       }
     }
+    if (signs) flip_mask<T>(a, flips);
     save();
   }
   __syncthreads();
@@ -476,6 +525,35 @@ size_t put_complex(std::vector<uint8_t>& blob, const std::vector<C>& v, int bits
   return put(blob, d.data(), d.size());
 }
 
+// How a 1-qubit gate is applied: X, sheared (m becomes (a, b), its divisor
+// goes into `scale`; `negate`: the second row's has the other sign), or by
+// its matrix. Only a gate applied everywhere can be sheared, and only by a
+// divisor of ordinary size (a user's matrix need not be unitary).
+uint8_t dense1_form(std::vector<C>& m, bool everywhere, std::complex<long double>& scale, bool& negate) {
+  using Cd = std::complex<double>;
+  const Cd u[4] = {{m[0].re, m[0].im}, {m[1].re, m[1].im}, {m[2].re, m[2].im}, {m[3].re, m[3].im}};
+  if (u[0] == 0.0 && u[3] == 0.0 && u[1] == 1.0 && u[2] == 1.0) return kFormX;
+  const double d = std::abs(u[0]);
+  if (!everywhere || !(d >= 0.5 && d <= 2.0)) return kFormGeneral;
+  const double eps = 2.3e-16 * d;
+  const bool same = std::abs(u[3] - u[0]) <= eps, opposite = std::abs(u[3] + u[0]) <= eps;
+  if (!(same || opposite) || !(std::abs(u[1]) <= 1.0001 * d) || !(std::abs(u[2]) <= 1.0001 * d)) return kFormGeneral;
+  const Cd a = u[1] / u[0], b = u[2] / u[3];
+  // a and b are rounded: the divisor that keeps the rows' norms takes half of
+  // that back (equal gates would add it up).
+  using Cl = std::complex<long double>;
+  const Cl l[4] = {Cl(u[0]), Cl(u[1]), Cl(u[2]), Cl(u[3])};
+  auto off = [&](const Cd& ratio, const Cl& entry, const Cl& div) {  // of an entry, times its share of the row
+    return entry == Cl(0) ? Cl(0) : (Cl(ratio) * div / entry - Cl(1)) * (std::norm(entry) / (std::norm(entry) + std::norm(div)));
+  };
+  scale *= l[0] * (Cl(1) - (off(a, l[1], l[0]) + off(b, l[2], l[3])) / Cl(2));
+  negate = opposite;
+  m = {C{a.real(), a.imag()}, C{b.real(), b.imag()}};
+  if (a.imag() == 0.0 && b.imag() == 0.0) return kFormReal;
+  if (a.real() == 0.0 && b.real() == 0.0) return kFormImag;
+  return kFormComplex;
+}
+
 }  // namespace
 
 bool register_pass_ok(const Target& s, const PlannedPass& p) {
@@ -491,8 +569,11 @@ bool register_pass_ok(const Target& s, const PlannedPass& p) {
   return true;
 }
 
-LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const StageConfig& cfg, StageUpload& up) {
-  LoweredPass lp;
+namespace {
+
+// False when the pass's blob is too large (nothing is uploaded then).
+bool lower_register(const Target& s, const PlannedPass& p, const StageConfig& cfg, StageUpload& up, bool shear,
+                    LoweredPass& lp) {
   lp.staged = true;
   TileGeom& geo = lp.geo;
   const int L = int(p.tile_bits.size());
@@ -593,6 +674,7 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
     bool has_table;
   };
   std::vector<Fix> fixes;
+  std::complex<long double> scale = 1.0L;  // product of the sheared gates' divisors
   for (size_t pi = 0; pi < passes.size(); ++pi) {
     const Pass& ps = passes[pi];
     RegPassHdr h{};
@@ -606,12 +688,11 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
       }
     h.pair = h.g[0] == 0 ? 1 : 0;
     h.first_gate = uint32_t(gates.size());
-    h.num_gates = uint16_t(ps.ops.size());
-    std::memcpy(blob.data() + pi * sizeof(RegPassHdr), &h, sizeof(h));
     for (size_t oi : ps.ops) {
       const RegOp& r = ops[oi];
       RegGate g{};
       Fix fx{gates.size(), 0, 0, false};
+      bool sign_after = false;
       g.gcm = r.gcm;
       g.gcv = r.gcv;
       if (r.dense) {
@@ -648,10 +729,8 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
           if (!(j & tmask) && (j & rcm) == rcv) pm |= 1u << j;
         g.pmask = rcm == 0 ? uint16_t(0xffffu) : uint16_t(pm);  // 0xffff: no register controls
         if (g.kind == kRegDense1) {
-          const bool real = m[0].im == 0 && m[1].im == 0 && m[2].im == 0 && m[3].im == 0;
-          const bool rx = m[0].im == 0 && m[3].im == 0 && m[1].re == 0 && m[2].re == 0;
-          const bool diag_real = m[0].im == 0 && m[3].im == 0;
-          g.spec = real ? kSpecReal : (rx ? kSpecRx : (diag_real ? kSpecDiagReal : kSpecGeneral));
+          const bool everywhere = shear && r.local_ctl_mask == 0 && r.gcm == 0;
+          g.spec = dense1_form(m, everywhere, scale, sign_after);
         }
         fx.data_off = put_complex(data, m, s.bits);
       } else {
@@ -714,7 +793,8 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
       }
       g.pred = (g.gcm != 0 || g.lcm != 0) ? 1 : 0;
       if (g.kind == kRegDense1)
-        g.op = g.pmask == 0xffffu ? uint16_t(kOpDense1 + 4 * g.spec + g.t0) : uint16_t(kOpDense1Masked);
+        g.op = uint16_t(g.t0 + (g.spec == kFormGeneral ? kOpDense1
+                                                       : (g.spec == kFormX ? kOpX : kOpShear + 4 * (g.spec - kFormReal))));
       else if (g.kind == kRegDense2)
         g.op = kOpDense2;
       else if (g.kind == kRegSign2)
@@ -725,7 +805,30 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
         g.op = kOpPhase;
       gates.push_back(g);
       fixes.push_back(fx);
+      if (sign_after) {
+        // Divisors of opposite sign: -1 where the target is 1.
+        RegGate z{};
+        z.kind = kRegSign2;
+        z.op = kOpSign2;
+        z.t0 = z.t1 = 63;
+        uint16_t mask = 0;
+        for (uint32_t j = 0; j < 16; ++j)
+          if ((j >> g.t0) & 1u) mask |= uint16_t(1u << j);
+        const uint16_t masks[4] = {mask, mask, mask, mask};
+        Fix zx{gates.size(), put(data, masks, 4), 0, false};
+        gates.push_back(z);
+        fixes.push_back(zx);
+      }
     }
+    if (pi + 1 == passes.size() && scale != std::complex<long double>(1.0L)) {
+      RegGate f{};
+      f.op = kOpScale;
+      Fix fx{gates.size(), put_complex(data, {C{double(scale.real()), double(scale.imag())}}, s.bits), 0, false};
+      gates.push_back(f);
+      fixes.push_back(fx);
+    }
+    h.num_gates = uint16_t(gates.size() - h.first_gate);
+    std::memcpy(blob.data() + pi * sizeof(RegPassHdr), &h, sizeof(h));
   }
   const size_t gates_off = blob.size();  // a multiple of 16
   const size_t data_base = gates_off + gates.size() * sizeof(RegGate);
@@ -737,7 +840,7 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
   std::memcpy(blob.data() + gates_off, gates.data(), gates.size() * sizeof(RegGate));
   blob.insert(blob.end(), data.begin(), data.end());
   blob.resize((blob.size() + 15) & ~size_t(15), 0);
-  if (blob.size() > kRegBlobBudget) throw Error(QVDG_ERR_UNSUPPORTED, "internal: register stage program too large");
+  if (blob.size() > kRegBlobBudget) return false;
 
   up.tc.resize((up.tc.size() + 15) & ~size_t(15), 0);
   geo.tc_offset = up.tc.size();
@@ -745,7 +848,19 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
   geo.num_gates = int(passes.size());
   up.tc.insert(up.tc.end(), blob.begin(), blob.end());
   lp.gate_offset = up.gates.size();
-  return lp;
+  return true;
+}
+
+}  // namespace
+
+LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const StageConfig& cfg, StageUpload& up) {
+  // The signs and the factor that sheared gates leave take some room of
+  // their own.
+  for (const bool shear : {true, false}) {
+    LoweredPass lp;
+    if (lower_register(s, p, cfg, up, shear, lp)) return lp;
+  }
+  throw Error(QVDG_ERR_UNSUPPORTED, "internal: register stage program too large");
 }
 
 size_t register_blob_budget() { return kRegBlobBudget; }

@@ -601,3 +601,33 @@ def test_shared_diagonal_passes_equal_separate_ones(oracle, bits, n):
         if n <= 13:
             expected = oracle.naive_statevector(program, n, initial=psi)
             assert max_distance(got[0][0], expected) < {32: 1e-5, 64: 1e-11}[bits]
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [5, 9, 13, 14])
+def test_register_stage_gate_forms(oracle, bits, n):
+    """Every form a register stage gives a 1-qubit gate, on every register
+    bit, with and without controls: sheared by a real, imaginary or complex
+    divisor of either sign, X, general, and matrices that are not unitary
+    (whose divisors it must not take)."""
+    from qevedo_simulator_b200 import Gate
+
+    rng = np.random.default_rng(n + bits)
+    h = np.pi / 2
+    ms = [Gate("rx", (h,)).matrix(), Gate("rx", (0.3,)).matrix(), Gate("ry", (h,)).matrix(), Gate("h").matrix(),
+          Gate("sx").matrix(), Gate("u", (h, -np.pi / 4, np.pi / 4)).matrix(), Gate("x").matrix(), Gate("y").matrix(),
+          Gate("u", (0.2, 1.1, 0.4)).matrix(), np.array([[1e-3, 0], [0, 1e3]]) @ Gate("h").matrix(),
+          np.array([[1.0, 0.25], [-0.5, -1.0]]), np.array([[1.0, 0.5], [0.25, 1.0]]) * 3]
+    psi = random_state(rng, n)
+    for m in ms:
+        ops = []
+        for q in range(n):
+            c = (q + 1) % n
+            ops += [Op([q], [], m / np.linalg.norm(m, 2)), Op([q], [(c, bool(q & 1))], Gate("z").matrix()),
+                    Op([q], [(c, True)], m / np.linalg.norm(m, 2)), Op([c], [], Gate("h").matrix())]
+        expected = oracle.naive_statevector(ops, n, initial=psi)
+        with DeviceState(n, bits) as st:
+            st.set_amplitudes(psi)
+            stats = st.apply_ops(ops, options(4, True))
+            assert stats["stages"] > 0
+            assert max_distance(st.amplitudes(), expected) < {32: 1e-5, 64: 1e-11}[bits]
