@@ -138,11 +138,31 @@ __host__ __device__ constexpr int ladder_to(int j) {
 }
 __host__ __device__ constexpr int ladder_from(int j) { return j ^ ((j << 1) & ((1 << kGroup) - 1)); }
 
+// Shared-memory accesses by 32-bit address: through a pointer chosen between
+// two tile buffers they become generic ones, with 64-bit address arithmetic
+// for every amplitude.
+__device__ __forceinline__ u64 lds64(uint32_t a) {
+  u64 v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ ulonglong2 lds128(uint32_t a) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts64(uint32_t a, u64 v) {
+  asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t a, u64 x, u64 y) {
+  asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
+}
+
 // One step on every subcube of the 2^nb-element tile. kLow: the group on the
 // lowest bits (lq = 0: its subcubes are contiguous, moved 16 bytes at a
 // time; nothing outside controls qubit 0).
 template <int G, bool kLow>
-__device__ __forceinline__ void apply_step(unsigned char* tile, int nb, const Tables& tab, int si, uint32_t form,
+__device__ __forceinline__ void apply_step(uint32_t tile, int nb, const Tables& tab, int si, uint32_t form,
                                            int entangler, const TileMap& map) {
   constexpr int S = 1 << G;
   const int lq = kLow ? 0 : tab.step[si].lq, q = tab.step[si].q;
@@ -167,13 +187,13 @@ __device__ __forceinline__ void apply_step(unsigned char* tile, int nb, const Ta
     if constexpr (kLow && G > 0) {
 #pragma unroll
       for (int j = 0; j < S; j += 2) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(tile + (base ^ at(j)));
+        const ulonglong2 v = lds128(tile + (base ^ at(j)));
         a[j] = v.x;
         a[j + 1] = v.y;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < S; ++j) a[j] = *reinterpret_cast<const u64*>(tile + (base ^ at(j)));
+      for (int j = 0; j < S; ++j) a[j] = lds64(tile + (base ^ at(j)));
     }
     // The ladder's gate into the group's first qubit is controlled by a bit
     // outside it: constant for the subcube.
@@ -228,24 +248,23 @@ __device__ __forceinline__ void apply_step(unsigned char* tile, int nb, const Ta
       if constexpr (kLow && G > 1) {
 #pragma unroll
         for (int j = 0; j < S; j += 2)
-          *reinterpret_cast<ulonglong2*>(tile + (to ^ at(j))) =
-              make_ulonglong2(a[ladder_from(j) & (S - 1)], a[ladder_from(j + 1) & (S - 1)]);
+          sts128(tile + (to ^ at(j)), a[ladder_from(j) & (S - 1)], a[ladder_from(j + 1) & (S - 1)]);
       } else {
 #pragma unroll
-        for (int j = 0; j < S; ++j) *reinterpret_cast<u64*>(tile + (to ^ at(ladder_to(j) & (S - 1)))) = a[j];
+        for (int j = 0; j < S; ++j) sts64(tile + (to ^ at(ladder_to(j) & (S - 1))), a[j]);
       }
     } else if constexpr (kLow && G > 0) {
 #pragma unroll
       for (int j = 0; j < S; j += 2)
-        *reinterpret_cast<ulonglong2*>(tile + (base ^ at(j))) = make_ulonglong2(a[j], a[j + 1]);
+        sts128(tile + (base ^ at(j)), a[j], a[j + 1]);
     } else {
 #pragma unroll
-      for (int j = 0; j < S; ++j) *reinterpret_cast<u64*>(tile + (base ^ at(j))) = a[j];
+      for (int j = 0; j < S; ++j) sts64(tile + (base ^ at(j)), a[j]);
     }
   }
 }
 
-__device__ __forceinline__ void run_step(unsigned char* tile, int nb, const Tables& tab, int si, uint32_t form,
+__device__ __forceinline__ void run_step(uint32_t tile, int nb, const Tables& tab, int si, uint32_t form,
                                          int entangler, const TileMap& map) {
   const int G = tab.step[si].G;
   if (tab.step[si].lq == 0) {
@@ -416,6 +435,7 @@ __global__ void __launch_bounds__(kThreadsPer, kMinBlocks) k_batch(const BatchLa
   __shared__ int ok;
   __shared__ int steps;
   const int L = p.tile_qubits;
+  const uint32_t tiles_s = static_cast<uint32_t>(__cvta_generic_to_shared(tiles));
   for (;;) {
     if (threadIdx.x == 0) item = *reinterpret_cast<volatile int*>(p.status) ? p.count : atomicAdd(p.queue, 1u);
     __syncthreads();
@@ -445,7 +465,7 @@ __global__ void __launch_bounds__(kThreadsPer, kMinBlocks) k_batch(const BatchLa
         build_tables(tab, steps, gates, n, c.form, entangler);
         __syncthreads();
         for (int si = 0; si < steps; ++si) {
-          run_step(tiles, n, tab, si, c.form, entangler, map);
+          run_step(tiles_s, n, tab, si, c.form, entangler, map);
           __syncthreads();
         }
       }
@@ -546,7 +566,7 @@ __global__ void __launch_bounds__(kThreadsPer, kMinBlocks) k_batch(const BatchLa
       const TileMap map = map_of(t);
       unsigned char* cur = buf[two ? k : 0];
       for (int si = 0; si < steps; ++si) {
-        run_step(cur, Lw, tab, si, c.form, entangler, map);
+        run_step(tiles_s + uint32_t(cur - tiles), Lw, tab, si, c.form, entangler, map);
         __syncthreads();
       }
       if (last) {
