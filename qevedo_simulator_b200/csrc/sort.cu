@@ -37,26 +37,58 @@ __global__ void __launch_bounds__(kThreads) k_hist(const uint64_t* __restrict__ 
   hist[size_t(threadIdx.x) * tiles + blockIdx.x] = counts[threadIdx.x];
 }
 
-// Exclusive scan of `count` values in place, one block of 1024 threads.
+// Exclusive scan of `count` values in place, one block of 1024 threads, 4096
+// consecutive values at a time, the next ones loaded while these are scanned
+// (a contiguous segment per thread, read with a stride between lanes, took
+// 53 us for a million keys' 62,720 values).
 __global__ void __launch_bounds__(1024) k_scan(uint32_t* __restrict__ v, size_t count) {
-  __shared__ uint32_t part[1024];
-  const size_t per = (count + 1023) / 1024;
-  const size_t first = size_t(threadIdx.x) * per;
-  uint32_t sum = 0;
-  for (size_t i = first; i < first + per && i < count; ++i) sum += v[i];
-  part[threadIdx.x] = sum;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const uint32_t add = threadIdx.x >= unsigned(o) ? part[threadIdx.x - o] : 0u;
+  __shared__ uint32_t warp_sums[2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto load = [&](size_t first) {
+    const size_t i = first + size_t(threadIdx.x) * 4;
+    uint4 x = make_uint4(0, 0, 0, 0);
+    if (i + 4 <= count) {
+      x = *reinterpret_cast<const uint4*>(v + i);
+    } else if (i < count) {
+      x.x = v[i];
+      if (i + 1 < count) x.y = v[i + 1];
+      if (i + 2 < count) x.z = v[i + 2];
+    }
+    return x;
+  };
+  uint32_t before = 0;
+  uint4 ahead = load(0);
+  int turn = 0;
+  for (size_t first = 0; first < count; first += 4096, turn ^= 1) {
+    const uint4 x = ahead;
+    if (first + 4096 < count) ahead = load(first + 4096);
+    const uint32_t sum = x.x + x.y + x.z + x.w;
+    uint32_t run = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += y;
+    }
+    if (lane == 31) warp_sums[turn][warp] = run;
     __syncthreads();
-    part[threadIdx.x] += add;
-    __syncthreads();
-  }
-  uint32_t run = part[threadIdx.x] - sum;  // exclusive prefix of this segment
-  for (size_t i = first; i < first + per && i < count; ++i) {
-    const uint32_t x = v[i];
-    v[i] = run;
-    run += x;
+    const uint32_t mine = warp_sums[turn][lane];
+    uint32_t all = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, all, o);
+      if (lane >= o) all += y;
+    }
+    const uint32_t base = before + __shfl_sync(0xffffffffu, all - mine, warp) + run - sum;
+    before += __shfl_sync(0xffffffffu, all, 31);
+    const size_t i = first + size_t(threadIdx.x) * 4;
+    const uint4 out = make_uint4(base, base + x.x, base + x.x + x.y, base + x.x + x.y + x.z);
+    if (i + 4 <= count) {
+      *reinterpret_cast<uint4*>(v + i) = out;
+    } else if (i < count) {
+      v[i] = out.x;
+      if (i + 1 < count) v[i + 1] = out.y;
+      if (i + 2 < count) v[i + 2] = out.z;
+    }
   }
 }
 
