@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kThreads) k_dense(cplx_t<T>* __restrict__ psi,
 struct LaneGeom {
   uint64_t rows;           // warp rows of 32 amplitudes the controls select
   uint64_t control_value;  // control bits that must be 1
-  uint8_t fixed[40];       // bits 0-4 and the control positions, ascending
+  uint8_t fixed[40];       // the control positions in the row's number, ascending
   int32_t num_fixed;
   uint8_t targets[4];      // target positions (matrix bit order), all below 5
 };
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_lanes(cplx_t<T>* __restrict_
     cplx_t<T> x[R];
 #pragma unroll
     for (int q = 0; q < R; ++q) {
-      base[q] = w0 + q < g.rows ? (insert_zeros(w0 + q, fixed, g.num_fixed) | g.control_value) + lane : ~uint64_t(0);
+      base[q] = w0 + q < g.rows ? ((insert_zeros(w0 + q, fixed, g.num_fixed) << 5) | g.control_value) + lane : ~uint64_t(0);
       if (base[q] != ~uint64_t(0)) x[q] = psi[base[q]];
     }
 #pragma unroll
@@ -599,11 +599,8 @@ void lanes_pick(StateImpl& s, const PlainGate& pg, uint64_t control_value, const
   LaneGeom g{};
   g.rows = uint64_t(1) << (s.n - 5 - ctrl.size());
   g.control_value = control_value;
-  std::vector<uint8_t> fixed = {0, 1, 2, 3, 4};
-  fixed.insert(fixed.end(), ctrl.begin(), ctrl.end());
-  std::sort(fixed.begin(), fixed.end());
-  g.num_fixed = int(fixed.size());
-  for (size_t i = 0; i < fixed.size(); ++i) g.fixed[i] = fixed[i];
+  g.num_fixed = int(ctrl.size());  // ascending
+  for (size_t i = 0; i < ctrl.size(); ++i) g.fixed[i] = uint8_t(ctrl[i] - 5);
   for (size_t j = 0; j < pg.targets.size(); ++j) g.targets[j] = uint8_t(pg.targets[j]);
   switch (pg.targets.size()) {
     case 1: return lanes_launch<T, 1>(s, g, mat);
