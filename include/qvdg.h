@@ -113,7 +113,7 @@ typedef struct {
   uint64_t passes;      /* full passes over the state (stages + relabels, or one per fused op) */
   uint64_t stages;      /* staged passes */
   double gate_seconds;  /* device time of the gate work (CUDA events) */
-  double bytes;         /* algorithmic HBM bytes of the gate work */
+  double bytes;         /* algorithmic HBM bytes of the gate work (diagonal passes that shared one counted once) */
   qvdg_options settings; /* the settings the run's plan was built with (planner = GREEDY: the learned pick
                           * or the caller's own) */
 } qvdg_stats;
@@ -135,7 +135,11 @@ const char* qvdg_version(void);
 qvdg_status qvdg_state_create(uint32_t num_qubits, uint32_t precision_bits, qvdg_state** out);
 
 /* Free the state and its device memory (reference: Drop of Buffer,
- * src/memory.rs:91-96). NULL is accepted. */
+ * src/memory.rs:91-96). NULL is accepted. The stream, events, workspaces and
+ * buffers of small states (at most 16 MB of amplitudes, 32 MB of workspace
+ * and 8 MB of pinned memory each, of four states) are kept for the next
+ * qvdg_state_create on the device and given back when an allocation of this
+ * library would fail without them. */
 qvdg_status qvdg_state_destroy(qvdg_state* state);
 
 /* Set the state to |0...0> and the identity layout. */
@@ -421,7 +425,9 @@ qvdg_status qvdg_batch_tuning(const qvdg_batch* batch, uint32_t* tile_qubits, ui
                               size_t capacity, size_t* count);
 
 /* Record the device time of every pass of later gate runs on this state
- * (off by default; the reference's timing counters, src/simulator.rs:128-146). */
+ * (off by default; the reference's timing counters, src/simulator.rs:128-146).
+ * While it is on, every pass is launched by itself; otherwise diagonal
+ * passes that nothing between them holds back share one. */
 qvdg_status qvdg_set_pass_timing(qvdg_state* state, int32_t enabled);
 
 /* Per-pass device seconds, algorithmic bytes and kind (1 staged tile pass,

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <memory>
@@ -41,17 +42,124 @@ struct qvdg_plan {
 
 namespace qvdg {
 
+namespace {
+
+// What a destroyed state leaves for the next one: its stream, events, status
+// word, workspaces, pinned staging and, where they are small, amplitudes.
+// Making and freeing them (above all the pinned memory, one to three
+// milliseconds) cost a statevector() of a few qubits ten times its gates.
+// At most kPoolStates of them wait, each within the limits below; a failing
+// allocation of this library gives them all back first. The pool itself is
+// never destroyed: the driver frees what is left at process exit.
+struct StateResources {
+  int device = 0;
+  void* amp = nullptr;
+  size_t amp_capacity = 0;
+  int* status = nullptr;
+  cudaStream_t stream = nullptr;
+  cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
+  DeviceScratch work, work2;
+  HostScratch host;
+};
+
+constexpr size_t kPoolStates = 4;
+constexpr size_t kPoolAmp = size_t(16) << 20, kPoolWork = size_t(16) << 20, kPoolHost = size_t(8) << 20;
+
+std::mutex g_pool_mutex;
+std::vector<StateResources>& pool() {
+  static auto* p = new std::vector<StateResources>();
+  return *p;
+}
+
+void free_resources(StateResources& r) {
+  if (r.amp) cudaFree(r.amp);
+  if (r.status) cudaFree(r.status);
+  r.work.release();
+  r.work2.release();
+  r.host.release();
+  if (r.ev_start) cudaEventDestroy(r.ev_start);
+  if (r.ev_stop) cudaEventDestroy(r.ev_stop);
+  if (r.stream) cudaStreamDestroy(r.stream);
+  r = StateResources();
+}
+
+// Resources on `device`, the smallest that hold `bytes` of amplitudes if any
+// do; false when none wait.
+bool take_resources(int device, size_t bytes, StateResources& out) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  auto& p = pool();
+  size_t best = p.size();
+  for (size_t i = 0; i < p.size(); ++i) {
+    if (p[i].device != device) continue;
+    const bool fits = p[i].amp_capacity >= bytes;
+    if (best == p.size() || (fits && (p[best].amp_capacity < bytes || p[i].amp_capacity < p[best].amp_capacity)))
+      best = i;
+  }
+  if (best == p.size()) return false;
+  out = p[best];
+  p.erase(p.begin() + long(best));
+  // Handles that a device reset has made invalid are dropped.
+  if (cudaStreamQuery(out.stream) != cudaSuccess) {
+    cudaGetLastError();
+    out = StateResources();
+    return false;
+  }
+  return true;
+}
+
+// The stream is idle.
+void give_resources(StateResources& r) {
+  if (r.amp_capacity > kPoolAmp) {
+    cudaFree(r.amp);
+    r.amp = nullptr;
+    r.amp_capacity = 0;
+  }
+  if (r.work.bytes > kPoolWork) r.work.release();
+  if (r.work2.bytes > kPoolWork) r.work2.release();
+  if (r.host.bytes > kPoolHost) r.host.release();
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (pool().size() < kPoolStates) {
+      pool().push_back(r);
+      r = StateResources();
+    }
+  }
+  free_resources(r);
+}
+
+// Gives back everything that waits; false when nothing did.
+bool drain_resources() {
+  std::vector<StateResources> all;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    all.swap(pool());
+  }
+  for (StateResources& r : all) free_resources(r);
+  return !all.empty();
+}
+
+}  // namespace
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+  cudaError_t err = cudaMalloc(p, bytes);
+  if (err != cudaSuccess) {
+    cudaGetLastError();
+    if (drain_resources()) err = cudaMalloc(p, bytes);
+    if (err != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+    }
+  }
+  return err;
+}
+
 void* DeviceScratch::get(size_t need) {
   if (need == 0) need = 1;
   if (need <= bytes) return ptr;
   release();
   size_t want = std::max(need, bytes * 2);
-  if (cudaMalloc(&ptr, want) != cudaSuccess) {
-    cudaGetLastError();
-    ptr = nullptr;
-    if (cudaMalloc(&ptr, need) != cudaSuccess) {
-      cudaGetLastError();
-      ptr = nullptr;
+  if (device_malloc(&ptr, want) != cudaSuccess) {
+    if (device_malloc(&ptr, need) != cudaSuccess) {
       bytes = 0;
       throw Error(QVDG_ERR_OUT_OF_MEMORY, "device workspace allocation failed");
     }
@@ -187,9 +295,7 @@ void upload_plan(const Program& p, uint32_t precision_bits, void** device, Devic
     std::memcpy(h.data() + align(gate_bytes), up.mats.data(), mat_bytes);
   }
   if (!up.tc.empty()) std::memcpy(h.data() + align(gate_bytes) + align(mat_bytes), up.tc.data(), up.tc.size());
-  if (cudaMalloc(device, h.size()) != cudaSuccess) {
-    cudaGetLastError();
-    *device = nullptr;
+  if (device_malloc(device, h.size()) != cudaSuccess) {
     throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate the plan's device memory");
   }
   QVDG_CUDA(cudaMemcpy(*device, h.data(), h.size(), cudaMemcpyHostToDevice));
@@ -275,22 +381,37 @@ qvdg_status qvdg_state_create(uint32_t num_qubits, uint32_t precision_bits, qvdg
       QVDG_CUDA(cudaGetDevice(&s.device));
       QVDG_CUDA(cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, s.device));
       s.amp_bytes = size_t(s.elem_bytes()) << num_qubits;
-      if (cudaMalloc(&s.amp, s.amp_bytes) != cudaSuccess) {
-        cudaGetLastError();
+      StateResources r;
+      const bool pooled = take_resources(s.device, s.amp_bytes, r);
+      s.amp = r.amp;
+      s.amp_capacity = r.amp_capacity;
+      s.status = r.status;
+      s.stream = r.stream;
+      s.ev_start = r.ev_start;
+      s.ev_stop = r.ev_stop;
+      s.work = r.work;
+      s.work2 = r.work2;
+      s.host = r.host;
+      if (s.amp_capacity < s.amp_bytes) {
+        if (s.amp) cudaFree(s.amp);
         s.amp = nullptr;
-        throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate " + std::to_string(s.amp_bytes) +
-                                                " bytes of device memory for " + std::to_string(num_qubits) +
-                                                " qubits");
+        s.amp_capacity = 0;
+        if (device_malloc(&s.amp, s.amp_bytes) != cudaSuccess)
+          throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate " + std::to_string(s.amp_bytes) +
+                                                  " bytes of device memory for " + std::to_string(num_qubits) +
+                                                  " qubits");
+        s.amp_capacity = s.amp_bytes;
       }
-      if (cudaMalloc(&s.status, 256) != cudaSuccess) {
-        cudaGetLastError();
-        s.status = nullptr;
-        throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate the state's status word");
+      if (!pooled) {
+        void* status = nullptr;
+        if (device_malloc(&status, 256) != cudaSuccess)
+          throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate the state's status word");
+        s.status = static_cast<int*>(status);
+        QVDG_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+        QVDG_CUDA(cudaEventCreate(&s.ev_start));
+        QVDG_CUDA(cudaEventCreate(&s.ev_stop));
       }
-      QVDG_CUDA(cudaMemset(s.status, 0, 256));
-      QVDG_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
-      QVDG_CUDA(cudaEventCreate(&s.ev_start));
-      QVDG_CUDA(cudaEventCreate(&s.ev_stop));
+      QVDG_CUDA(cudaMemsetAsync(s.status, 0, 256, s.stream));
       s.layout.resize(num_qubits);
       for (uint32_t q = 0; q < num_qubits; ++q) s.layout[q] = q;
       launch_zero(s);
@@ -307,16 +428,24 @@ qvdg_status qvdg_state_create(uint32_t num_qubits, uint32_t precision_bits, qvdg
 qvdg_status qvdg_state_destroy(qvdg_state* st) {
   if (!st) return QVDG_OK;
   StateImpl& s = st->s;
-  if (s.stream) cudaStreamSynchronize(s.stream);
-  if (s.amp) cudaFree(s.amp);
-  if (s.status) cudaFree(s.status);
-  s.work.release();
-  s.work2.release();
-  s.host.release();
+  const bool idle = s.stream && cudaStreamSynchronize(s.stream) == cudaSuccess;
   for (cudaEvent_t e : s.pass_events) cudaEventDestroy(e);
-  if (s.ev_start) cudaEventDestroy(s.ev_start);
-  if (s.ev_stop) cudaEventDestroy(s.ev_stop);
-  if (s.stream) cudaStreamDestroy(s.stream);
+  StateResources r;
+  r.device = s.device;
+  r.amp = s.amp;
+  r.amp_capacity = s.amp_capacity;
+  r.status = s.status;
+  r.stream = s.stream;
+  r.ev_start = s.ev_start;
+  r.ev_stop = s.ev_stop;
+  r.work = s.work;
+  r.work2 = s.work2;
+  r.host = s.host;
+  // A state that was never whole, or whose device has failed, leaves nothing.
+  if (idle && s.status && s.ev_stop)
+    give_resources(r);
+  else
+    free_resources(r);
   delete st;
   return QVDG_OK;
 }

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "batch.hpp"
+#include "engine.hpp"
 
 struct qvdg_batch {
   int device = 0;
@@ -155,7 +156,7 @@ BatchLaunch shape(qvdg_batch* b, const BatchLaunch& base, const std::vector<uint
   QVDG_CUDA(cudaStreamSynchronize(b->stream));
   if (*work) cudaFree(*work);
   *work = nullptr;
-  QVDG_CUDA(cudaMalloc(work, o_queue + queue_bytes));
+  QVDG_CUDA(device_malloc(work, o_queue + queue_bytes));
   char* d = static_cast<char*>(*work);
   QVDG_CUDA(cudaMemcpyAsync(d + o_tasks, w.tasks.data(), w.tasks.size() * sizeof(BatchTask), cudaMemcpyHostToDevice,
                             b->stream));
@@ -260,7 +261,7 @@ qvdg_batch* batch_create(const qvdg_layered_circuit* circuits, size_t count, con
     const size_t o_mats = align256(o_gates + std::max<size_t>(b->num_matrices, 1) * kBatchGateSlots * sizeof(float2));
     const size_t o_out = align256(o_mats + std::max<size_t>(matrices.size(), 1) * sizeof(double));
     const size_t total = o_out + b->outputs * sizeof(double);
-    QVDG_CUDA(cudaMalloc(&b->dev, total));
+    QVDG_CUDA(device_malloc(&b->dev, total));
     char* base = static_cast<char*>(b->dev);
     b->matrices = reinterpret_cast<double*>(base + o_mats);
     if (!matrices.empty())
@@ -297,13 +298,13 @@ qvdg_batch* batch_create(const qvdg_layered_circuit* circuits, size_t count, con
     }
     if (slots) {
       slots = std::min<size_t>(slots, std::max<size_t>(1, kSlotBudget / (slot_elems * sizeof(float2))));
-      while (cudaMalloc(&b->slots, slots * slot_elems * sizeof(float2)) != cudaSuccess) {
+      while (device_malloc(&b->slots, slots * slot_elems * sizeof(float2)) != cudaSuccess) {
         cudaGetLastError();
         b->slots = nullptr;
         if (slots == 1) throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate the batch's device memory");
         slots /= 2;
       }
-      QVDG_CUDA(cudaMalloc(&b->partials, std::max<size_t>(partials, 1) * sizeof(double)));
+      QVDG_CUDA(device_malloc(&b->partials, std::max<size_t>(partials, 1) * sizeof(double)));
     }
     whole.slots = static_cast<float2*>(b->slots);
     whole.partials = static_cast<double*>(b->partials);

@@ -11,6 +11,10 @@
 
 namespace qvdg {
 
+// cudaMalloc that first gives back what destroyed states left (api.cpp)
+// before it fails; *p is then null.
+cudaError_t device_malloc(void** p, size_t bytes);
+
 // A device buffer that grows on demand (never shrinks while its owner lives).
 struct DeviceScratch {
   void* ptr = nullptr;
@@ -57,6 +61,7 @@ struct StateImpl {
   int bits = 32;
   void* amp = nullptr;  // 2^n interleaved complex in `bits` precision
   size_t amp_bytes = 0;
+  size_t amp_capacity = 0;  // bytes allocated (a reused buffer may be larger)
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   std::vector<uint32_t> layout;  // logical -> physical

@@ -15,8 +15,7 @@
 #include <random>
 #include <vector>
 
-#include "common.cuh"
-#include "qvdg.h"
+#include "engine.hpp"
 
 struct qvdg_mlp {
   int device = 0;
@@ -196,7 +195,7 @@ void ensure(qvdg_mlp* m, size_t rows) {
   if (m->buf) cudaFree(m->buf);
   m->buf = nullptr;
   m->cap = 0;
-  QVDG_CUDA(cudaMalloc(&m->buf, acts_floats(rows, m->in, m->hid) * sizeof(float)));
+  QVDG_CUDA(device_malloc(reinterpret_cast<void**>(&m->buf), acts_floats(rows, m->in, m->hid) * sizeof(float)));
   m->cap = rows;
 }
 
@@ -265,7 +264,7 @@ qvdg_mlp* mlp_create(uint32_t in, uint32_t hid, uint64_t seed) {
     m->hid = hid;
     m->nparams = size_t(hid) * in + hid + size_t(hid) * hid + hid + hid + 1;
     QVDG_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
-    QVDG_CUDA(cudaMalloc(&m->params, 4 * m->nparams * sizeof(float)));
+    QVDG_CUDA(device_malloc(reinterpret_cast<void**>(&m->params), 4 * m->nparams * sizeof(float)));
     m->grads = m->params + m->nparams;
     m->adam_m = m->grads + m->nparams;
     m->adam_v = m->adam_m + m->nparams;
@@ -341,8 +340,8 @@ float mlp_train(qvdg_mlp* m, const float* x, const float* t, size_t rows, uint32
   // The whole data set stays on the device; batches are gathered rows.
   float *data = nullptr;
   uint32_t* idx = nullptr;
-  QVDG_CUDA(cudaMalloc(&data, rows * (m->in + 1) * sizeof(float)));
-  if (cudaMalloc(&idx, rows * sizeof(uint32_t)) != cudaSuccess) {
+  QVDG_CUDA(device_malloc(reinterpret_cast<void**>(&data), rows * (m->in + 1) * sizeof(float)));
+  if (device_malloc(reinterpret_cast<void**>(&idx), rows * sizeof(uint32_t)) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(data);
     throw Error(QVDG_ERR_OUT_OF_MEMORY, "cannot allocate the training index");

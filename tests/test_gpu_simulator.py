@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from conftest import max_distance, random_state
-from qevedo_simulator_b200 import Circuit, DeviceState, library, options, run, statevector
+from qevedo_simulator_b200 import Circuit, DeviceState, Gate, library, options, run, statevector
 
 pytestmark = pytest.mark.gpu
 
@@ -365,3 +365,37 @@ def test_sampler_is_bit_exact_around_blocks_of_chunks(oracle, bits, n):
         held = st.amplitudes()  # in the state's own precision
         got = st.sample_unordered(u)
     assert np.array_equal(got, oracle.sample_from_amplitudes(held, u, bits))
+
+
+@pytest.mark.parametrize("threads", [1, 6])
+def test_states_reuse_what_earlier_ones_left(threads):
+    """States made and destroyed by several threads at once, of sizes whose
+    buffers are kept, replaced or given back: each starts as |0...0> in the
+    identity layout with its own results, and what waits stays bounded."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from cuda.bindings import runtime as rt
+
+    def free_bytes():
+        return rt.cudaMemGetInfo()[1]
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        for _ in range(12):
+            n, bits = int(rng.choice([1, 3, 8, 14, 19, 21])), int(rng.choice([32, 64]))
+            with DeviceState(n, bits) as st:
+                assert st.layout() == list(range(n)) and st.norm_sqr() == 1.0 and st.probability_one(n - 1) == 0.0
+                st.apply(Gate("ry", (0.8,)).matrix(), [n - 1])
+                if n > 1:
+                    st.swap_physical([(0, n - 1)])
+                z = st.expect_z_all()
+                assert abs(z[n - 1] - np.cos(0.8)) < 1e-6 and np.all(np.abs(z[:n - 1] - 1.0) < 1e-6)
+                assert st.sample_unordered(rng.random(50)).max() <= 1 << (n - 1)
+        return True
+
+    with DeviceState(3, 32):
+        pass
+    before = free_bytes()
+    with ThreadPoolExecutor(threads) as pool:
+        assert all(pool.map(work, range(threads)))
+    assert before - free_bytes() <= 4 * (16 + 16 + 16 + 2) << 20
