@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <stdexcept>
 #include <string>
 
@@ -79,6 +80,18 @@ struct Error : std::runtime_error {
   } while (0)
 
 #define QVDG_LAUNCH_CHECK() QVDG_CUDA(cudaGetLastError())
+
+// Runs a kernel's set-up (its shared-memory limit) once per device.
+struct OncePerDevice {
+  std::atomic<uint64_t> done{0};
+  template <typename F>
+  void operator()(int device, F&& f) {
+    const uint64_t bit = device >= 0 && device < 64 ? uint64_t(1) << device : 0;
+    if (bit && (done.load(std::memory_order_acquire) & bit)) return;
+    f();
+    done.fetch_or(bit, std::memory_order_release);
+  }
+};
 
 inline int ceil_log2(uint64_t x) {
   int r = 0;

@@ -17,6 +17,7 @@
 
 #include <algorithm>
 
+#include "dense_wide.hpp"
 #include "engine.hpp"
 
 namespace qvdg {
@@ -33,10 +34,23 @@ struct DenseGeom {
   int32_t num_fixed;
 };
 
+// Threads of a k_dense block and the rows it computes at a time. From four
+// qubits on the multiply-adds count as much as HBM (six: 1.9 ms of them at
+// full rate for 28 qubits of complex64, 0.66 ms of HBM), and one whose three
+// operands are all new registers runs at two thirds of the rate. Two rows
+// (four for K = 4) at a time share each amplitude, two groups share each
+// matrix entry, and complex64 reads two entries at once; small blocks leave
+// the wide gates' registers three of them per SM. 28 qubits complex64: K = 4
+// 0.83-0.92 -> 0.82 ms, K = 5 1.70-1.85 -> 1.36, K = 6 3.28 -> 2.87.
+template <typename T, int K>
+constexpr int kDenseThreads = sizeof(T) == 4 && K >= 5 ? 128 : kThreads;
+template <typename T, int K>
+constexpr int kDenseRows = sizeof(T) == 4 ? (K == 4 ? 4 : 2) : 1;
+
 template <typename T, int K, int G, bool VEC>
-__global__ void __launch_bounds__(kThreads) k_dense(cplx_t<T>* __restrict__ psi, const DenseGeom g,
-                                                    const cplx_t<T>* __restrict__ mat) {
-  constexpr int D = 1 << K;
+__global__ void __launch_bounds__(kDenseThreads<T, K>, sizeof(T) == 4 && K >= 5 ? 3 : 1)
+    k_dense(cplx_t<T>* __restrict__ psi, const DenseGeom g, const cplx_t<T>* __restrict__ mat) {
+  constexpr int D = 1 << K, ROWS = kDenseRows<T, K>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx_t<T>* sm = reinterpret_cast<cplx_t<T>*>(smem_raw);
   __shared__ uint8_t fixed[40];
@@ -64,22 +78,43 @@ __global__ void __launch_bounds__(kThreads) k_dense(cplx_t<T>* __restrict__ psi,
         for (int q = 0; q < G; ++q) x[q][h] = psi[base[q] + g.offsets[h]];
     }
 #pragma unroll 1
-    for (int r = 0; r < D; ++r) {
-      cplx_t<T> acc[G];
+    for (int r = 0; r < D; r += ROWS) {
+      cplx_t<T> acc[ROWS][G];
 #pragma unroll
-      for (int q = 0; q < G; ++q) acc[q] = make_c<T>(T(0), T(0));
+      for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-      for (int c = 0; c < D; ++c) {
-        const cplx_t<T> m = sm[r * D + c];
+        for (int q = 0; q < G; ++q) acc[i][q] = make_c<T>(T(0), T(0));
+      if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int q = 0; q < G; ++q) cmac<T>(acc[q], m, x[q][c]);
-      }
-      if constexpr (VEC) {
-        *reinterpret_cast<float4*>(psi + base[0] + g.offsets[r]) =
-            make_float4(acc[0].x, acc[0].y, acc[G - 1].x, acc[G - 1].y);
+        for (int c = 0; c < D; c += 2) {
+          float4 m[ROWS];
+#pragma unroll
+          for (int i = 0; i < ROWS; ++i) m[i] = *reinterpret_cast<const float4*>(sm + (r + i) * D + c);
+#pragma unroll
+          for (int q = 0; q < G; ++q) {
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) cmac<T>(acc[i][q], make_float2(m[i].x, m[i].y), x[q][c]);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) cmac<T>(acc[i][q], make_float2(m[i].z, m[i].w), x[q][c + 1]);
+          }
+        }
       } else {
 #pragma unroll
-        for (int q = 0; q < G; ++q) psi[base[q] + g.offsets[r]] = acc[q];
+        for (int c = 0; c < D; ++c) {
+          const cplx_t<T> m = sm[r * D + c];
+#pragma unroll
+          for (int q = 0; q < G; ++q) cmac<T>(acc[0][q], m, x[q][c]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        if constexpr (VEC) {
+          *reinterpret_cast<float4*>(psi + base[0] + g.offsets[r + i]) =
+              make_float4(acc[i][0].x, acc[i][0].y, acc[i][G - 1].x, acc[i][G - 1].y);
+        } else {
+#pragma unroll
+          for (int q = 0; q < G; ++q) psi[base[q] + g.offsets[r + i]] = acc[i][q];
+        }
       }
     }
   }
@@ -559,24 +594,28 @@ unsigned grid_for(const StateImpl& s, uint64_t work_items) {
 
 template <typename T, int K, int G, bool VEC>
 void dense_launch(StateImpl& s, const DenseGeom& g, const void* mat) {
+  constexpr int threads = kDenseThreads<T, K>;
   const size_t smem = size_t(1) << (2 * K);
   const size_t bytes = smem * sizeof(cplx_t<T>);
-  static bool configured = false;  // per instantiation
-  if (!configured) {
+  static OncePerDevice once;  // per instantiation
+  once(s.device, [&] {
     QVDG_CUDA(cudaFuncSetAttribute(k_dense<T, K, G, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    configured = true;
-  }
-  k_dense<T, K, G, VEC><<<grid_for(s, g.n_iter / G), kThreads, bytes, s.stream>>>(
-      static_cast<cplx_t<T>*>(s.amp), g, static_cast<const cplx_t<T>*>(mat));
+  });
+  const uint64_t blocks = (g.n_iter / G + threads - 1) / threads;
+  const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(blocks, uint64_t(s.sms) * 16)));
+  k_dense<T, K, G, VEC><<<grid, threads, bytes, s.stream>>>(static_cast<cplx_t<T>*>(s.amp), g,
+                                                            static_cast<const cplx_t<T>*>(mat));
   QVDG_LAUNCH_CHECK();
 }
 
 template <typename T, int K>
 void dense_pick(StateImpl& s, const DenseGeom& g, const void* mat, bool bit0_free) {
-  if constexpr (K <= 4) {
+  // Two groups per thread (two neighbours as one 16-byte load) as far as
+  // their amplitudes fit the registers.
+  if constexpr (K <= 4 || (K == 5 && sizeof(T) == 4)) {
     if (g.n_iter >= 2) {
-      if (sizeof(T) == 4 && bit0_free)
-        return dense_launch<T, K, 2, true>(s, g, mat);
+      if constexpr (sizeof(T) == 4)
+        if (bit0_free) return dense_launch<T, K, 2, true>(s, g, mat);
       return dense_launch<T, K, 2, false>(s, g, mat);
     }
   }
@@ -721,6 +760,9 @@ void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices) {
       return;
     }
   }
+  // 5-6 qubits: matrix products on tiles, unless too few amplitudes are
+  // selected for one.
+  if (launch_dense_wide(s, pg, mat)) return;
   switch (k) {
     case 1: return dense_pick<T, 1>(s, g, mat, bit0_free);
     case 2: return dense_pick<T, 2>(s, g, mat, bit0_free);

@@ -603,6 +603,33 @@ def test_shared_diagonal_passes_equal_separate_ones(oracle, bits, n):
             assert max_distance(got[0][0], expected) < {32: 1e-5, 64: 1e-11}[bits]
 
 
+@pytest.mark.parametrize("bits, n", [(32, 10), (32, 11), (32, 12), (32, 16), (32, 22), (64, 9), (64, 10), (64, 11),
+                                     (64, 21)])
+def test_wide_dense_gates_as_tile_products(oracle, bits, n):
+    """5- and 6-qubit gates below, at and above the smallest tile and on the
+    large tiles: targets low, high, spread and unordered, with and without
+    controls (bit 0 among them)."""
+    rng = np.random.default_rng(n * bits)
+    psi = random_state(rng, n)
+    cases = []
+    for k in (5, 6):
+        cases += [(list(range(k)), []), (list(range(n - k, n))[::-1], []), ([0] + list(range(n - k + 1, n)), [])]
+        for c in (0, 1, 3):
+            if k + c <= n:
+                qs = random_qubits(rng, n, k + c)
+                cases.append((qs[:k], [(q, bool(rng.integers(0, 2))) for q in qs[k:]]))
+        if n > k:
+            cases.append((random_qubits(rng, n - 1, k), []))
+            cases[-1] = ([q + 1 for q in cases[-1][0]], [(0, True)])
+    with DeviceState(n, bits) as st:
+        for targets, controls in cases:
+            m = random_unitary(rng, len(targets))
+            st.set_amplitudes(psi)
+            st.apply(m, targets, controls)
+            expected = oracle.naive_statevector([Op(targets, controls, m)], n, initial=psi)
+            assert max_distance(st.amplitudes(), expected) < TOL[bits], (targets, controls)
+
+
 @pytest.mark.parametrize("bits", [32, 64])
 @pytest.mark.parametrize("n", [5, 9, 13, 14])
 def test_register_stage_gate_forms(oracle, bits, n):
