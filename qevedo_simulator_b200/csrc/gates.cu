@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kThreads) k_diag_run(cplx_t<T>* __restrict__ p
 // moves is read and written once, as long as both accesses are coalesced):
 // a swap of a low bit with a high one scatters single amplitudes, 8 bytes
 // of a 32-byte sector. So a block moves whole tiles: the tile's bits are the
-// low `m` bits, their images under pi, and more bits up to kSwapTileBits,
+// low `m` bits, their images under pi, and more bits up to kSwapMaxBits,
 // closed under pi. Then pi maps tile t to the tile t' whose index bits are
 // swapped and element e of it to image(e), and a block reads both tiles of a
 // pair as rows of 2^m contiguous amplitudes (256 bytes), and writes each
@@ -450,8 +450,12 @@ __global__ void __launch_bounds__(kThreads) k_diag_run(cplx_t<T>* __restrict__ p
 // plus constants.
 // Tiles of 16 KB: with 8 KB ones a complex64 pass ran at 0.51-0.54 of the
 // copy rate (complex128, 16 KB, at 0.76-0.83).
-constexpr int kSwapTileBits = 11;  // most (complex64); 10 for complex128
-constexpr int kSwapElems = (1 << kSwapTileBits) / kThreads;
+// A complex64 state of 2^32 bytes or more whose rows scatter (four low bits
+// or more leave the row) takes 512-byte rows and 32 KB tiles instead: half as
+// many pages a byte (30 qubits, random swaps 5.2 -> 3.8 ms); one block per SM
+// makes them slower elsewhere (27 qubits 0.40 -> 0.49 ms).
+constexpr int kSwapMaxBits = 12;
+constexpr int kSwapElems = 8;  // of a tile per thread (complex128: 4)
 
 struct SwapGeom {
   uint64_t tiles;                 // 2^(n - k)
@@ -459,10 +463,10 @@ struct SwapGeom {
   int32_t np;                     // swapped pairs of tile-index bits
   int32_t moves;                  // image is not the identity
   uint8_t a[32], b[32];           // those pairs
-  uint8_t fixed[kSwapTileBits];   // the tile's physical bits, ascending
-  uint8_t bit[kSwapTileBits];     // physical bit of element bit i (the low m ones are 0..m-1)
-  uint8_t image[kSwapTileBits];   // element bit that element bit i moves to
-  // Element i * kThreads: its offset in the state, its place in shared
+  uint8_t fixed[kSwapMaxBits];   // the tile's physical bits, ascending
+  uint8_t bit[kSwapMaxBits];     // physical bit of element bit i (the low m ones are 0..m-1)
+  uint8_t image[kSwapMaxBits];   // element bit that element bit i moves to
+  // Element i * threads: its offset in the state, its place in shared
   // memory and the place of its image.
   uint64_t off[kSwapElems];
   uint16_t pos[kSwapElems], from[kSwapElems];
@@ -472,13 +476,14 @@ __host__ __device__ __forceinline__ uint32_t swap_pos(uint32_t e, int m) {
   return e ^ ((e >> m) & ((1u << m) - 1u));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_swap_bits(cplx_t<T>* __restrict__ psi,
+template <typename T, int kSwapThreads>
+__global__ void __launch_bounds__(kSwapThreads) k_swap_bits(cplx_t<T>* __restrict__ psi,
                                                         const __grid_constant__ SwapGeom g) {
   constexpr int E = sizeof(T) == 4 ? kSwapElems : kSwapElems / 2;  // elements of a tile per thread
-  __shared__ cplx_t<T> buf[2][E * kThreads];
-  __shared__ uint8_t fixed[kSwapTileBits];
-  if (threadIdx.x < kSwapTileBits) fixed[threadIdx.x] = g.fixed[threadIdx.x];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx_t<T>(*buf)[E * kSwapThreads] = reinterpret_cast<cplx_t<T>(*)[E * kSwapThreads]>(smem_raw);
+  __shared__ uint8_t fixed[kSwapMaxBits];
+  if (threadIdx.x < kSwapMaxBits) fixed[threadIdx.x] = g.fixed[threadIdx.x];
   __syncthreads();
   uint64_t off = 0;
   uint32_t x0 = 0;
@@ -487,7 +492,7 @@ __global__ void __launch_bounds__(kThreads) k_swap_bits(cplx_t<T>* __restrict__ 
     x0 |= ((threadIdx.x >> j) & 1u) << g.image[j];
   }
   const uint32_t pos = swap_pos(threadIdx.x, g.m), from = swap_pos(x0, g.m);
-  auto live = [&](int i) { return threadIdx.x + uint32_t(i) * kThreads < (1u << g.k); };
+  auto live = [&](int i) { return threadIdx.x + uint32_t(i) * kSwapThreads < (1u << g.k); };
   auto partner = [&](uint64_t t) {
     uint64_t t2 = t;
     for (int p = 0; p < g.np; ++p) {
@@ -849,9 +854,13 @@ void launch_swap_bits(StateImpl& s, const std::vector<std::pair<uint32_t, uint32
   for (uint32_t q = 0; q < s.n; ++q) pi[q] = q;
   for (auto& pr : pairs) std::swap(pi[pr.first], pi[pr.second]);
   SwapGeom g{};
-  // 256-byte rows, 16 KB tiles.
-  const uint32_t m = std::min<uint32_t>(s.bits == 32 ? 5 : 4, s.n);
-  const uint32_t most = std::min<uint32_t>(s.bits == 32 ? kSwapTileBits : kSwapTileBits - 1, s.n);
+  // 256-byte rows and 16 KB tiles, or 512 bytes and 32 KB.
+  int scattered = 0;
+  for (uint32_t q = 0; q < 5 && q < s.n; ++q) scattered += pi[q] > 5 ? 1 : 0;
+  const bool large = s.bits == 32 && s.amp_bytes >= (size_t(1) << 32) && scattered >= 4;
+  const uint32_t m = std::min<uint32_t>(s.bits == 32 ? (large ? 6 : 5) : 4, s.n);
+  const uint32_t most = std::min<uint32_t>(s.bits == 32 ? (large ? 12 : 11) : 10, s.n);
+  const uint32_t threads = large ? 512 : 256;
   // Element bits: the low bits, each one's image outside them next to it
   // (row bit i for low bit i as far as that goes), then more bits or pairs.
   std::vector<uint32_t> bits;
@@ -902,14 +911,14 @@ void launch_swap_bits(StateImpl& s, const std::vector<std::pair<uint32_t, uint32
     g.image[i] = uint8_t(std::find(bits.begin(), bits.end(), pi[bits[i]]) - bits.begin());
     if (pi[bits[i]] != bits[i]) g.moves = 1;
   }
-  for (uint32_t i = 0; i < uint32_t(kSwapElems) && i * kThreads < (1u << g.k); ++i) {
+  for (uint32_t i = 0; i < uint32_t(kSwapElems) && i * threads < (1u << g.k); ++i) {
     uint32_t image = 0;
     for (int j = 0; j < g.k; ++j)
-      if ((i * kThreads >> j) & 1u) {
+      if ((i * threads >> j) & 1u) {
         g.off[i] |= uint64_t(1) << g.bit[j];
         image |= 1u << g.image[j];
       }
-    g.pos[i] = uint16_t(swap_pos(i * kThreads, g.m));
+    g.pos[i] = uint16_t(swap_pos(i * threads, g.m));
     g.from[i] = uint16_t(swap_pos(image, g.m));
   }
   // Tile-index bit of a physical bit outside the tile.
@@ -925,10 +934,18 @@ void launch_swap_bits(StateImpl& s, const std::vector<std::pair<uint32_t, uint32
       ++g.np;
     }
   const unsigned grid = unsigned(std::min<uint64_t>(g.tiles, uint64_t(s.sms) * 16));
-  if (s.bits == 32)
-    k_swap_bits<float><<<grid, kThreads, 0, s.stream>>>(static_cast<float2*>(s.amp), g);
-  else
-    k_swap_bits<double><<<grid, kThreads, 0, s.stream>>>(static_cast<double2*>(s.amp), g);
+  const size_t smem = size_t(large ? 64 : 32) << 10;  // two tiles
+  if (large) {
+    static OncePerDevice once;
+    once(s.device, [&] {
+      QVDG_CUDA(cudaFuncSetAttribute(k_swap_bits<float, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    });
+    k_swap_bits<float, 512><<<grid, 512, smem, s.stream>>>(static_cast<float2*>(s.amp), g);
+  } else if (s.bits == 32) {
+    k_swap_bits<float, 256><<<grid, 256, smem, s.stream>>>(static_cast<float2*>(s.amp), g);
+  } else {
+    k_swap_bits<double, 256><<<grid, 256, smem, s.stream>>>(static_cast<double2*>(s.amp), g);
+  }
   QVDG_LAUNCH_CHECK();
 }
 

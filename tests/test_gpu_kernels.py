@@ -658,3 +658,32 @@ def test_register_stage_gate_forms(oracle, bits, n):
             stats = st.apply_ops(ops, options(4, True))
             assert stats["stages"] > 0
             assert max_distance(st.amplitudes(), expected) < {32: 1e-5, 64: 1e-11}[bits]
+
+
+def test_swap_passes_of_a_large_state():
+    """The large tiles of a 4 GiB state whose rows scatter: every amplitude at
+    its place, and back again."""
+    import torch
+
+    n = 29
+    st = DeviceState(n, 32)
+    pointer, _ = st.device_buffer()
+
+    class Buffer:
+        __cuda_array_interface__ = {"shape": (1 << n,), "data": (pointer, False), "version": 3, "typestr": "<c8"}
+
+    view = torch.as_tensor(Buffer(), device="cuda")
+    torch.view_as_real(view)[:, 0] = torch.arange(1 << n, device="cuda", dtype=torch.int32).view(torch.float32)
+    torch.view_as_real(view)[:, 1] = 0
+    pairs = [(0, 28), (1, 9), (2, 17), (3, 23), (4, 11), (5, 6), (7, 26), (12, 13)]
+    torch.cuda.synchronize()
+    st.swap_physical(pairs)
+    index = torch.arange(1 << n, device="cuda", dtype=torch.int64)
+    for a, b in pairs:
+        d = ((index >> a) ^ (index >> b)) & 1
+        index ^= (d << a) | (d << b)
+    held = torch.view_as_real(view)[:, 0].view(torch.int32)
+    assert torch.equal(held, index.to(torch.int32))
+    st.swap_physical(pairs)
+    assert torch.equal(held, torch.arange(1 << n, device="cuda", dtype=torch.int32))
+    st.close()
