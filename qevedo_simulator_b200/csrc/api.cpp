@@ -59,7 +59,8 @@ struct StateResources {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   DeviceScratch work, work2;
-  HostScratch host;
+  HostScratch host, stage;
+  cudaEvent_t stage_event[2] = {nullptr, nullptr};
 };
 
 constexpr size_t kPoolStates = 4;
@@ -77,6 +78,9 @@ void free_resources(StateResources& r) {
   r.work.release();
   r.work2.release();
   r.host.release();
+  r.stage.release();
+  for (cudaEvent_t e : r.stage_event)
+    if (e) cudaEventDestroy(e);
   if (r.ev_start) cudaEventDestroy(r.ev_start);
   if (r.ev_stop) cudaEventDestroy(r.ev_stop);
   if (r.stream) cudaStreamDestroy(r.stream);
@@ -392,6 +396,8 @@ qvdg_status qvdg_state_create(uint32_t num_qubits, uint32_t precision_bits, qvdg
       s.work = r.work;
       s.work2 = r.work2;
       s.host = r.host;
+      s.stage = r.stage;
+      std::copy(r.stage_event, r.stage_event + 2, s.stage_event);
       if (s.amp_capacity < s.amp_bytes) {
         if (s.amp) cudaFree(s.amp);
         s.amp = nullptr;
@@ -441,6 +447,8 @@ qvdg_status qvdg_state_destroy(qvdg_state* st) {
   r.work = s.work;
   r.work2 = s.work2;
   r.host = s.host;
+  r.stage = s.stage;
+  std::copy(s.stage_event, s.stage_event + 2, r.stage_event);
   // A state that was never whole, or whose device has failed, leaves nothing.
   if (idle && s.status && s.ev_stop)
     give_resources(r);
@@ -479,7 +487,7 @@ qvdg_status qvdg_state_set_amplitudes(qvdg_state* st, const double* amplitudes, 
     for (uint64_t first = 0; first < count; first += chunk) {
       const uint64_t c = std::min<uint64_t>(chunk, count - first);
       double* d = static_cast<double*>(s.work.get(c * 16));
-      QVDG_CUDA(cudaMemcpyAsync(d, amplitudes + 2 * first, c * 16, cudaMemcpyHostToDevice, s.stream));
+      copy_to_device(s, d, amplitudes + 2 * first, c * 16);
       launch_import(s, first, c, d);
       QVDG_CUDA(cudaStreamSynchronize(s.stream));
     }
@@ -496,8 +504,7 @@ qvdg_status qvdg_state_get_amplitudes(const qvdg_state* cst, double* amplitudes,
       const uint64_t c = std::min<uint64_t>(chunk, count - first);
       double* d = static_cast<double*>(s.work.get(c * 16));
       launch_export(s, first, c, d);
-      QVDG_CUDA(cudaMemcpyAsync(amplitudes + 2 * first, d, c * 16, cudaMemcpyDeviceToHost, s.stream));
-      QVDG_CUDA(cudaStreamSynchronize(s.stream));
+      copy_to_host(s, amplitudes + 2 * first, d, c * 16);
     }
   });
 }

@@ -72,6 +72,8 @@ struct StateImpl {
   DeviceScratch work;            // device workspace (uploads, reductions, sampling)
   DeviceScratch work2;
   HostScratch host;              // pinned staging
+  HostScratch stage;             // pinned chunks of large copies (transfer.cpp),
+  cudaEvent_t stage_event[2] = {nullptr, nullptr};  // and the last copy of each
   int device = 0;
   int sms = 148;
   int* status = nullptr;  // device word set by kernels whose bounded waits gave up
@@ -108,6 +110,13 @@ void launch_zero(StateImpl& s);
 void launch_export(StateImpl& s, uint64_t first, uint64_t count, double* out_dev);
 void launch_import(StateImpl& s, uint64_t first, uint64_t count, const double* in_dev);
 void launch_scale(StateImpl& s, double factor);
+
+// ---- transfer.cpp
+// Copies between the device and a caller's memory, in order on the state's
+// stream; copy_to_host is complete on return, copy_to_device's source must
+// stay until the stream has been waited for.
+void copy_to_host(StateImpl& s, void* dst, const void* src, size_t bytes);
+void copy_to_device(StateImpl& s, void* dst, const void* src, size_t bytes);
 
 // ---- measure.cu
 double norm_sqr(StateImpl& s);

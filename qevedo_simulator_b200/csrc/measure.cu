@@ -701,8 +701,7 @@ void probabilities_t(StateImpl& s, double* out_host) {
     k_probs<T><<<unsigned(umin64(blocks_for(count, kThreads), uint64_t(s.sms) * 16)), kThreads, 0,
                  s.stream>>>(static_cast<const cplx_t<T>*>(s.amp), d, first, count, tables, nt);
     QVDG_LAUNCH_CHECK();
-    QVDG_CUDA(cudaMemcpyAsync(out_host + first, d, count * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
-    QVDG_CUDA(cudaStreamSynchronize(s.stream));
+    copy_to_host(s, out_host + first, d, count * sizeof(double));
   }
 }
 
@@ -750,12 +749,10 @@ size_t sample_device_t(StateImpl& s, size_t shots, const double* uniforms_host, 
   uint64_t* tables = reinterpret_cast<uint64_t*>(w + o_tables);
   const cplx_t<T>* psi = static_cast<const cplx_t<T>*>(s.amp);
 
-  QVDG_CUDA(cudaMemcpyAsync(uni, uniforms_host, shots * 8, cudaMemcpyHostToDevice, s.stream));
-  static bool configured = false;  // per instantiation
-  if (!configured) {
+  static OncePerDevice once;  // per instantiation
+  once(s.device, [] {
     QVDG_CUDA(cudaFuncSetAttribute(k_fold<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, fold_smem<T>()));
-    configured = true;
-  }
+  });
   auto fold = [&](uint64_t items, const uint32_t* which, double* to, int at_checkpoints) {
     k_fold<T><<<unsigned((items + kFoldChunks - 1) / kFoldChunks), 32 * kFoldWarps, fold_smem<T>(), s.stream>>>(
         psi, len, chunk_len, items, which, prefix, to, at_checkpoints);
@@ -764,6 +761,8 @@ size_t sample_device_t(StateImpl& s, size_t shots, const double* uniforms_host, 
   fold(nchunks, nullptr, sums, 0);
   k_prefix<<<1, 256, 0, s.stream>>>(sums, nchunks, prefix);
   QVDG_LAUNCH_CHECK();
+  // Staged while the chunks are summed.
+  copy_to_device(s, uni, uniforms_host, shots * 8);
   k_target_keys<<<blocks_for(shots, kThreads), kThreads, 0, s.stream>>>(uni, shots, prefix + nchunks, keys);
   QVDG_LAUNCH_CHECK();
   DeviceScratch& sort_work = s.work2;
@@ -810,8 +809,7 @@ size_t sample_t(StateImpl& s, size_t shots, const double* uniforms_host, uint64_
   if (shots == 0) return 0;
   uint64_t *out = nullptr, *keys = nullptr, *tmp = nullptr;
   const size_t found = sample_device_t<T>(s, shots, uniforms_host, &out, &keys, &tmp);
-  if (found > 0) QVDG_CUDA(cudaMemcpyAsync(out_host, out, found * 8, cudaMemcpyDeviceToHost, s.stream));
-  QVDG_CUDA(cudaStreamSynchronize(s.stream));
+  if (found > 0) copy_to_host(s, out_host, out, found * 8);
   return found;
 }
 

@@ -399,3 +399,38 @@ def test_states_reuse_what_earlier_ones_left(threads):
     with ThreadPoolExecutor(threads) as pool:
         assert all(pool.map(work, range(threads)))
     assert before - free_bytes() <= 4 * (16 + 16 + 16 + 2) << 20
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("n", [16, 17, 18, 20, 23])
+def test_large_copies_through_staging_chunks(n, pinned):
+    """Amplitudes and probabilities in and out below, at and over the sizes
+    where copies go through two pinned chunks, from ordinary and from pinned
+    arrays, also right after one another."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    if pinned:
+        psi = torch.from_numpy(psi).pin_memory().numpy()
+    with DeviceState(n, 64) as st:
+        for _ in range(2):
+            st.set_amplitudes(psi)
+            assert np.array_equal(st.amplitudes(), psi)
+            psi[:] = psi[::-1].copy()
+        st.set_amplitudes(psi)
+        p = st.probabilities()
+        assert np.allclose(p, np.abs(psi) ** 2, rtol=1e-14, atol=0)
+
+
+@pytest.mark.parametrize("shots", [131071, 131072, 131073, 262145, 1000003])
+def test_outcomes_through_staging_chunks(oracle, shots):
+    """Uniforms in and outcomes out over the same sizes: each outcome is the
+    reference sampler's."""
+    rng = np.random.default_rng(shots)
+    psi = rng.standard_normal(1 << 10) + 1j * rng.standard_normal(1 << 10)
+    u = rng.random(shots)
+    with DeviceState(10, 64) as st:
+        st.set_amplitudes(psi / np.linalg.norm(psi))
+        got = st.sample_unordered(u)
+        assert np.array_equal(got, oracle.sample_from_amplitudes(st.amplitudes(), u, 64))
