@@ -283,7 +283,7 @@ constexpr int kFoldChunks = 16;
 constexpr int kFoldWarps = 5;    // the chains' and four that convert
 constexpr int kFoldStages = 4;
 constexpr int kFoldWindow = 512;  // bytes per chunk per window
-constexpr int kCheckpoint = 256;  // amplitudes
+constexpr int kCheckpoint = 64;  // amplitudes
 
 template <typename T>
 constexpr int fold_smem() {
