@@ -29,6 +29,9 @@ struct qvdg_mlp {
   // Activations and gradients for `cap` rows.
   size_t cap = 0;
   float* buf = nullptr;
+  // Pinned rows and results of short forward passes.
+  float* host = nullptr;
+  size_t host_floats = 0;
   cudaStream_t stream = nullptr;
 };
 
@@ -249,6 +252,52 @@ float backward(qvdg_mlp* m, const Acts& a, int rows) {
   return float(s / rows);
 }
 
+// The whole network over a few rows in one launch, rows read from and results
+// written to mapped host memory: the planner ranks some hundred passes per
+// plan, where three launches and two copies took most of the time. A block
+// takes kRowsPer rows, a thread one unit of a layer, with the same chains of
+// additions as k_dense_fwd (k ascending, then the bias), so the same results.
+constexpr int kRowsPer = 8;
+constexpr uint32_t kShortIn = 64, kShortHid = 256;
+constexpr size_t kShortRows = 8192;
+
+__global__ void __launch_bounds__(int(kShortHid)) k_forward_short(const float* __restrict__ x, int rows, int in, int hid,
+                                                                 const Views p, float* __restrict__ y) {
+  __shared__ __align__(16) float xs[kRowsPer][kShortIn], a1[kRowsPer][kShortHid], a2[kRowsPer][kShortHid];
+  const int r0 = blockIdx.x * kRowsPer, n = min(kRowsPer, rows - r0);
+  for (int i = threadIdx.x; i < kRowsPer * in; i += blockDim.x)
+    xs[i / in][i % in] = i / in < n ? x[size_t(r0) * in + i] : 0.f;
+  __syncthreads();
+  auto layer = [&](const float* W, const float* b, int width, const float* src, int pitch, float (*dst)[kShortHid]) {
+    for (int o = threadIdx.x; o < hid; o += blockDim.x) {
+      float acc[kRowsPer];
+#pragma unroll
+      for (int r = 0; r < kRowsPer; ++r) acc[r] = 0.f;
+      for (int k = 0; k < width; k += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(W + size_t(o) * width + k);
+#pragma unroll
+        for (int r = 0; r < kRowsPer; ++r) {
+          const float4 v = *reinterpret_cast<const float4*>(src + r * pitch + k);
+          acc[r] = fmaf(v.x, w.x, acc[r]);
+          acc[r] = fmaf(v.y, w.y, acc[r]);
+          acc[r] = fmaf(v.z, w.z, acc[r]);
+          acc[r] = fmaf(v.w, w.w, acc[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kRowsPer; ++r) dst[r][o] = fmaxf(acc[r] + b[o], 0.f);
+    }
+    __syncthreads();
+  };
+  layer(p.W1, p.b1, in, &xs[0][0], int(kShortIn), a1);
+  layer(p.W2, p.b2, hid, &a1[0][0], int(kShortHid), a2);
+  if (int(threadIdx.x) < n) {
+    float acc = 0.f;
+    for (int k = 0; k < hid; ++k) acc = fmaf(a2[threadIdx.x][k], p.W3[k], acc);
+    y[r0 + threadIdx.x] = acc + p.b3[0];
+  }
+}
+
 void upload(qvdg_mlp* m, const Acts& a, const float* x, const float* t, size_t rows) {
   QVDG_CUDA(cudaMemcpyAsync(a.X, x, rows * m->in * sizeof(float), cudaMemcpyHostToDevice, m->stream));
   if (t) QVDG_CUDA(cudaMemcpyAsync(a.t, t, rows * sizeof(float), cudaMemcpyHostToDevice, m->stream));
@@ -294,6 +343,7 @@ void mlp_destroy(qvdg_mlp* m) {
   if (!m) return;
   cudaSetDevice(m->device);
   if (m->stream) cudaStreamSynchronize(m->stream);
+  if (m->host) cudaFreeHost(m->host);
   if (m->buf) cudaFree(m->buf);
   if (m->params) cudaFree(m->params);
   if (m->stream) cudaStreamDestroy(m->stream);
@@ -314,6 +364,25 @@ void mlp_set_params(qvdg_mlp* m, const float* in) {
 
 void mlp_forward(qvdg_mlp* m, const float* x, size_t rows, float* y) {
   QVDG_CUDA(cudaSetDevice(m->device));
+  if (rows <= kShortRows && m->in <= kShortIn && m->hid <= kShortHid && m->in % 4 == 0 && m->hid % 4 == 0) {
+    const size_t need = rows * (m->in + 1);
+    if (need > m->host_floats) {
+      if (m->host) cudaFreeHost(m->host);
+      m->host = nullptr;
+      m->host_floats = 0;
+      QVDG_CUDA(cudaMallocHost(&m->host, 2 * need * sizeof(float)));
+      m->host_floats = 2 * need;
+    }
+    std::copy(x, x + rows * m->in, m->host);
+    float* out = m->host + rows * m->in;
+    const unsigned threads = std::max<unsigned>(32, (m->hid + 31) / 32 * 32);
+    k_forward_short<<<unsigned((rows + kRowsPer - 1) / kRowsPer), threads, 0, m->stream>>>(
+        m->host, int(rows), int(m->in), int(m->hid), views(m->params, m->in, m->hid), out);
+    QVDG_LAUNCH_CHECK();
+    QVDG_CUDA(cudaStreamSynchronize(m->stream));
+    std::copy(out, out + rows, y);
+    return;
+  }
   ensure(m, rows);
   const Acts a = acts(m->buf, m->cap, m->in, m->hid);
   upload(m, a, x, nullptr, rows);
