@@ -89,8 +89,9 @@ typedef struct {
   /* QVDG_PLANNER_GREEDY: plan with the settings given here.
    * QVDG_PLANNER_LEARNED: build every candidate setting
    * (qvdg_planner_candidates) and run the one the registered cost model
-   * (qvdg_cost_model_set) predicts fastest; max_fused_qubits, staged,
-   * tile_qubits and math are then only the fallback, used for complex128
+   * (qvdg_cost_model_set) predicts fastest (on states of at most 10 qubits
+   * the staged fp32 one, a single launch, without ranking); max_fused_qubits,
+   * staged, tile_qubits and math are then only the fallback, used for complex128
    * states or when no model is registered for the current device. */
   uint32_t planner;
   /* QVDG_MATH_FP32: every gate on the CUDA cores. QVDG_MATH_TENSOR

@@ -14,6 +14,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <limits>
 #include <map>
@@ -52,6 +53,8 @@ qvdg_options make(uint32_t fused, uint32_t staged, uint32_t math) {
   o.planner = QVDG_PLANNER_GREEDY;
   return o;
 }
+
+constexpr uint32_t kOneTileQubits = 10;
 
 }  // namespace
 
@@ -131,6 +134,19 @@ Program choose_program(const Target& t, const std::vector<HOp>& ops, const qvdg_
     return build_program(t, ops, o, search, from_zero);
   }
   const std::vector<qvdg_options> cands = learned_candidates(t.bits);
+  // A state of one small tile: the register-staged plan is a single launch
+  // whatever the circuit, where the others launch once per fused gate, and
+  // ranking the candidates takes longer than any of them runs (one gate on 5
+  // qubits: 165 us ranked, 69 us staged).
+  size_t fixed = cands.size();
+  if (t.n <= kOneTileQubits)
+    fixed = size_t(std::find_if(cands.begin(), cands.end(),
+                                [](const qvdg_options& o) { return o.staged && o.math == QVDG_MATH_FP32; }) -
+                   cands.begin());
+  if (fixed < cands.size() && !predicted) {
+    if (chosen) *chosen = cands[fixed];
+    return build_program(t, ops, cands[fixed], search, from_zero);
+  }
   std::vector<Program> progs(cands.size());
   parallel_for(cands.size(), [&](size_t i) { progs[i] = build_program(t, ops, cands[i], search, from_zero); });
   std::vector<const Program*> ptrs;
@@ -139,6 +155,7 @@ Program choose_program(const Target& t, const std::vector<HOp>& ops, const qvdg_
   size_t best = 0;
   for (size_t i = 1; i < sec.size(); ++i)
     if (sec[i] < sec[best]) best = i;
+  if (fixed < cands.size()) best = fixed;
   if (chosen) *chosen = cands[best];
   if (predicted) *predicted = sec;
   return std::move(progs[best]);
