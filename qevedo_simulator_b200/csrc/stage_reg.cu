@@ -48,10 +48,14 @@ constexpr size_t kRegBlobBudget = 64 * 1024;
 enum : uint8_t { kRegDense1 = 0, kRegDense2 = 1, kRegSign = 2, kRegPhase = 3, kRegSign2 = 4 };
 enum : uint8_t { kFormGeneral = 0, kFormReal = 1, kFormImag = 2, kFormComplex = 3, kFormX = 4 };
 
-// Shared-memory position of tile element e: bits 1-3 XORed with bits 5-7,
-// 9-11 and 13-15 (bit 0 is kept, so element pairs 2v, 2v+1 stay one 16-byte
-// slot for cp.async). XOR-linear and an involution.
-__host__ __device__ __forceinline__ uint32_t reg_swz(uint32_t e) {
+// Shared-memory position of tile element e, XOR-linear. complex64: bits 1-3
+// XORed with bits 5-7, 9-11 and 13-15 (bit 0 is kept, so element pairs 2v,
+// 2v+1 stay one 16-byte slot for cp.async). complex128, whose elements are
+// 16 bytes and go eight lanes at a time: bits 0-2 XORed with every higher
+// three, so that any three neighbouring bits reach all eight places.
+template <typename T>
+__device__ __forceinline__ uint32_t reg_swz(uint32_t e) {
+  if (sizeof(T) == 8) return e ^ (((e >> 3) ^ (e >> 6) ^ (e >> 9)) & 7u);
   return e ^ (((e >> 4) ^ (e >> 8) ^ (e >> 12)) & 14u);
 }
 
@@ -245,7 +249,7 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
   const uint32_t nsub = 1u << (L - 4);
   uint32_t bit[4];  // byte distance (swizzled) of each register bit
 #pragma unroll
-  for (int i = 0; i < 4; ++i) bit[i] = reg_swz(1u << h.g[i]) * uint32_t(sizeof(C2));
+  for (int i = 0; i < 4; ++i) bit[i] = reg_swz<T>(1u << h.g[i]) * uint32_t(sizeof(C2));
   const uint32_t first = h.first_gate, last = first + h.num_gates;
   for (uint32_t s = threadIdx.x; s < nsub; s += blockDim.x) {
     uint32_t eb = s;
@@ -257,7 +261,7 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
     // Register j at the subcube's place XOR the places of j's bits (the
     // swizzle is XOR-linear).
     unsigned char* const bytes = reinterpret_cast<unsigned char*>(tile);
-    const uint32_t place = reg_swz(eb) * uint32_t(sizeof(C2));
+    const uint32_t place = reg_swz<T>(eb) * uint32_t(sizeof(C2));
     auto at = [&](int j) {
       uint32_t o = place;
 #pragma unroll
@@ -445,7 +449,7 @@ __global__ void __launch_bounds__(reg_threads<T>(), 2)
     const uint64_t base = insert_zeros(t, tile_bits, L);
     for (uint32_t u = tid; u < units; u += blockDim.x) {
       const uint32_t e = u * per16;
-      cp_async16(smem_u32(dst + reg_swz(e)), psi + phys(base, e));
+      cp_async16(smem_u32(dst + reg_swz<T>(e)), psi + phys(base, e));
     }
   };
 
@@ -471,7 +475,7 @@ __global__ void __launch_bounds__(reg_threads<T>(), 2)
     for (int p = 0; p < geo.num_gates; ++p) run_register_pass<T>(tile, hdrs[p], gates, blob, L, base);
     for (uint32_t u = tid; u < units; u += blockDim.x) {
       const uint32_t e = u * per16;
-      *reinterpret_cast<uint4*>(psi + phys(base, e)) = *reinterpret_cast<const uint4*>(tile + reg_swz(e));
+      *reinterpret_cast<uint4*>(psi + phys(base, e)) = *reinterpret_cast<const uint4*>(tile + reg_swz<T>(e));
     }
     __syncthreads();
     cur ^= other;
@@ -876,18 +880,19 @@ void launch_stage_reg(StateImpl& s, const LoweredPass& lp, const DeviceUpload& d
   const int cap = s.bits == 32 ? reg_threads<float>() : reg_threads<double>();
   const int threads = std::max(32, std::min(cap, 1 << (lp.geo.L - 4)));
   const uint64_t grid = std::min<uint64_t>(lp.geo.num_tiles, uint64_t(s.sms) * (buffers == 1 ? 2 : 1));
-  auto launch = [&](auto* psi, auto kernel, size_t& configured) {
-    if (smem > configured) {
-      QVDG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-      configured = smem;
-    }
+  auto launch = [&](auto* psi, auto kernel, OncePerDevice& once) {
+    once(s.device, [&] {
+      // Two tiles and the largest program, the most any pass takes.
+      QVDG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(2 * (size_t(8) << 13) + kRegBlobBudget)));
+    });
     kernel<<<unsigned(grid), threads, smem, s.stream>>>(psi, lp.geo, dev.tc, buffers);
   };
-  static size_t configured[2] = {0, 0};
+  static OncePerDevice once[2];
   if (s.bits == 32)
-    launch(static_cast<float2*>(s.amp), k_stage_reg<float>, configured[0]);
+    launch(static_cast<float2*>(s.amp), k_stage_reg<float>, once[0]);
   else
-    launch(static_cast<double2*>(s.amp), k_stage_reg<double>, configured[1]);
+    launch(static_cast<double2*>(s.amp), k_stage_reg<double>, once[1]);
   QVDG_LAUNCH_CHECK();
 }
 
