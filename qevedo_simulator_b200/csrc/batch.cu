@@ -85,14 +85,17 @@ __device__ __forceinline__ TileMap low_map(int bits, uint32_t tile) { return Til
 
 // A register group of a pass: G gates of one layer on local bits
 // lq..lq+G-1, which hold qubits q..q+G-1.
+// Gates whose rows are led by their off-diagonal entries (`flip`, a bit
+// each) are an X and then the diagonal form: the X is only where the subcube
+// is read from.
 struct Step {
   int32_t G, lq, q;
-  uint32_t layer;
+  uint32_t layer, flip;
 };
 
 struct Tables {
   Step step[kMaxSteps];
-  float2 gate[kMaxSteps][kGroup][4];          // per gate: (a, b), (off, -) or the 2x2 matrix
+  float2 gate[kMaxSteps][kGroup][4];          // per gate: (a, b), or the 2x2 matrix
   float2 left[kMaxSteps][2][1 << kGroup];     // factors after the rotations, by the outside control's value
   float2 right[kMaxSteps][1 << kGroup];       // factors before them
 };
@@ -180,20 +183,28 @@ __device__ __forceinline__ void apply_step(uint32_t tile, int nb, const Tables& 
     return o;
   };
   const uint32_t all = at(S - 1);
+  uint32_t flip = 0;
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+    if ((tab.step[si].flip >> g) & 1u) flip ^= place[g];
   for (uint32_t b = threadIdx.x; b < subcubes; b += blockDim.x) {
     const uint32_t e = ((b & ~low_mask) << G) | (b & low_mask);
     const uint32_t base = swz(e) * 8u;
     u64 a[S];
+    const uint32_t from = base ^ flip;
     if constexpr (kLow && G > 0) {
+      // (16-byte pairs: a flip of bit 0 swaps each one's halves.)
+      const uint32_t pair = from & ~8u;
+      const bool odd = (from & 8u) != 0;
 #pragma unroll
       for (int j = 0; j < S; j += 2) {
-        const ulonglong2 v = lds128(tile + (base ^ at(j)));
-        a[j] = v.x;
-        a[j + 1] = v.y;
+        const ulonglong2 v = lds128(tile + (pair ^ at(j)));
+        a[j] = odd ? v.y : v.x;
+        a[j + 1] = odd ? v.x : v.y;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < S; ++j) a[j] = lds64(tile + (base ^ at(j)));
+      for (int j = 0; j < S; ++j) a[j] = lds64(tile + (from ^ at(j)));
     }
     // The ladder's gate into the group's first qubit is controlled by a bit
     // outside it: constant for the subcube.
@@ -206,22 +217,12 @@ __device__ __forceinline__ void apply_step(uint32_t tile, int nb, const Tables& 
       for (int g = 0; g < G; ++g) {
         const float2 r = tab.gate[si][g][0];
         const u64 ra = pack(make_float2(r.x, r.x)), rb = pack(make_float2(r.y, r.y));
-        if (tab.gate[si][g][1].x == 0.f) {
 #pragma unroll
-          for (int j = 0; j < S; ++j) {
-            if (j & (1 << g)) continue;
-            const u64 x0 = a[j], x1 = a[j | (1 << g)];
-            a[j] = fma2(ra, x1, x0);
-            a[j | (1 << g)] = fma2(rb, x0, x1);
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < S; ++j) {
-            if (j & (1 << g)) continue;
-            const u64 x0 = a[j], x1 = a[j | (1 << g)];
-            a[j] = fma2(ra, x0, x1);
-            a[j | (1 << g)] = fma2(rb, x1, x0);
-          }
+        for (int j = 0; j < S; ++j) {
+          if (j & (1 << g)) continue;
+          const u64 x0 = a[j], x1 = a[j | (1 << g)];
+          a[j] = fma2(ra, x1, x0);
+          a[j | (1 << g)] = fma2(rb, x0, x1);
         }
       }
     } else {
@@ -293,7 +294,7 @@ __device__ void add_steps(Tables& tab, int& count, uint32_t layer, int q0, int q
   int q = q0;
   for (int g = 0; g < groups; ++g) {
     const int size = small + (g < extra ? 1 : 0);
-    tab.step[count++] = Step{size, lq0 + q - q0, q, layer};
+    tab.step[count++] = Step{size, lq0 + q - q0, q, layer, 0u};
     q += size;
   }
 }
@@ -308,20 +309,23 @@ __device__ void build_tables(Tables& tab, int count, const float2* __restrict__ 
     if (g >= s.G) continue;
     const float2* rec = gates + size_t(kBatchGateSlots) * (size_t(s.layer) * n + s.q + g);
     for (int k = 0; k < 4; ++k)
-      if (k < 2 || !(form & kBatchShear)) tab.gate[i / kGroup][g][k] = rec[k];
+      if (k < 1 || !(form & kBatchShear)) tab.gate[i / kGroup][g][k] = rec[k];
   }
   for (int i = threadIdx.x; i < count << kGroup; i += blockDim.x) {
     const int si = i >> kGroup, j = i & ((1 << kGroup) - 1);
     const Step s = tab.step[si];
     if (j >= (1 << s.G)) continue;
     float2 l = make_float2(1.f, 0.f), r = make_float2(1.f, 0.f);
+    uint32_t flip = 0;
     if (form & kBatchShear)
       for (int b = 0; b < s.G; ++b) {
         const float2* rec = gates + size_t(kBatchGateSlots) * (size_t(s.layer) * n + s.q + b);
-        const int bit = (j >> b) & 1;
+        const int bit = (j >> b) & 1, off = rec[1].x != 0.f ? 1 : 0;
+        flip |= uint32_t(off) << b;
         l = cmul(l, rec[2 + bit]);
-        r = cmul(r, rec[4 + bit]);
+        r = cmul(r, rec[4 + (bit ^ off)]);
       }
+    if (j == 0) tab.step[si].flip = flip;
     float2 l1 = l;
     if (entangler == QVDG_ENTANGLE_CZ_LADDER) {
       if (__popc(j & (j >> 1)) & 1) l = make_float2(-l.x, -l.y);
