@@ -25,6 +25,8 @@
 // bounds the kernel is the latency of each gate's chain (its record, then
 // its matrix, then the arithmetic), so warps count for more than a second
 // buffer: one CTA with two buffers left a complex128 stage 8 warps per SM.
+// (26-qubit complex128 grid circuit of depth 20, 14 stages: 43.7 ms then,
+// 23.7 now, of which sheared gates and sign flips are a fifth.)
 // Only a pass whose gate data leave no room for a second CTA keeps two
 // buffers, the next tile's copies in flight while the current is computed.
 
@@ -249,7 +251,8 @@ __device__ void run_register_pass(cplx_t<T>* tile, const RegPassHdr& h, const Re
   const uint32_t nsub = 1u << (L - 4);
   uint32_t bit[4];  // byte distance (swizzled) of each register bit
 #pragma unroll
-  for (int i = 0; i < 4; ++i) bit[i] = reg_swz<T>(1u << h.g[i]) * uint32_t(sizeof(C2));
+  for (int i = 0; i < 4; ++i)  // a reduction of equal lanes: in uniform registers (24.3 -> 23.7 ms)
+    bit[i] = __reduce_or_sync(0xffffffffu, reg_swz<T>(1u << h.g[i]) * uint32_t(sizeof(C2)));
   const uint32_t first = h.first_gate, last = first + h.num_gates;
   for (uint32_t s = threadIdx.x; s < nsub; s += blockDim.x) {
     uint32_t eb = s;
