@@ -434,3 +434,39 @@ def test_outcomes_through_staging_chunks(oracle, shots):
         st.set_amplitudes(psi / np.linalg.norm(psi))
         got = st.sample_unordered(u)
         assert np.array_equal(got, oracle.sample_from_amplitudes(st.amplitudes(), u, 64))
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [1, 2, 3, 9, 10, 11, 13, 16, 17, 21])
+def test_reductions_on_one_and_many_blocks(bits, n):
+    """Norm, P(1) of every bit alone and together, and Pauli strings with X/Y
+    inside and beyond a 16-byte vector, twice in a row, on states of less than
+    a block to every block of the grid, against numpy in 64 bits."""
+    rng = np.random.default_rng(n + bits)
+    psi = random_state(rng, n)
+    with DeviceState(n, bits) as st:
+        st.set_amplitudes(psi)
+        v = st.amplitudes()  # in the state's own precision
+        p = np.abs(v) ** 2
+        index = np.arange(1 << n)
+        p1 = np.array([p[(index >> q) & 1 == 1].sum() for q in range(n)])
+        labels = ["Z" * n, "X" * n, "Y" + "I" * (n - 1), "I" * (n - 1) + "Y", "I" * (n - 1) + "X"]
+        labels += ["".join(rng.choice(list("IXYZ"), n)) for _ in range(4)]
+        for _ in range(2):
+            assert abs(st.norm_sqr() - p.sum()) < 1e-13
+            assert np.allclose([st.probability_one(q) for q in range(n)], p1, rtol=0, atol=1e-13)
+            assert np.allclose(st.expect_z_all(), p.sum() - 2 * p1, rtol=0, atol=1e-13)
+            for label in labels:
+                w, phase = v.copy(), np.ones(1 << n, dtype=complex)
+                x = 0
+                for q, c in enumerate(reversed(label)):
+                    bit = (index >> q) & 1
+                    if c in "XY":
+                        x |= 1 << q
+                    if c == "Z":
+                        phase = phase * (1 - 2 * bit)
+                    if c == "Y":
+                        phase = phase * np.where(bit == 1, -1j, 1j)
+                w = np.empty_like(v)
+                w[index ^ x] = phase * v
+                assert abs(st.expect_pauli(label) - np.vdot(v, w).real) < 1e-13, label
