@@ -30,7 +30,7 @@ namespace qvdg {
 
 namespace {
 
-constexpr int kWideMaxItems = 16;  // elements a thread copies
+constexpr int kWideMaxItems = 32;  // elements a thread copies
 
 struct WideGeom {
   uint64_t tiles;
@@ -188,18 +188,20 @@ void launch(StateImpl& s, const PlainGate& pg, const void* mat) {
   for (size_t i = 0; i < fixed.size(); ++i) g.fixed[i] = uint8_t(fixed[i]);
   g.tiles = uint64_t(1) << (s.n - fixed.size());
   g.pairs = sizeof(T) == 4 && bits[0] == 0;
-  // The five element bits a warp's lanes step over: group bits take their
+  // The element bits that the lanes of one shared-memory access step over
+  // (128 bytes: 16 lanes of 8-byte elements, 8 of 16): group bits take their
   // own place, target bits are folded into the places left.
+  constexpr uint32_t kLaneBits = sizeof(T) == 4 ? 4 : 3;
   const size_t skip = g.pairs ? 1 : 0;
   uint32_t used = 0;
-  for (size_t i = skip; i < bits.size() && i < skip + 5; ++i) {
+  for (size_t i = skip; i < bits.size() && i < skip + kLaneBits; ++i) {
     const auto it = std::find(groups.begin(), groups.end(), bits[i]);
     if (it != groups.end()) used |= 1u << (it - groups.begin());
   }
-  for (size_t i = skip; i < bits.size() && i < skip + 5; ++i) {
+  for (size_t i = skip; i < bits.size() && i < skip + kLaneBits; ++i) {
     const auto it = std::find(pg.targets.begin(), pg.targets.end(), bits[i]);
     if (it == pg.targets.end()) continue;
-    for (uint32_t p = 0; p < 5 && (1 << p) < NG; ++p)
+    for (uint32_t p = 0; p < kLaneBits && (1 << p) < NG; ++p)
       if (!((used >> p) & 1)) {
         used |= 1u << p;
         g.fold[it - pg.targets.begin()] = uint8_t(1u << p);
@@ -239,32 +241,55 @@ void launch(StateImpl& s, const PlainGate& pg, const void* mat) {
 
 }  // namespace
 
-// Which gates take the tile product: all 6-qubit gates of complex128 (a group
-// per thread does not fit its registers: 26 qubits 2.76 ms, tiles 1.88), and
-// the others while one thread per group would leave SMs idle (fewer than two
-// blocks of groups per SM). On larger states the group kernel is faster (28
-// qubits complex64: 1.7-1.85 and 3.28 ms for 5 and 6 qubits, tiles 2.1 and
-// 3.6; 26 qubits complex128, 5 qubits: 0.88 ms, tiles 1.06-1.2).
+// Which gates take the tile product.
+//   - All 6-qubit gates of complex128: a group per thread does not fit its
+//     registers (26 qubits 2.76 ms; tiles with 4 x 2 a thread 1.92, 8 x 4
+//     1.67).
+//   - Gates on states where one thread per group would leave SMs idle (fewer
+//     than two blocks of groups per SM).
+//   - Gates that leave none of the lowest bits free: neighbouring threads'
+//     groups then lie 8 amplitudes or more apart (complex128: 4), and the
+//     group kernel's loads fetch a sector for each lane. 28 qubits complex64,
+//     targets 0, 1, 2 and others, group kernel and tiles: 5 qubits 2.64 and
+//     1.87 ms, 6 qubits 3.37-4.17 and 3.22; 26 qubits complex128, 5 qubits,
+//     targets 0, 1 and others 0.93 and 0.89, with 2 too 1.13 and 0.91.
+// For the other gates on larger states the group kernel is faster (28 qubits
+// complex64: 1.35-1.7 and 2.9-3.05 ms for 5 and 6 qubits, tiles 1.9-2.0 and
+// 3.25-3.4; 26 qubits complex128, 5 qubits: 0.86 ms, tiles 0.89).
 bool launch_dense_wide(StateImpl& s, const PlainGate& pg, const void* mat) {
   const size_t k = pg.targets.size();
   const int free_bits = int(s.n) - int(pg.controls.size());  // index bits of the selected amplitudes
   if ((k != 5 && k != 6) || free_bits < (s.bits == 32 ? 11 : 10)) return false;
   const bool few = (uint64_t(1) << (free_bits - int(k))) < uint64_t(s.sms) * 2 * 256;
+  uint64_t taken = 0;
+  for (uint32_t t : pg.targets) taken |= uint64_t(1) << t;
+  for (auto& c : pg.controls) taken |= uint64_t(1) << c.first;
+  const uint64_t lowest = s.bits == 32 ? 7 : 3;
+  const bool scattered = (taken & lowest) == lowest;
   if (s.bits == 32) {
-    if (!few) return false;
-    if (k == 6)
-      launch<float, 6, 32, 4, 2>(s, pg, mat);
-    else
-      launch<float, 5, 64, 4, 2>(s, pg, mat);
+    if (few) {
+      if (k == 6)
+        launch<float, 6, 32, 4, 2>(s, pg, mat);
+      else
+        launch<float, 5, 64, 4, 2>(s, pg, mat);
+    } else {
+      if (!scattered) return false;
+      if (k == 6)
+        launch<float, 6, 64, 16, 2>(s, pg, mat);
+      else
+        launch<float, 5, 128, 16, 2>(s, pg, mat);
+    }
   } else if (k == 6) {
     // Tiles of 2048 amplitudes once they give every SM two.
     if (free_bits >= 11 && (uint64_t(1) << (free_bits - 11)) >= uint64_t(s.sms) * 2)
-      launch<double, 6, 32, 4, 2>(s, pg, mat);
+      launch<double, 6, 32, 8, 4>(s, pg, mat);
     else
       launch<double, 6, 16, 4, 1>(s, pg, mat);
-  } else {
-    if (!few) return false;
+  } else if (few) {
     launch<double, 5, 32, 4, 1>(s, pg, mat);
+  } else {
+    if (!scattered) return false;
+    launch<double, 5, 128, 8, 4>(s, pg, mat);
   }
   return true;
 }

@@ -630,6 +630,24 @@ def test_wide_dense_gates_as_tile_products(oracle, bits, n):
             assert max_distance(st.amplitudes(), expected) < TOL[bits], (targets, controls)
 
 
+@pytest.mark.parametrize("bits, n", [(32, 22), (32, 23), (64, 22)])
+def test_wide_dense_gates_with_no_low_bit_free(oracle, bits, n):
+    """5- and 6-qubit gates whose targets and controls take the lowest bits,
+    on both sides of the sizes from which those go as tile products."""
+    rng = np.random.default_rng(n * bits)
+    psi = random_state(rng, n)
+    cases = []
+    for k in (5, 6):
+        cases += [(list(range(k))[::-1], []), ([2, n - 1, 0, 9, 1, 5][:k], []), (list(range(1, k + 1)), [(0, False)])]
+    with DeviceState(n, bits) as st:
+        for targets, controls in cases:
+            m = random_unitary(rng, len(targets))
+            st.set_amplitudes(psi)
+            st.apply(m, targets, controls)
+            expected = oracle.naive_statevector([Op(targets, controls, m)], n, initial=psi)
+            assert max_distance(st.amplitudes(), expected) < TOL[bits], (targets, controls)
+
+
 @pytest.mark.parametrize("bits", [32, 64])
 @pytest.mark.parametrize("n", [5, 9, 13, 14])
 def test_register_stage_gate_forms(oracle, bits, n):
