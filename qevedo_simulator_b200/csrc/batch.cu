@@ -42,6 +42,11 @@
 // addresses. Ladder order is preserved: groups run in ascending qubit order
 // and a ladder gate only touches the qubits of its own and the previous
 // group.
+//
+// Shared-memory and integer issue bound it (384 circuits of 10-22 qubits, 4-12
+// layers: ALU pipe 61 % busy, shared memory 49 %, FMA 14 %, HBM 9 %): one CTA
+// per wide circuit, a layer per two passes and four multiply-adds a rotation
+// took 112 ms, this 11.4.
 
 #include <cuda_runtime.h>
 

@@ -337,7 +337,8 @@ __global__ void __launch_bounds__(kThreads) k_diag(cplx_t<T>* __restrict__ psi, 
 // in the block's tile (constants) and from the tile's number (through byte
 // tables in shared memory), each part holding all eight gates' indices as
 // 16-bit fields of one 16-byte word. A thread moves 16-byte vectors, four
-// in flight.
+// in flight. 28-qubit QFT of a general state: 27 diagonal passes of 0.79 ms
+// become 9, three alone and six of 0.75-1.15 ms, 31.7 -> 16.5 ms in all.
 constexpr int kRunUnroll = 4;
 constexpr int kRunTileBits = 10;  // vectors of a block's tile: kThreads * kRunUnroll
 
@@ -447,7 +448,8 @@ __global__ void __launch_bounds__(kThreads) k_diag_run(cplx_t<T>* __restrict__ p
 // over low bits hit distinct banks both when they write rows (low bits
 // vary) and when they read mapped elements (row bits vary). All three maps
 // of e are linear in its bits, so a thread's elements are its first one's
-// plus constants.
+// plus constants. A random swap pass at 30 qubits: about 17 ms with one thread
+// per amplitude, 3.7 ms now (0.70 of the copy rate; 27 qubits 0.83).
 // Tiles of 16 KB: with 8 KB ones a complex64 pass ran at 0.51-0.54 of the
 // copy rate (complex128, 16 KB, at 0.76-0.83).
 // A complex64 state of 2^32 bytes or more whose rows scatter (four low bits
