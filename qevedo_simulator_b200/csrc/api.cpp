@@ -321,8 +321,8 @@ void apply_program(StateImpl& s, const std::vector<HOp>& ops, const qvdg_options
 }
 
 // One op as a single plain pass (StateVector::apply, src/state.rs:181-198),
-// without the planner: its matrix through the pinned staging buffer, one
-// launch, one synchronisation (planning, timing events and their reads took
+// without the planner: its matrix in the launch's parameters (larger ones
+// through the pinned staging buffer), one launch, one synchronisation (planning, timing events and their reads took
 // two thirds of a small state's 42 us). A state still |0...0> goes through
 // the planner, whose zero-start pass moves little of it.
 void apply_single(StateImpl& s, const HOp& op) {
@@ -340,8 +340,11 @@ void apply_single(StateImpl& s, const HOp& op) {
   pass.staged = false;
   pass.ops.push_back(op);
   const LoweredPass lp = lower_pass(prog.target, pass, prog.cfg, prog.upload);
-  const DeviceUpload dev = upload_program(s, prog, s.work);
-  launch_pass(s, lp, dev);
+  if (lp.block || lp.pair ||
+      !launch_plain_gate_inline(s, lp.plain, prog.upload.mats.data() + 2 * lp.plain.matrix_offset)) {
+    const DeviceUpload dev = upload_program(s, prog, s.work);
+    launch_pass(s, lp, dev);
+  }
   QVDG_CUDA(cudaStreamSynchronize(s.stream));
 }
 

@@ -96,6 +96,9 @@ struct StateImpl {
 // Launch one plain gate pass; `matrices` is the device copy of the upload
 // (complex in the state's precision).
 void launch_plain_gate(StateImpl& s, const PlainGate& g, const void* matrices);
+// The same with its matrix (row-major, or the diagonal; re, im pairs) in the
+// launch's parameters, if it is small enough for that; false if not.
+bool launch_plain_gate_inline(StateImpl& s, const PlainGate& g, const double* matrix);
 // Whether diagonal `g` fits beside the gates of `run`, and adding it.
 bool diag_run_fits(const DiagRun& run, const PlainGate& g, int bits);
 void diag_run_add(DiagRun& run, const PlainGate& g);

@@ -26,6 +26,30 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// A gate's matrix as a kernel gets it: on the device, or in the launch's own
+// parameters. A single gate on a small state is mostly latency (17 qubits
+// complex128: 30 us a call), and the copy ahead of the kernel took 2-3 us of
+// it: 40 gates of 1-6 qubits 1.22 -> 1.16 ms. At most 1 KB; a 4-qubit matrix
+// of complex128 would fill the 4 KB that every launch can carry.
+template <typename T>
+struct MatDevice {
+  const cplx_t<T>* p;
+  __device__ const cplx_t<T>& operator[](int i) const { return p[i]; }
+};
+template <typename T, int N>
+struct MatInline {
+  cplx_t<T> v[N];
+  __device__ const cplx_t<T>& operator[](int i) const { return v[i]; }
+};
+template <typename T, int N>
+MatInline<T, N> mat_inline(const double* host, int count) {
+  MatInline<T, N> m{};
+  for (int i = 0; i < count; ++i) m.v[i] = make_c<T>(T(host[2 * i]), T(host[2 * i + 1]));
+  return m;
+}
+constexpr int kInlineDense = 3;     // qubits of a dense gate that goes inline
+constexpr int kInlineDiagonal = 6;  // and of a diagonal one
+
 struct DenseGeom {
   uint64_t n_iter;         // number of groups
   uint64_t control_value;  // control bits that must be 1
@@ -47,9 +71,9 @@ constexpr int kDenseThreads = sizeof(T) == 4 && K >= 5 ? 128 : kThreads;
 template <typename T, int K>
 constexpr int kDenseRows = sizeof(T) == 4 ? (K == 4 ? 4 : 2) : 1;
 
-template <typename T, int K, int G, bool VEC>
+template <typename T, int K, int G, bool VEC, typename M>
 __global__ void __launch_bounds__(kDenseThreads<T, K>, sizeof(T) == 4 && K >= 5 ? 3 : 1)
-    k_dense(cplx_t<T>* __restrict__ psi, const DenseGeom g, const cplx_t<T>* __restrict__ mat) {
+    k_dense(cplx_t<T>* __restrict__ psi, const __grid_constant__ DenseGeom g, const __grid_constant__ M mat) {
   constexpr int D = 1 << K, ROWS = kDenseRows<T, K>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx_t<T>* sm = reinterpret_cast<cplx_t<T>*>(smem_raw);
@@ -138,9 +162,10 @@ struct LaneGeom {
   uint8_t targets[4];      // target positions (matrix bit order), all below 5
 };
 
-template <typename T, int K, int R>
-__global__ void __launch_bounds__(kThreads) k_dense_lanes(cplx_t<T>* __restrict__ psi, const LaneGeom g,
-                                                          const cplx_t<T>* __restrict__ mat) {
+template <typename T, int K, int R, typename M>
+__global__ void __launch_bounds__(kThreads) k_dense_lanes(cplx_t<T>* __restrict__ psi,
+                                                          const __grid_constant__ LaneGeom g,
+                                                          const __grid_constant__ M mat) {
   constexpr int D = 1 << K;
   __shared__ uint8_t fixed[40];
   if (threadIdx.x < 40) fixed[threadIdx.x] = g.fixed[threadIdx.x];
@@ -296,9 +321,9 @@ struct DiagGeom {
   int32_t k;
 };
 
-template <typename T, int G>
-__global__ void __launch_bounds__(kThreads) k_diag(cplx_t<T>* __restrict__ psi, const DiagGeom g,
-                                                   const cplx_t<T>* __restrict__ diag) {
+template <typename T, int G, typename M>
+__global__ void __launch_bounds__(kThreads) k_diag(cplx_t<T>* __restrict__ psi, const __grid_constant__ DiagGeom g,
+                                                   const __grid_constant__ M diag) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx_t<T>* sm = reinterpret_cast<cplx_t<T>*>(smem_raw);
   __shared__ uint8_t ctrl[40], tgt[16];
@@ -600,48 +625,66 @@ unsigned grid_for(const StateImpl& s, uint64_t work_items) {
 }
 
 template <typename T, int K, int G, bool VEC>
-void dense_launch(StateImpl& s, const DenseGeom& g, const void* mat) {
+void dense_launch(StateImpl& s, const DenseGeom& g, const void* mat, const double* host) {
   constexpr int threads = kDenseThreads<T, K>;
   const size_t smem = size_t(1) << (2 * K);
   const size_t bytes = smem * sizeof(cplx_t<T>);
-  static OncePerDevice once;  // per instantiation
-  once(s.device, [&] {
-    QVDG_CUDA(cudaFuncSetAttribute(k_dense<T, K, G, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-  });
   const uint64_t blocks = (g.n_iter / G + threads - 1) / threads;
   const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(blocks, uint64_t(s.sms) * 16)));
-  k_dense<T, K, G, VEC><<<grid, threads, bytes, s.stream>>>(static_cast<cplx_t<T>*>(s.amp), g,
-                                                            static_cast<const cplx_t<T>*>(mat));
+  auto* psi = static_cast<cplx_t<T>*>(s.amp);
+  if constexpr (K <= kInlineDense) {
+    if (host) {
+      using M = MatInline<T, 1 << (2 * K)>;
+      k_dense<T, K, G, VEC, M><<<grid, threads, bytes, s.stream>>>(psi, g, mat_inline<T, 1 << (2 * K)>(host, 1 << (2 * K)));
+      QVDG_LAUNCH_CHECK();
+      return;
+    }
+  }
+  using M = MatDevice<T>;
+  if constexpr (K == 6) {  // more than the default 48 KB
+    static OncePerDevice once;  // per instantiation
+    once(s.device, [&] {
+      QVDG_CUDA(
+          cudaFuncSetAttribute(k_dense<T, K, G, VEC, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+    });
+  }
+  k_dense<T, K, G, VEC, M><<<grid, threads, bytes, s.stream>>>(psi, g, M{static_cast<const cplx_t<T>*>(mat)});
   QVDG_LAUNCH_CHECK();
 }
 
 template <typename T, int K>
-void dense_pick(StateImpl& s, const DenseGeom& g, const void* mat, bool bit0_free) {
+void dense_pick(StateImpl& s, const DenseGeom& g, const void* mat, const double* host, bool bit0_free) {
   // Two groups per thread (two neighbours as one 16-byte load) as far as
   // their amplitudes fit the registers.
   if constexpr (K <= 4 || (K == 5 && sizeof(T) == 4)) {
     if (g.n_iter >= 2) {
       if constexpr (sizeof(T) == 4)
-        if (bit0_free) return dense_launch<T, K, 2, true>(s, g, mat);
-      return dense_launch<T, K, 2, false>(s, g, mat);
+        if (bit0_free) return dense_launch<T, K, 2, true>(s, g, mat, host);
+      return dense_launch<T, K, 2, false>(s, g, mat, host);
     }
   }
-  dense_launch<T, K, 1, false>(s, g, mat);
+  dense_launch<T, K, 1, false>(s, g, mat, host);
 }
 
 template <typename T, int K>
-void lanes_launch(StateImpl& s, const LaneGeom& g, const void* mat) {
+void lanes_launch(StateImpl& s, const LaneGeom& g, const void* mat, const double* host) {
   constexpr int R = 4;
   const uint64_t warps_needed = (g.rows + R - 1) / R;
   const unsigned grid = grid_for(s, warps_needed * 32);
-  k_dense_lanes<T, K, R><<<grid, kThreads, 0, s.stream>>>(static_cast<cplx_t<T>*>(s.amp), g,
-                                                          static_cast<const cplx_t<T>*>(mat));
+  auto* psi = static_cast<cplx_t<T>*>(s.amp);
+  constexpr int kEntries = 1 << (2 * K);
+  if (host)
+    k_dense_lanes<T, K, R, MatInline<T, kEntries>>
+        <<<grid, kThreads, 0, s.stream>>>(psi, g, mat_inline<T, kEntries>(host, kEntries));
+  else
+    k_dense_lanes<T, K, R, MatDevice<T>>
+        <<<grid, kThreads, 0, s.stream>>>(psi, g, MatDevice<T>{static_cast<const cplx_t<T>*>(mat)});
   QVDG_LAUNCH_CHECK();
 }
 
 template <typename T>
 void lanes_pick(StateImpl& s, const PlainGate& pg, uint64_t control_value, const std::vector<uint8_t>& ctrl,
-                const void* mat) {
+                const void* mat, const double* host) {
   LaneGeom g{};
   g.rows = uint64_t(1) << (s.n - 5 - ctrl.size());
   g.control_value = control_value;
@@ -649,14 +692,14 @@ void lanes_pick(StateImpl& s, const PlainGate& pg, uint64_t control_value, const
   for (size_t i = 0; i < ctrl.size(); ++i) g.fixed[i] = uint8_t(ctrl[i] - 5);
   for (size_t j = 0; j < pg.targets.size(); ++j) g.targets[j] = uint8_t(pg.targets[j]);
   switch (pg.targets.size()) {
-    case 1: return lanes_launch<T, 1>(s, g, mat);
-    case 2: return lanes_launch<T, 2>(s, g, mat);
-    default: return lanes_launch<T, 3>(s, g, mat);
+    case 1: return lanes_launch<T, 1>(s, g, mat, host);
+    case 2: return lanes_launch<T, 2>(s, g, mat, host);
+    default: return lanes_launch<T, 3>(s, g, mat, host);
   }
 }
 
 template <typename T>
-void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices) {
+void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices, const double* host) {
   const int k = int(pg.targets.size());
   const int c = int(pg.controls.size());
   uint64_t control_value = 0;
@@ -666,7 +709,7 @@ void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices) {
     if (cv.second) control_value |= uint64_t(1) << cv.first;
   }
   std::sort(ctrl.begin(), ctrl.end());
-  const cplx_t<T>* mat = static_cast<const cplx_t<T>*>(matrices) + pg.matrix_offset;
+  const cplx_t<T>* mat = matrices ? static_cast<const cplx_t<T>*>(matrices) + pg.matrix_offset : nullptr;
   if (pg.diagonal) {
     DiagGeom g{};
     g.n_iter = uint64_t(1) << (s.n - c);
@@ -677,10 +720,18 @@ void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices) {
     for (int j = 0; j < k; ++j) g.targets[j] = uint8_t(pg.targets[j]);
     const bool bit0_ctrl = c > 0 && ctrl[0] == 0;
     const size_t bytes = (size_t(1) << k) * sizeof(cplx_t<T>);
-    if (g.n_iter >= 2 && !bit0_ctrl)
-      k_diag<T, 2><<<grid_for(s, g.n_iter / 2), kThreads, bytes, s.stream>>>(static_cast<cplx_t<T>*>(s.amp), g, mat);
+    auto* psi = static_cast<cplx_t<T>*>(s.amp);
+    auto launch = [&](const auto& m) {
+      using M = std::decay_t<decltype(m)>;
+      if (g.n_iter >= 2 && !bit0_ctrl)
+        k_diag<T, 2, M><<<grid_for(s, g.n_iter / 2), kThreads, bytes, s.stream>>>(psi, g, m);
+      else
+        k_diag<T, 1, M><<<grid_for(s, g.n_iter), kThreads, bytes, s.stream>>>(psi, g, m);
+    };
+    if (host)
+      launch(mat_inline<T, 1 << kInlineDiagonal>(host, 1 << k));
     else
-      k_diag<T, 1><<<grid_for(s, g.n_iter), kThreads, bytes, s.stream>>>(static_cast<cplx_t<T>*>(s.amp), g, mat);
+      launch(MatDevice<T>{mat});
     QVDG_LAUNCH_CHECK();
     return;
   }
@@ -703,15 +754,15 @@ void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices) {
     bool lanes = k <= 3 && s.n >= 5;
     for (uint32_t t : pg.targets) lanes = lanes && t < 5;
     for (uint8_t cq : ctrl) lanes = lanes && cq >= 5;
-    if (lanes) return lanes_pick<T>(s, pg, control_value, ctrl, mat);
+    if (lanes) return lanes_pick<T>(s, pg, control_value, ctrl, mat, host);
   }
-  // complex64, no controls, targets (nearly) all among bits 0-3 -- each
-  // group one short contiguous run -- and a state of at least one tile:
+  // complex64, 4 qubits, no controls, targets (nearly) all among bits 0-3 --
+  // each group one short contiguous run -- and a state of at least one tile:
   // stage tiles through shared memory (coalesced) instead. With fewer low
   // targets the direct kernel's accesses are coalesced enough and it is faster.
   int low_targets = 0;
   for (uint32_t t : pg.targets) low_targets += t < 4 ? 1 : 0;
-  if (sizeof(T) == 4 && c == 0 && k >= 2 && k <= 4 && low_targets >= std::min(k, 3) &&
+  if (sizeof(T) == 4 && c == 0 && k == 4 && low_targets >= 3 &&
       s.n >= uint32_t(kTileBits) + 1) {
     DenseTileGeom tg{};
     int lb = kTileBits, nhigh = 0;
@@ -748,21 +799,11 @@ void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices) {
       const unsigned grid = unsigned(std::min<uint64_t>(tg.tiles, uint64_t(s.sms) * 3));
       auto* psi = static_cast<float2*>(s.amp);
       auto* m = reinterpret_cast<const float2*>(mat);
-      static bool configured[5] = {false, false, false, false, false};
-      if (!configured[k]) {
-        const void* fn = k == 2 ? reinterpret_cast<const void*>(k_dense_tile<2>)
-                                : (k == 3 ? reinterpret_cast<const void*>(k_dense_tile<3>)
-                                          : reinterpret_cast<const void*>(k_dense_tile<4>));
-        QVDG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-        configured[k] = true;
-      }
-      switch (k) {
-        case 2:
-          k_dense_tile<2><<<grid, kThreads, bytes, s.stream>>>(psi, tg, m);
-          break;
-        case 3: k_dense_tile<3><<<grid, kThreads, bytes, s.stream>>>(psi, tg, m); break;
-        default: k_dense_tile<4><<<grid, kThreads, bytes, s.stream>>>(psi, tg, m); break;
-      }
+      static OncePerDevice once;
+      once(s.device, [&] {
+        QVDG_CUDA(cudaFuncSetAttribute(k_dense_tile<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+      });
+      k_dense_tile<4><<<grid, kThreads, bytes, s.stream>>>(psi, tg, m);
       QVDG_LAUNCH_CHECK();
       return;
     }
@@ -771,12 +812,12 @@ void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices) {
   // selected for one.
   if (launch_dense_wide(s, pg, mat)) return;
   switch (k) {
-    case 1: return dense_pick<T, 1>(s, g, mat, bit0_free);
-    case 2: return dense_pick<T, 2>(s, g, mat, bit0_free);
-    case 3: return dense_pick<T, 3>(s, g, mat, bit0_free);
-    case 4: return dense_pick<T, 4>(s, g, mat, bit0_free);
-    case 5: return dense_pick<T, 5>(s, g, mat, bit0_free);
-    case 6: return dense_pick<T, 6>(s, g, mat, bit0_free);
+    case 1: return dense_pick<T, 1>(s, g, mat, host, bit0_free);
+    case 2: return dense_pick<T, 2>(s, g, mat, host, bit0_free);
+    case 3: return dense_pick<T, 3>(s, g, mat, host, bit0_free);
+    case 4: return dense_pick<T, 4>(s, g, mat, host, bit0_free);
+    case 5: return dense_pick<T, 5>(s, g, mat, host, bit0_free);
+    case 6: return dense_pick<T, 6>(s, g, mat, host, bit0_free);
     default: throw Error(4, "dense gates on more than 6 qubits are not supported");
   }
 }
@@ -810,9 +851,18 @@ int layout_tables(StateImpl& s, uint64_t** dev_tables) {
 
 void launch_plain_gate(StateImpl& s, const PlainGate& g, const void* matrices) {
   if (s.bits == 32)
-    plain_gate<float>(s, g, matrices);
+    plain_gate<float>(s, g, matrices, nullptr);
   else
-    plain_gate<double>(s, g, matrices);
+    plain_gate<double>(s, g, matrices, nullptr);
+}
+
+bool launch_plain_gate_inline(StateImpl& s, const PlainGate& g, const double* matrix) {
+  if (g.tensor || g.targets.size() > size_t(g.diagonal ? kInlineDiagonal : kInlineDense)) return false;
+  if (s.bits == 32)
+    plain_gate<float>(s, g, nullptr, matrix);
+  else
+    plain_gate<double>(s, g, nullptr, matrix);
+  return true;
 }
 
 bool diag_run_fits(const DiagRun& run, const PlainGate& g, int bits) {

@@ -649,6 +649,31 @@ def test_wide_dense_gates_with_no_low_bit_free(oracle, bits, n):
 
 
 @pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [4, 7, 14])
+def test_single_gates_inline_and_uploaded(oracle, bits, n):
+    """apply() of dense gates on 1-4 qubits and diagonals on 1-7, the largest
+    whose matrices travel with the launch and the smallest that do not: low,
+    high and unordered targets, with and without controls."""
+    rng = np.random.default_rng(n * bits)
+    psi = random_state(rng, n)
+    cases = []
+    for k in range(1, min(7, n) + 1):
+        d = np.exp(1j * rng.uniform(0, 2 * np.pi, 1 << k))
+        for m in [np.diag(d)] + ([random_unitary(rng, k)] if k <= 4 else []):
+            cases += [(list(range(k)), [], m), (list(range(n - k, n))[::-1], [], m)]
+            for c in (1, 2):
+                if k + c <= n:
+                    qs = random_qubits(rng, n, k + c)
+                    cases.append((qs[:k], [(q, bool(rng.integers(0, 2))) for q in qs[k:]], m))
+    with DeviceState(n, bits) as st:
+        for targets, controls, m in cases:
+            st.set_amplitudes(psi)
+            st.apply(m, targets, controls)
+            expected = oracle.naive_statevector([Op(targets, controls, m)], n, initial=psi)
+            assert max_distance(st.amplitudes(), expected) < TOL[bits], (targets, controls)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
 @pytest.mark.parametrize("n", [5, 9, 13, 14])
 def test_register_stage_gate_forms(oracle, bits, n):
     """Every form a register stage gives a 1-qubit gate, on every register
