@@ -470,3 +470,23 @@ def test_reductions_on_one_and_many_blocks(bits, n):
                 w = np.empty_like(v)
                 w[index ^ x] = phase * v
                 assert abs(st.expect_pauli(label) - np.vdot(v, w).real) < 1e-13, label
+
+
+@pytest.mark.parametrize("shots", [1, 2, 31, 64, 1000, 4095, 4096, 4097, 8192, 8193, 20481, 300001])
+def test_sorted_shots_of_every_block_size(oracle, shots):
+    """Targets sorted by one block and by tiles, at the edges of both and with
+    a last tile of one key: spread, in few values, all equal and descending.
+    Outcomes against the reference sampler's, counts against numpy's."""
+    rng = np.random.default_rng(shots)
+    n = 9
+    psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    with DeviceState(n, 64) as st:
+        st.set_amplitudes(psi / np.linalg.norm(psi))
+        v = st.amplitudes()
+        for u in (rng.random(shots), np.floor(rng.random(shots) * 7) / 7, np.full(shots, 0.625),
+                  np.linspace(0, 1, shots, endpoint=False)[::-1].copy()):
+            want = oracle.sample_from_amplitudes(v, u, 64)
+            assert np.array_equal(st.sample_unordered(u), want)
+            keys, counts = st.sample_counts(u, [(q, q) for q in range(n)])
+            k, c = np.unique(want, return_counts=True)
+            assert dict(zip(keys.tolist(), counts.tolist())) == dict(zip(k.tolist(), c.tolist()))
