@@ -449,23 +449,43 @@ __global__ void __launch_bounds__(32 * kFoldWarps) k_fold(const cplx_t<T>* __res
 }
 
 // prefix[0] = 0, prefix[c + 1] = prefix[c] + sums[c], sequentially
-// (src/measure.rs:119-124).
+// (src/measure.rs:119-124). A chain of dependent additions (8.4 cycles each)
+// in one thread: it works on registers, 16 sums read ahead of their additions,
+// and the block copies in and out. 8192 chunks: 70 us with a global store per
+// addition, 47 now (a thousand shots of 30 qubits: 2.07 -> 1.97 ms).
 __global__ void __launch_bounds__(256) k_prefix(const double* __restrict__ sums, uint64_t nchunks,
                                                 double* __restrict__ prefix) {
-  constexpr int kTile = 2048;
-  __shared__ double tile[kTile];
+  constexpr int kTile = 2048, kAhead = 16;
+  __shared__ __align__(16) double tile[kTile];
   double p = 0.0;
   if (threadIdx.x == 0) prefix[0] = 0.0;
   for (uint64_t t0 = 0; t0 < nchunks; t0 += kTile) {
     const int n = int(umin64(kTile, nchunks - t0));
+    for (int i = threadIdx.x; i < kTile; i += blockDim.x) tile[i] = i < n ? sums[t0 + i] : 0.0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) tile[i] = sums[t0 + i];
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int i = 0; i < n; ++i) {
-        p = __dadd_rn(p, tile[i]);
-        prefix[t0 + i + 1] = p;
+    if (threadIdx.x == 0) {
+      double2* v = reinterpret_cast<double2*>(tile);
+      double2 next[kAhead / 2];
+#pragma unroll
+      for (int e = 0; e < kAhead / 2; ++e) next[e] = v[e];
+      for (int i = 0; i < n; i += kAhead) {
+        double2 x[kAhead / 2];
+#pragma unroll
+        for (int e = 0; e < kAhead / 2; ++e) x[e] = next[e];
+        const int j = (i + kAhead < kTile ? i + kAhead : 0) / 2;
+#pragma unroll
+        for (int e = 0; e < kAhead / 2; ++e) next[e] = v[j + e];
+#pragma unroll
+        for (int e = 0; e < kAhead / 2; ++e) {
+          x[e].x = p = __dadd_rn(p, x[e].x);
+          x[e].y = p = __dadd_rn(p, x[e].y);
+          v[i / 2 + e] = x[e];
+        }
       }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) prefix[t0 + i + 1] = tile[i];
+    __syncthreads();
   }
 }
 
