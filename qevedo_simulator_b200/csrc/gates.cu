@@ -624,13 +624,28 @@ unsigned grid_for(const StateImpl& s, uint64_t work_items) {
   return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(blocks, uint64_t(s.sms) * 16)));
 }
 
+// The grid of a gate pass. A state that gives every SM 128 blocks is covered
+// by `many` of them per SM, started in order, so that the SMs read and write
+// neighbouring memory; 16 per SM stride over all of it. Each block sets its
+// tables up, which smaller states and wider gates do not make up for. 16 per
+// SM and many: 28 qubits complex64, gates on 1, 2, 3 qubits 0.700, 0.700, 0.685
+// and 0.668, 0.658, 0.650 ms; 26 qubits complex128 0.371, 0.360, 0.354 and
+// 0.340, 0.338, 0.339, a 2-qubit diagonal 0.394 and 0.347; low targets (64 per
+// SM) 0.695, 0.727 and 0.671, 0.683, 0.361, 0.365 and 0.343, 0.357. 4-qubit
+// gates and 3-qubit ones on low targets are slower so, and 22 qubits too (a
+// diagonal 0.032 and 0.035 ms).
+unsigned gate_grid(const StateImpl& s, uint64_t blocks, int many) {
+  const uint64_t per_sm = blocks >= uint64_t(s.sms) * 128 ? uint64_t(many) : 16;
+  return unsigned(std::max<uint64_t>(1, std::min(blocks, uint64_t(s.sms) * per_sm)));
+}
+
 template <typename T, int K, int G, bool VEC>
 void dense_launch(StateImpl& s, const DenseGeom& g, const void* mat, const double* host) {
   constexpr int threads = kDenseThreads<T, K>;
   const size_t smem = size_t(1) << (2 * K);
   const size_t bytes = smem * sizeof(cplx_t<T>);
   const uint64_t blocks = (g.n_iter / G + threads - 1) / threads;
-  const unsigned grid = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(blocks, uint64_t(s.sms) * 16)));
+  const unsigned grid = gate_grid(s, blocks, K <= 3 ? 128 : 16);
   auto* psi = static_cast<cplx_t<T>*>(s.amp);
   if constexpr (K <= kInlineDense) {
     if (host) {
@@ -669,8 +684,8 @@ void dense_pick(StateImpl& s, const DenseGeom& g, const void* mat, const double*
 template <typename T, int K>
 void lanes_launch(StateImpl& s, const LaneGeom& g, const void* mat, const double* host) {
   constexpr int R = 4;
-  const uint64_t warps_needed = (g.rows + R - 1) / R;
-  const unsigned grid = grid_for(s, warps_needed * 32);
+  const uint64_t blocks = ((g.rows + R - 1) / R * 32 + kThreads - 1) / kThreads;
+  const unsigned grid = gate_grid(s, blocks, K <= 2 ? 64 : 16);
   auto* psi = static_cast<cplx_t<T>*>(s.amp);
   constexpr int kEntries = 1 << (2 * K);
   if (host)
@@ -724,9 +739,9 @@ void plain_gate(StateImpl& s, const PlainGate& pg, const void* matrices, const d
     auto launch = [&](const auto& m) {
       using M = std::decay_t<decltype(m)>;
       if (g.n_iter >= 2 && !bit0_ctrl)
-        k_diag<T, 2, M><<<grid_for(s, g.n_iter / 2), kThreads, bytes, s.stream>>>(psi, g, m);
+        k_diag<T, 2, M><<<gate_grid(s, (g.n_iter / 2 + kThreads - 1) / kThreads, 128), kThreads, bytes, s.stream>>>(psi, g, m);
       else
-        k_diag<T, 1, M><<<grid_for(s, g.n_iter), kThreads, bytes, s.stream>>>(psi, g, m);
+        k_diag<T, 1, M><<<gate_grid(s, (g.n_iter + kThreads - 1) / kThreads, 128), kThreads, bytes, s.stream>>>(psi, g, m);
     };
     if (host)
       launch(mat_inline<T, 1 << kInlineDiagonal>(host, 1 << k));

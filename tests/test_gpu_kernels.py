@@ -730,3 +730,20 @@ def test_swap_passes_of_a_large_state():
     st.swap_physical(pairs)
     assert torch.equal(held, torch.arange(1 << n, device="cuda", dtype=torch.int32))
     st.close()
+
+
+def test_gates_on_grids_of_many_blocks(oracle):
+    """One gate of each plain kernel on a state that gives every SM more than
+    128 blocks, one after another."""
+    n = 25
+    rng = np.random.default_rng(n)
+    psi = random_state(rng, n)
+    d = lambda k: np.diag(np.exp(1j * rng.uniform(0, 2 * np.pi, 1 << k)))
+    ops = [Op([17], [], random_unitary(rng, 1)), Op([9], [(0, True)], random_unitary(rng, 1)),
+           Op([3], [], random_unitary(rng, 1)), Op([4, 1], [], random_unitary(rng, 2)), Op([20, 2], [], d(2)),
+           Op([11], [(0, False)], d(1))]
+    with DeviceState(n, 32) as st:
+        st.set_amplitudes(psi)
+        for op in ops:
+            st.apply(op.matrix, op.targets, op.controls)
+        assert max_distance(st.amplitudes(), oracle.naive_statevector(ops, n, initial=psi)) < TOL[32]
