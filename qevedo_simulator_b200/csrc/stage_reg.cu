@@ -16,8 +16,9 @@
 // the square roots of X, Y and W) is divided by them: x0 + a x1 and
 // x1 + b x0, two multiply-adds per amplitude for real or imaginary a and b,
 // four for complex ones, half of what the matrix takes. The stage's last
-// register pass multiplies by the product of the divisors, and their signs
-// join the sign flips. A +-1 diagonal (CZ and the like) only toggles sign
+// register pass multiplies by the product of the divisors, an earlier one where
+// that product would leave the numbers' range, and their signs join the sign
+// flips. A +-1 diagonal (CZ and the like) only toggles sign
 // bits, consecutive ones together; a (controlled) X moves registers.
 //
 // A tile's 16-byte cp.async copies and its stores back to HBM are covered by
@@ -46,6 +47,12 @@ namespace {
 
 constexpr int kRegThreads = 512;
 constexpr size_t kRegBlobBudget = 64 * 1024;
+// How far the product of the divisors left out may go from 1 (a power of two)
+// before the state is multiplied by it: until then the amplitudes are off by
+// its inverse, and 200 gates with a divisor of 1/2 would take complex64 ones
+// past 2^128. 2^40 leaves a state that is not normalised the rest of the range;
+// unitary gates (divisors from 1/sqrt 2) reach it once in 80 of them.
+constexpr int scale_limit(int bits) { return bits == 32 ? 40 : 200; }
 
 enum : uint8_t { kRegDense1 = 0, kRegDense2 = 1, kRegSign = 2, kRegPhase = 3, kRegSign2 = 4 };
 enum : uint8_t { kFormGeneral = 0, kFormReal = 1, kFormImag = 2, kFormComplex = 3, kFormX = 4 };
@@ -681,7 +688,15 @@ bool lower_register(const Target& s, const PlannedPass& p, const StageConfig& cf
     bool has_table;
   };
   std::vector<Fix> fixes;
-  std::complex<long double> scale = 1.0L;  // product of the sheared gates' divisors
+  std::complex<long double> scale = 1.0L;  // product of the sheared gates' divisors so far left out
+  auto put_scale = [&] {
+    RegGate f{};
+    f.op = kOpScale;
+    Fix fx{gates.size(), put_complex(data, {C{double(scale.real()), double(scale.imag())}}, s.bits), 0, false};
+    gates.push_back(f);
+    fixes.push_back(fx);
+    scale = 1.0L;
+  };
   for (size_t pi = 0; pi < passes.size(); ++pi) {
     const Pass& ps = passes[pi];
     RegPassHdr h{};
@@ -812,6 +827,7 @@ bool lower_register(const Target& s, const PlannedPass& p, const StageConfig& cf
         g.op = kOpPhase;
       gates.push_back(g);
       fixes.push_back(fx);
+      if (g.op < kOpX && std::abs(std::ilogb(std::abs(scale))) >= scale_limit(s.bits)) put_scale();
       if (sign_after) {
         // Divisors of opposite sign: -1 where the target is 1.
         RegGate z{};
@@ -827,13 +843,7 @@ bool lower_register(const Target& s, const PlannedPass& p, const StageConfig& cf
         fixes.push_back(zx);
       }
     }
-    if (pi + 1 == passes.size() && scale != std::complex<long double>(1.0L)) {
-      RegGate f{};
-      f.op = kOpScale;
-      Fix fx{gates.size(), put_complex(data, {C{double(scale.real()), double(scale.imag())}}, s.bits), 0, false};
-      gates.push_back(f);
-      fixes.push_back(fx);
-    }
+    if (pi + 1 == passes.size() && scale != std::complex<long double>(1.0L)) put_scale();
     h.num_gates = uint16_t(gates.size() - h.first_gate);
     std::memcpy(blob.data() + pi * sizeof(RegPassHdr), &h, sizeof(h));
   }

@@ -703,6 +703,39 @@ def test_register_stage_gate_forms(oracle, bits, n):
             assert max_distance(st.amplitudes(), expected) < {32: 1e-5, 64: 1e-11}[bits]
 
 
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [5, 9, 13])
+@pytest.mark.parametrize("kind", ["shrinking", "growing", "hadamard"])
+def test_register_stages_of_many_sheared_gates(oracle, bits, n, kind):
+    """Some 200 sheared gates in one stage: matrices whose divisors are all
+    1/2 (projections on |+>, the phases between near 1, so the state keeps
+    most of its norm), all nearly 2 (undone by the diagonals between), and H.
+    The state stays within its range whatever the divisors' product is."""
+    from qevedo_simulator_b200 import Gate
+
+    rng = np.random.default_rng(n + bits)
+    m = {"shrinking": np.full((2, 2), 0.5), "growing": np.array([[1.9, 0.05], [0.05, 1.9]]),
+         "hadamard": Gate("h").matrix()}[kind]
+    parts = [list(range(a, min(a + 5, n))) for a in range(0, n, 5)]
+    ops = []
+    for _ in range(255 // (n + len(parts))):
+        ops += [Op([q], [], m) for q in range(n)]
+        for qs in parts:
+            d = np.exp(1j * rng.uniform(-0.05, 0.05, 1 << len(qs)))
+            ops.append(Op(qs, [], np.diag(d / 1.9 ** len(qs) if kind == "growing" else d)))
+    psi = np.ones(1 << n) / 2 ** (n / 2) if kind == "shrinking" else random_state(rng, n)
+    expected = oracle.naive_statevector(ops, n, initial=psi)
+    norm = np.linalg.norm(expected)
+    assert 1e-6 < norm < 1e6
+    with DeviceState(n, bits) as st:
+        st.set_amplitudes(psi)
+        stats = st.apply_ops(ops, options(4, True))
+        if n <= (13 if bits == 32 else 12):  # one tile
+            assert stats["stages"] == 1
+        # Each of the gates rounds an amplitude by a few units in the last place.
+        assert max_distance(st.amplitudes(), expected) < {32: 4 * 255 * 2.0 ** -24, 64: 4 * 255 * 2.0 ** -53}[bits] * norm
+
+
 def test_swap_passes_of_a_large_state():
     """The large tiles of a 4 GiB state whose rows scatter: every amplitude at
     its place, and back again."""
