@@ -27,7 +27,7 @@ struct BatchWide {
   uint32_t tiles;           // of a pass
   uint32_t phases;          // tile passes: A and B in turn
   uint32_t layers;          // of an A and a B pass together
-  int32_t previous;         // the wide circuit that had the slot before (-1: none)
+  int32_t previous;         // the wide circuit with layers that had the slot before (-1: none)
   int32_t tile_bits, low, high;  // tile qubits; pass B's low qubits and first high one
   int32_t reserved;
   // Tiles of the circuit that are done before phase p begins (the first A

@@ -10,7 +10,7 @@
 #include <string>
 #include <vector>
 
-#include "batch.hpp"
+#include "batch_plan.hpp"
 #include "engine.hpp"
 
 struct qvdg_batch {
@@ -43,7 +43,6 @@ namespace {
 constexpr int kTileMin = 12, kTileMax = 14;
 constexpr int kMaxCtasPerSm = 4;
 constexpr size_t kSlotBudget = size_t(8) << 30;  // of wide circuits' states at a time
-constexpr uint32_t kMaxDepth = 5;                // layers of an A and B pass (their tables fit kMaxSteps groups)
 
 void require(bool ok, const std::string& message) {
   if (!ok) throw Error(QVDG_ERR_INVALID, message);
@@ -52,8 +51,9 @@ void require(bool ok, const std::string& message) {
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Whether a tile shape can run every circuit: wide circuits (n > L) run on
-// tiles of L - 1 qubits and need the pass-B tile (high n-L+1 qubits plus
-// r >= 1 low ones) to fit, n <= 2(L - 1) - 1.
+// tiles of min(L, 13) qubits (batch_plan.cpp), and pass B's needs two low
+// qubits or more below the high ones: n <= 2 L - 3 for L = 12 and 13, and every
+// n up to kBatchMaxQubits for L = 14.
 bool shape_fits(uint32_t max_qubits, int L) { return max_qubits <= uint32_t(L) || max_qubits <= uint32_t(2 * L - 3); }
 
 // Persistent CTAs for a shape: all resident CTAs (at most kMaxCtasPerSm per SM).
@@ -61,88 +61,12 @@ int ctas_for(const qvdg_batch* b, int threads, int L) {
   return b->sms * std::min(batch_kernel_occupancy(threads, L), kMaxCtasPerSm);
 }
 
-// The work of a set of circuits on tiles of L qubits, in the order CTAs take
-// it: waves of wide circuits, as many as there are slots, each wave pass by
-// pass; then the circuits that fit a tile.
-struct Work {
-  std::vector<BatchWide> wide;
-  std::vector<uint32_t> wide_of;  // per circuit
-  std::vector<BatchTask> tasks;
-  uint64_t partials = 0;          // doubles
-};
-
-constexpr uint64_t kPartialRow = 16;  // doubles per tile
-
-// Wide circuits run on tiles of 13 qubits (the largest tile leaves two of
-// them per CTA, so that copies fly under the computation), or the tile's own
-// 12. Pass B keeps 2^r contiguous amplitudes: 64 bytes, or a 32-byte sector
-// where that lets an A and B pass take a layer more.
-void wide_shape(uint32_t n, int L, BatchWide& w) {
-  w.tile_bits = std::min(L, 13);
-  w.low = 2 * w.tile_bits - 3 - int(n) >= 2 ? 3 : 2;
-  w.high = int(n) - (w.tile_bits - w.low);
-  w.layers = std::min<uint32_t>(uint32_t(w.tile_bits - w.high) + 1, kMaxDepth);
-  w.tiles = uint32_t(1) << (n - uint32_t(w.tile_bits));
-}
-
-size_t wide_count(const std::vector<BatchCircuit>& circuits, const std::vector<uint32_t>& order, int L) {
-  size_t k = 0;
-  for (uint32_t i : order) k += circuits[i].num_qubits > uint32_t(L);
-  return k;
-}
-
-Work plan_work(const std::vector<BatchCircuit>& circuits, const std::vector<uint32_t>& order, int L, int ctas,
-               size_t slots, uint64_t slot_elems) {
-  Work w;
-  w.wide_of.assign(circuits.size(), 0);
-  std::vector<uint32_t> wide;  // circuits, largest first as in `order`
-  uint64_t pass_tiles = 0;
-  for (uint32_t i : order)
-    if (circuits[i].num_qubits > uint32_t(L)) {
-      BatchWide x{};
-      const uint32_t k = uint32_t(wide.size());
-      wide_shape(circuits[i].num_qubits, L, x);
-      x.phases = 2 * ((circuits[i].num_layers + x.layers - 1) / x.layers);
-      x.slot = (k % slots) * slot_elems;
-      x.previous = k >= slots ? int32_t(k - slots) : -1;
-      x.partials = w.partials;
-      w.partials += uint64_t(x.tiles) * kPartialRow;
-      w.wide_of[i] = k;
-      w.wide.push_back(x);
-      wide.push_back(i);
-      if (k < slots) pass_tiles += x.tiles;
-    }
-  // Tiles of a task: several where that still leaves every CTA a few tasks
-  // of each pass (a task builds its gate tables once).
-  uint32_t grain = 1;
-  while (grain < 8 && pass_tiles >= uint64_t(grain) * 2 * 6 * uint64_t(ctas)) grain *= 2;
-  for (size_t first = 0; first < wide.size(); first += slots) {
-    const size_t end = std::min(wide.size(), first + slots);
-    uint32_t phases = 0;
-    for (size_t k = first; k < end; ++k) phases = std::max(phases, w.wide[k].phases);
-    for (uint32_t p = 0; p <= phases; ++p)
-      for (size_t k = first; k < end; ++k) {
-        const BatchWide& x = w.wide[k];
-        if (p > x.phases) continue;
-        if (p == x.phases || p == 0) {
-          w.tasks.push_back({wide[k], p, 0, 1});
-          continue;
-        }
-        const uint32_t g = std::min(grain, x.tiles);
-        for (uint32_t t = 0; t < x.tiles; t += g) w.tasks.push_back({wide[k], p, t, g});
-      }
-  }
-  for (uint32_t i : order)
-    if (circuits[i].num_qubits <= uint32_t(L)) w.tasks.push_back({i, 0, 0, 1});
-  return w;
-}
-
 // Plans the circuits of `order` on a shape and puts their work on the device
 // (an allocation of its own in *work, replacing what it held). The circuits'
 // `wide` fields follow.
 BatchLaunch shape(qvdg_batch* b, const BatchLaunch& base, const std::vector<uint32_t>& order, int L, int threads,
                   int ctas, size_t slots, uint64_t slot_elems, void** work) {
-  const Work w = plan_work(b->circuits, order, L, ctas, std::max<size_t>(slots, 1), slot_elems);
+  const BatchWork w = plan_batch(b->circuits, order, L, ctas, std::max<size_t>(slots, 1), slot_elems);
   require(w.tasks.size() < (size_t(1) << 31), "the batch has too many tiles");
   BatchLaunch l = base;
   l.tile_qubits = L;
@@ -294,7 +218,7 @@ qvdg_batch* batch_create(const qvdg_layered_circuit* circuits, size_t count, con
     size_t slots = 0, partials = 0;
     for (const Shape& s : shapes) {
       slots = std::max(slots, wide_count(b->circuits, order, s.L));
-      partials = std::max<size_t>(partials, plan_work(b->circuits, order, s.L, s.ctas, 1, slot_elems).partials);
+      partials = std::max<size_t>(partials, plan_batch(b->circuits, order, s.L, s.ctas, 1, slot_elems).partials);
     }
     if (slots) {
       slots = std::min<size_t>(slots, std::max<size_t>(1, kSlotBudget / (slot_elems * sizeof(float2))));

@@ -66,8 +66,8 @@ def test_small_batch_matches_the_naive_oracle(oracle):
 
 @pytest.mark.parametrize("tile,threads", [(12, 128), (13, 256), (14, 512)])
 def test_wide_circuits_match_the_per_circuit_path(tile, threads):
-    """Circuits wider than the tile run in HBM slots (two double-buffered
-    tile passes per layer on tiles of L - 1 qubits); compared with
+    """Circuits wider than the tile run in HBM slots (an A and a B pass of
+    tiles of 12 or 13 qubits for one to five layers); compared with
     complex128 runs of the same circuits through apply_ops on single
     states."""
     specs = [(15, 3, 1), (17, 4, 2), (18, 2, 3), (20, 3, 4), (min(22, 2 * tile - 3), 2, 5), (tile + 1, 3, 6),
@@ -86,6 +86,47 @@ def test_wide_circuits_match_the_per_circuit_path(tile, threads):
         flat, _ = b.run()
         for i, (got, exp) in enumerate(zip(b.split(flat), expected)):
             assert np.abs(got - exp).max() < Z_TOL, (i, specs[i], np.abs(got - exp).max())
+
+
+@pytest.mark.parametrize("tile", [12, 13, 14])
+@pytest.mark.parametrize("entangler", ["cx", "cz", "none"])
+def test_wide_circuits_of_many_layers(tile, entangler):
+    """More layers than an A and a B pass take together, whole rounds of them
+    and rounds with one to four left over, against complex128 runs."""
+    specs = [(tile + 1, 5, 1), (tile + 1, 11, 2), (15, 9, 3), (16, 8, 4), (18, 7, 5), (2 * tile - 4, 7, 6)]
+    circuits, expected = [], []
+    for w, layers, seed in specs:
+        g = library.hea_layers(w, layers, seed)
+        circuits.append((w, g, entangler))
+        with DeviceState(w, 64) as st:
+            st.apply_ops(layered_circuit(w, g, entangler).ops(), options(4, staged=False))
+            expected.append(st.expect_z_all())
+    with Batch(circuits, tile_qubits=tile, threads=256) as b:
+        flat, _ = b.run()
+        for i, (got, exp) in enumerate(zip(b.split(flat), expected)):
+            assert np.abs(got - exp).max() < Z_TOL, (i, specs[i], np.abs(got - exp).max())
+
+
+def test_more_wide_circuits_than_slots():
+    """The 64 slots of 24 qubits that a batch holds at most, taken over by 62
+    of 148 circuits, with circuits of no layers, whose results wait for
+    nobody, between: every copy of a circuit gives what it gives alone."""
+    kinds = [(24, 2, "cx", 6), (24, 1, "cz", 64), (24, 0, "cx", 16), (22, 2, "cx", 30), (22, 1, "none", 20),
+             (16, 0, "cz", 6), (15, 7, "cx", 6)]
+    circuits, alone = [], []
+    for k, (w, layers, ent, copies) in enumerate(kinds):
+        c = (w, library.hea_layers(w, layers, k), ent)
+        with Batch([c], tile_qubits=14, threads=256) as b:
+            alone += [b.run()[0]] * copies
+        circuits += [c] * copies
+        with DeviceState(w, 64) as st:
+            st.apply_ops(layered_circuit(*c).ops(), options(4, staged=False))
+            assert np.abs(alone[-1] - st.expect_z_all()).max() < Z_TOL, k
+    order = np.random.default_rng(1).permutation(len(circuits))
+    with Batch([circuits[i] for i in order], tile_qubits=14, threads=256) as b:
+        for _ in range(3):
+            for i, got in zip(order, b.split(b.run()[0])):
+                assert np.array_equal(got, alone[i]), i
 
 
 def test_autotuned_graph_replays_and_new_parameters():
