@@ -49,7 +49,8 @@ namespace {
 // Making and freeing them (above all the pinned memory, one to three
 // milliseconds) cost a statevector() of a few qubits ten times its gates.
 // At most kPoolStates of them wait, each within the limits below; a failing
-// allocation of this library gives them all back first. The pool itself is
+// allocation of this library gives them all back first. Amplitudes whose
+// address a caller has had are not among them. The pool itself is
 // never destroyed: the driver frees what is left at process exit.
 struct StateResources {
   int device = 0;
@@ -439,6 +440,18 @@ qvdg_status qvdg_state_destroy(qvdg_state* st) {
   StateImpl& s = st->s;
   const bool idle = s.stream && cudaStreamSynchronize(s.stream) == cudaSuccess;
   for (cudaEvent_t e : s.pass_events) cudaEventDestroy(e);
+  if (s.amp_given) {
+    // A caller's kernels may still use the amplitudes on streams of its own:
+    // they are waited for, and the buffer goes to no other state.
+    int current = s.device;
+    cudaGetDevice(&current);
+    if (current != s.device) cudaSetDevice(s.device);
+    cudaDeviceSynchronize();
+    if (current != s.device) cudaSetDevice(current);
+    cudaFree(s.amp);
+    s.amp = nullptr;
+    s.amp_capacity = 0;
+  }
   StateResources r;
   r.device = s.device;
   r.amp = s.amp;
@@ -641,6 +654,7 @@ qvdg_status qvdg_state_device_buffer(const qvdg_state* st, void** pointer, size_
   return guarded([&] {
     const StateImpl& s = impl(st);
     if (pointer) *pointer = s.amp;
+    if (pointer) s.amp_given = true;
     if (bytes) *bytes = s.amp_bytes;
     s.zero_state = false;  // the caller may write through the pointer
   });

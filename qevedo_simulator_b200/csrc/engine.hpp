@@ -62,6 +62,7 @@ struct StateImpl {
   void* amp = nullptr;  // 2^n interleaved complex in `bits` precision
   size_t amp_bytes = 0;
   size_t amp_capacity = 0;  // bytes allocated (a reused buffer may be larger)
+  mutable bool amp_given = false;  // its address was handed out: others may use it, on any stream
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   std::vector<uint32_t> layout;  // logical -> physical

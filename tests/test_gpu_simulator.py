@@ -490,3 +490,44 @@ def test_sorted_shots_of_every_block_size(oracle, shots):
             keys, counts = st.sample_counts(u, [(q, q) for q in range(n)])
             k, c = np.unique(want, return_counts=True)
             assert dict(zip(keys.tolist(), counts.tolist())) == dict(zip(k.tolist(), c.tolist()))
+
+
+def device_view(st):
+    """A state's amplitudes, in physical order, as a torch tensor on its own
+    device buffer."""
+    import torch
+
+    pointer, _ = st.device_buffer()
+
+    class Buffer:
+        __cuda_array_interface__ = {"shape": (1 << st.num_qubits,), "data": (pointer, False), "version": 3,
+                                    "typestr": "<c8" if st.precision_bits == 32 else "<c16"}
+
+    return torch.as_tensor(Buffer(), device="cuda")
+
+
+@pytest.mark.parametrize("n", [10, 20, 22])
+def test_closing_a_state_waits_for_its_buffer_s_readers(n):
+    """A read of the device buffer that is still queued on another stream when
+    its state is closed, and others are made and used at once, gives the closed
+    state's amplitudes: buffers of sizes that are kept for the next state and
+    of one that is not."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    psi = random_state(rng, n).astype(np.complex64)
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        st = DeviceState(n, 32)
+        st.set_amplitudes(psi)
+        view = device_view(st)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(50_000_000)  # some 30 ms
+            held = view.clone()
+        st.close()
+        with DeviceState(n, 32) as other, DeviceState(n, 32) as third:
+            for s in (other, third):
+                s.apply(Gate("h").matrix(), [0])
+                s.norm_sqr()
+        side.synchronize()
+        assert np.array_equal(held.cpu().numpy(), psi)
