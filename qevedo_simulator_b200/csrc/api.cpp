@@ -350,10 +350,10 @@ void apply_single(StateImpl& s, const HOp& op) {
 }
 
 // src/measure.rs:68-87. A state still |0...0> reads 0 with certainty and
-// stays as it is.
+// stays as it is, unless others may have written into it.
 int measure_qubit(StateImpl& s, uint32_t qubit, double uniform, bool reset) {
   require(qubit < s.n, "qubit out of range");
-  if (s.zero_state && !(uniform < 0.0)) return 0;
+  if (s.zero_state && !s.amp_given && !(uniform < 0.0)) return 0;
   s.zero_state = false;
   return measure(s, s.layout[qubit], uniform, reset);
 }

@@ -531,3 +531,25 @@ def test_closing_a_state_waits_for_its_buffer_s_readers(n):
                 s.norm_sqr()
         side.synchronize()
         assert np.array_equal(held.cpu().numpy(), psi)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+def test_measure_reads_what_was_written_through_the_device_buffer(bits):
+    """A pointer taken before zero() still writes into the state: measure and
+    reset answer from the amplitudes."""
+    import torch
+
+    n = 4
+    with DeviceState(n, bits) as st:
+        view = device_view(st)
+        for reset in (False, True):
+            st.zero()
+            view.zero_()
+            view[6] = 1
+            torch.cuda.synchronize()
+            if reset:
+                st.reset(1, 0.5)
+                st.reset(0, 0.5)
+            else:
+                assert [st.measure(q, 0.5) for q in range(n)] == [0, 1, 1, 0]
+            assert np.argmax(np.abs(st.amplitudes())) == (4 if reset else 6)
