@@ -426,8 +426,9 @@ qvdg_status qvdg_batch_info(const qvdg_batch* batch, qvdg_batch_summary* info);
 qvdg_status qvdg_batch_tuning(const qvdg_batch* batch, uint32_t* tile_qubits, uint32_t* threads, double* seconds,
                               size_t capacity, size_t* count);
 
-/* Record the device time of every pass of later gate runs on this state
- * (off by default; the reference's timing counters, src/simulator.rs:128-146).
+/* Record the device time of every pass of later gate runs on this state,
+ * qvdg_apply and the collapse of qvdg_measure and qvdg_reset among them (off
+ * by default; the reference's timing counters, src/simulator.rs:128-146).
  * While it is on, every pass is launched by itself; otherwise diagonal
  * passes that nothing between them holds back share one. */
 qvdg_status qvdg_set_pass_timing(qvdg_state* state, int32_t enabled);

@@ -325,9 +325,10 @@ void apply_program(StateImpl& s, const std::vector<HOp>& ops, const qvdg_options
 // without the planner: its matrix in the launch's parameters (larger ones
 // through the pinned staging buffer), one launch, one synchronisation (planning, timing events and their reads took
 // two thirds of a small state's 42 us). A state still |0...0> goes through
-// the planner, whose zero-start pass moves little of it.
+// the planner, whose zero-start pass moves little of it, and so does one whose
+// passes are timed.
 void apply_single(StateImpl& s, const HOp& op) {
-  if (s.zero_state) {
+  if (s.zero_state || s.record_passes) {
     qvdg_options opt;
     qvdg_default_options(&opt);
     opt.staged = 0;
@@ -353,6 +354,24 @@ void apply_single(StateImpl& s, const HOp& op) {
 // stays as it is, unless others may have written into it.
 int measure_qubit(StateImpl& s, uint32_t qubit, double uniform, bool reset) {
   require(qubit < s.n, "qubit out of range");
+  if (s.record_passes) {  // the collapse as a timed pass, a reset's flip as another
+    const double p1 = std::min(std::max(probability_one(s, s.layout[qubit]), 0.0), 1.0);
+    const bool one = uniform < p1;
+    const C keep{1.0 / std::sqrt(one ? p1 : 1.0 - p1), 0.0}, zero{0.0, 0.0};
+    HOp op;
+    op.targets = {qubit};
+    op.matrix = HMatrix::diagonal(one ? std::vector<C>{zero, keep} : std::vector<C>{keep, zero});
+    op.diagonal = true;
+    apply_single(s, op);
+    if (reset && one) {
+      HOp x;
+      x.targets = {qubit};
+      x.matrix = HMatrix(2);
+      x.matrix.at(0, 1) = x.matrix.at(1, 0) = {1.0, 0.0};
+      apply_single(s, x);
+    }
+    return one ? 1 : 0;
+  }
   if (s.zero_state && !s.amp_given && !(uniform < 0.0)) return 0;
   s.zero_state = false;
   return measure(s, s.layout[qubit], uniform, reset);

@@ -553,3 +553,30 @@ def test_measure_reads_what_was_written_through_the_device_buffer(bits):
             else:
                 assert [st.measure(q, 0.5) for q in range(n)] == [0, 1, 1, 0]
             assert np.argmax(np.abs(st.amplitudes())) == (4 if reset else 6)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+def test_single_gates_and_measurements_are_timed(bits):
+    """With pass timing on, apply, measure and reset record their own pass,
+    on a state that is |0...0> and on one that is not."""
+    n = 12
+    with DeviceState(n, bits) as st:
+        whole = (8 if bits == 32 else 16) * 2 << n
+        st.set_pass_timing(True)
+        st.apply_ops(library.qft(n).ops(), options(4, staged=False))
+        assert len(st.pass_times()[0]) > 1
+        for controls in ([], [(3, True)]):
+            st.apply(Gate("ry", (0.8,)).matrix(), [1], controls)
+            seconds, moved, _ = st.pass_times()
+            assert len(seconds) == 1 and seconds[0] > 0 and moved[0] == whole / (1 + len(controls))
+        st.apply_ops(library.qft(n).ops(), options(4, staged=False))
+        st.measure(2, 0.3)
+        assert len(st.pass_times()[0]) == 1
+        st.apply_ops(library.qft(n).ops(), options(4, staged=False))
+        st.reset(2, 0.3)
+        assert len(st.pass_times()[0]) == 1
+        st.zero()
+        st.apply_ops(library.qft(n).ops(), options(4, staged=False))
+        st.zero()
+        assert st.measure(5, 0.5) == 0
+        assert len(st.pass_times()[0]) == 1
