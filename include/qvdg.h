@@ -111,10 +111,12 @@ typedef struct {
 typedef struct {
   uint64_t gates;       /* ops given */
   uint64_t kernels;     /* fused ops applied */
-  uint64_t passes;      /* full passes over the state (stages + relabels, or one per fused op) */
+  uint64_t passes;      /* passes planned: stages, or one per fused op. In a run that does not time its passes,
+                         * diagonal ones may share a pass over the state: still counted singly here */
   uint64_t stages;      /* staged passes */
   double gate_seconds;  /* device time of the gate work (CUDA events) */
-  double bytes;         /* algorithmic HBM bytes of the gate work (diagonal passes that shared one counted once) */
+  double bytes;         /* algorithmic HBM bytes of the gate work: what a run moved (a shared pass once), so
+                         * not always `passes` times a pass; qvdg_plan_info's are those of its passes */
   qvdg_options settings; /* the settings the run's plan was built with (planner = GREEDY: the learned pick
                           * or the caller's own) */
 } qvdg_stats;
