@@ -50,9 +50,14 @@ constexpr size_t kRegBlobBudget = 64 * 1024;
 // How far the product of the divisors left out may go from 1 (a power of two)
 // before the state is multiplied by it: until then the amplitudes are off by
 // its inverse, and 200 gates with a divisor of 1/2 would take complex64 ones
-// past 2^128. 2^40 leaves a state that is not normalised the rest of the range;
-// unitary gates (divisors from 1/sqrt 2) reach it once in 80 of them.
-constexpr int scale_limit(int bits) { return bits == 32 ? 40 : 200; }
+// past 2^128. 2^40 (complex128: 2^200) leaves a state that is not normalised
+// the rest of the range; unitary gates (divisors from 1/sqrt 2) reach it once
+// in 80 of them.
+bool scale_far(const std::complex<long double>& scale, int bits) {
+  const long double size = scale.real() * scale.real() + scale.imag() * scale.imag();
+  const long double limit = bits == 32 ? 0x1p80L : 0x1p400L;
+  return size > limit || size * limit < 1.0L;
+}
 
 enum : uint8_t { kRegDense1 = 0, kRegDense2 = 1, kRegSign = 2, kRegPhase = 3, kRegSign2 = 4 };
 enum : uint8_t { kFormGeneral = 0, kFormReal = 1, kFormImag = 2, kFormComplex = 3, kFormX = 4 };
@@ -827,7 +832,7 @@ bool lower_register(const Target& s, const PlannedPass& p, const StageConfig& cf
         g.op = kOpPhase;
       gates.push_back(g);
       fixes.push_back(fx);
-      if (g.op < kOpX && std::abs(std::ilogb(std::abs(scale))) >= scale_limit(s.bits)) put_scale();
+      if (g.op < kOpX && scale_far(scale, s.bits)) put_scale();
       if (sign_after) {
         // Divisors of opposite sign: -1 where the target is 1.
         RegGate z{};
