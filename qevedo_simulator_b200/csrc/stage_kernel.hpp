@@ -100,6 +100,8 @@ void launch_block(StateImpl& s, const LoweredPass& lp, const DeviceUpload& dev);
 // Register-blocked CUDA-core stages (stage_reg.cu): gates unfused, four tile
 // bits per register pass.
 bool register_pass_ok(const Target& s, const PlannedPass& p);
+// Whether the pass's gate program fits a launch; one that does not is split.
+bool register_pass_fits(const Target& s, const PlannedPass& p, const StageConfig& cfg);
 LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const StageConfig& cfg, StageUpload& up);
 void launch_stage_reg(StateImpl& s, const LoweredPass& lp, const DeviceUpload& dev);
 size_t tc_smem_bytes(const TileGeom& geo);

@@ -434,6 +434,31 @@ void share_diagonal_passes(Program& prog, const std::vector<uint64_t>& touches) 
   flush();
 }
 
+// Register stages whose gate programs exceed what a launch holds, cut in two
+// until they fit (a single gate does: 16 KB at most).
+std::vector<PlannedPass> split_large_stages(const Target& t, std::vector<PlannedPass> passes, const StageConfig& cfg) {
+  if (!cfg.reg || cfg.low_bits < 1) return passes;
+  std::vector<PlannedPass> out, left;
+  for (PlannedPass& whole : passes) {
+    left.push_back(std::move(whole));
+    while (!left.empty()) {
+      PlannedPass p = std::move(left.back());
+      left.pop_back();
+      if (p.ops.size() < 2 || !register_pass_ok(t, p) || register_pass_fits(t, p, cfg)) {
+        out.push_back(std::move(p));
+        continue;
+      }
+      PlannedPass second = p;
+      const auto middle = long(p.ops.size() / 2);
+      second.ops.erase(second.ops.begin(), second.ops.begin() + middle);
+      p.ops.resize(size_t(middle));
+      left.push_back(std::move(second));
+      left.push_back(std::move(p));
+    }
+  }
+  return out;
+}
+
 }  // namespace
 
 Program build_program(const Target& t, const std::vector<HOp>& ops, const qvdg_options& opt,
@@ -452,7 +477,7 @@ Program build_program(const Target& t, const std::vector<HOp>& ops, const qvdg_o
   // Tensor-core plain passes' bf16 matrices (by pass; empty for the others).
   std::vector<PlainTcBlob> blobs;
   if (opt.staged) {
-    passes = plan_stages(ops, t.layout, t.n, prog.cfg, max_fused);
+    passes = split_large_stages(t, plan_stages(ops, t.layout, t.n, prog.cfg, max_fused), prog.cfg);
   } else {
     // One pass per fused op (src/simulator.rs:136-143). With the gates math,
     // an eligible group is applied member by member in registers instead of

@@ -885,7 +885,25 @@ LoweredPass lower_register_pass(const Target& s, const PlannedPass& p, const Sta
   throw Error(QVDG_ERR_UNSUPPORTED, "internal: register stage program too large");
 }
 
-size_t register_blob_budget() { return kRegBlobBudget; }
+bool register_pass_fits(const Target& s, const PlannedPass& p, const StageConfig& cfg) {
+  // At most: a register pass's header, the record and the matrix, or the
+  // diagonal with its controls and the index parts, of each gate.
+  const size_t elem = s.bits == 32 ? 8 : 16;
+  size_t bytes = 0;
+  for (const HOp& op : p.ops) {
+    const size_t k = op.targets.size();
+    const size_t data = op.diagonal ? (elem << (k + op.controls.size())) + 32 : elem << (2 * k);
+    bytes += sizeof(RegPassHdr) + sizeof(RegGate) + ((data + 15) & ~size_t(15));
+  }
+  if (bytes <= kRegBlobBudget) return true;
+  // Sheared or not, as lower_register_pass tries them.
+  for (const bool shear : {true, false}) {
+    LoweredPass lp;
+    StageUpload up;
+    if (lower_register(s, p, cfg, up, shear, lp)) return true;
+  }
+  return false;
+}
 
 void launch_stage_reg(StateImpl& s, const LoweredPass& lp, const DeviceUpload& dev) {
   const size_t tile_bytes = (s.bits == 32 ? 8 : 16) << lp.geo.L;

@@ -736,6 +736,30 @@ def test_register_stages_of_many_sheared_gates(oracle, bits, n, kind):
         assert max_distance(st.amplitudes(), expected) < {32: 4 * 255 * 2.0 ** -24, 64: 4 * 255 * 2.0 ** -53}[bits] * norm
 
 
+@pytest.mark.parametrize("bits", [32, 64])
+def test_stages_split_to_fit_shared_memory(oracle, bits):
+    """Stages whose gate data exceed what a launch holds, as several: the
+    default staged plan in both precisions, and the learned planner's on a
+    state of 10 qubits."""
+    from test_planner import large_stages
+
+    n = 12
+    psi = random_state(np.random.default_rng(bits), n)
+    for ops in large_stages(bits):
+        expected = oracle.naive_statevector(ops, n, initial=psi)
+        with DeviceState(n, bits) as st:
+            st.set_amplitudes(psi)
+            st.apply_ops(ops, options(4, True))
+            assert max_distance(st.amplitudes(), expected) < {32: 1e-5, 64: 1e-11}[bits]
+    small = [Op([q % 10 for q in op.targets], op.controls, op.matrix) for op in ops if len(op.targets) == 1]
+    small = [op for s in small for op in (s, Op(list(range(10)), [], random_diagonal(np.random.default_rng(1), 10)))]
+    expected = oracle.naive_statevector(small, 10, initial=psi[:1024])
+    with DeviceState(10, bits) as st:
+        st.set_amplitudes(psi[:1024])
+        st.apply_ops(small, options(planner="learned"))
+        assert max_distance(st.amplitudes(), expected) < {32: 1e-5, 64: 1e-11}[bits]
+
+
 def test_swap_passes_of_a_large_state():
     """The large tiles of a 4 GiB state whose rows scatter: every amplitude at
     its place, and back again."""

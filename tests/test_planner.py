@@ -122,3 +122,36 @@ def test_programs_from_zero_apply_every_fused_op(kind):
         fused = costmodel.fused_ops(ops, n, opts, from_zero=True)
         pairs = int(np.sum(rows[:, 21] == 1))
         assert rows.shape[0] + pairs == len(fused), (kind, opts.math, opts.max_fused_qubits)
+
+
+def large_stages(bits):
+    """Circuits of 12 qubits whose gates do not fit one register stage's
+    64 KB (256 dense 2-qubit gates: in complex128 alone): dense 2-qubit
+    gates, and diagonals on 4, 8 and 10 qubits with a gate between."""
+    from qevedo_simulator_b200 import Op
+
+    rng = np.random.Generator(np.random.PCG64(bits))
+    out = []
+    for count, k in ((256, 2), (256, -4), (64, -8), (9, -10)):
+        ops = []
+        for i in range(count):
+            qs = [int(q) for q in rng.permutation(12)[:abs(k)]]
+            if k > 0:
+                m = np.linalg.qr(rng.standard_normal((1 << k, 1 << k)) + 1j * rng.standard_normal((1 << k, 1 << k)))[0]
+            else:
+                m = np.diag(np.exp(2j * np.pi * rng.random(1 << -k)))
+                ops.append(Op([qs[0]], [], np.array([[0.6, 0.8j], [0.8j, 0.6]])))
+            ops.append(Op(qs, [], m))
+        out.append(ops)
+    return out
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+def test_stages_larger_than_their_shared_memory_are_split(bits):
+    """The default staged plan takes any number and width of gates: a stage
+    whose gate data exceed what a launch holds becomes several."""
+    for ops in large_stages(bits):
+        for n in (12, 15):
+            rows = costmodel.plan_features(ops, n, options(4, staged=True), precision_bits=bits)
+            # 12 qubits are one tile: as many stages as the gate data fill, and not many more.
+            assert rows.shape[0] <= (24 if n == 12 else len(ops))
