@@ -142,8 +142,8 @@ qvdg_status qvdg_state_create(uint32_t num_qubits, uint32_t precision_bits, qvdg
  * buffers of small states (at most 16 MB of amplitudes, 32 MB of workspace
  * and 8 MB of pinned memory each, of four states) are kept for the next
  * qvdg_state_create on the device and given back when an allocation of this
- * library would fail without them. A buffer that qvdg_state_device_buffer has
- * handed out is freed instead, once the device's work is done. */
+ * library would fail without them. If qvdg_state_device_buffer has handed the
+ * buffer out, the call waits for all work on the device. */
 qvdg_status qvdg_state_destroy(qvdg_state* state);
 
 /* Set the state to |0...0> and the identity layout. */

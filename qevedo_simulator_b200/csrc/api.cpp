@@ -49,8 +49,9 @@ namespace {
 // Making and freeing them (above all the pinned memory, one to three
 // milliseconds) cost a statevector() of a few qubits ten times its gates.
 // At most kPoolStates of them wait, each within the limits below; a failing
-// allocation of this library gives them all back first. Amplitudes whose
-// address a caller has had are not among them. The pool itself is
+// allocation of this library gives them all back first. Nothing uses them any
+// more: where a caller has had the amplitudes' address, destroying the state
+// waits for the whole device. The pool itself is
 // never destroyed: the driver frees what is left at process exit.
 struct StateResources {
   int device = 0;
@@ -457,19 +458,15 @@ qvdg_status qvdg_state_create(uint32_t num_qubits, uint32_t precision_bits, qvdg
 qvdg_status qvdg_state_destroy(qvdg_state* st) {
   if (!st) return QVDG_OK;
   StateImpl& s = st->s;
-  const bool idle = s.stream && cudaStreamSynchronize(s.stream) == cudaSuccess;
+  bool idle = s.stream && cudaStreamSynchronize(s.stream) == cudaSuccess;
   for (cudaEvent_t e : s.pass_events) cudaEventDestroy(e);
   if (s.amp_given) {
-    // A caller's kernels may still use the amplitudes on streams of its own:
-    // they are waited for, and the buffer goes to no other state.
+    // A caller's kernels may still use the amplitudes on streams of its own.
     int current = s.device;
     cudaGetDevice(&current);
     if (current != s.device) cudaSetDevice(s.device);
-    cudaDeviceSynchronize();
+    idle = cudaDeviceSynchronize() == cudaSuccess && idle;
     if (current != s.device) cudaSetDevice(current);
-    cudaFree(s.amp);
-    s.amp = nullptr;
-    s.amp_capacity = 0;
   }
   StateResources r;
   r.device = s.device;
