@@ -140,11 +140,15 @@ qvdg_status qvdg_state_create(uint32_t num_qubits, uint32_t precision_bits, qvdg
 /* Free the state and its device memory (reference: Drop of Buffer,
  * src/memory.rs:91-96). NULL is accepted. The stream, events, workspaces and
  * buffers of small states (at most 16 MB of amplitudes, 32 MB of workspace
- * and 8 MB of pinned memory each, of four states) are kept for the next
- * qvdg_state_create on the device and given back when an allocation of this
- * library would fail without them. If qvdg_state_device_buffer has handed the
+ * and 12 MB of pinned memory each, of four states) are kept for the next
+ * qvdg_state_create on the device and given back by qvdg_release_cached, or
+ * when an allocation of this library would fail without them. If qvdg_state_device_buffer has handed the
  * buffer out, the call waits for all work on the device. */
 qvdg_status qvdg_state_destroy(qvdg_state* state);
+
+/* Free what destroyed states have left, on every device (another allocator of
+ * the process may need it). No counterpart in the reference. */
+qvdg_status qvdg_release_cached(void);
 
 /* Set the state to |0...0> and the identity layout. */
 qvdg_status qvdg_state_zero(qvdg_state* state);

@@ -27,6 +27,7 @@ _SIGNATURES = {
     "qvdg_version": (ct.c_char_p, []),
     "qvdg_state_create": (ct.c_int, [ct.c_uint32, ct.c_uint32, ct.POINTER(_P)]),
     "qvdg_state_destroy": (ct.c_int, [_P]),
+    "qvdg_release_cached": (ct.c_int, []),
     "qvdg_state_zero": (ct.c_int, [_P]),
     "qvdg_state_info": (ct.c_int, [_P, ct.POINTER(ct.c_uint32), ct.POINTER(ct.c_uint32)]),
     "qvdg_state_set_amplitudes": (ct.c_int, [_P, ct.POINTER(ct.c_double), ct.c_size_t]),
@@ -147,6 +148,12 @@ def bit_probabilities_noalloc(pointer: int, num_qubits: int, precision_bits: int
     check(lib().qvdg_bit_probabilities_noalloc(ct.c_void_p(pointer), int(num_qubits), int(precision_bits),
                                                ct.c_void_p(stream), as_double_ptr(p1), ct.byref(total)))
     return p1[:num_qubits], total.value
+
+
+def release_cached():
+    """Free the device and pinned memory that closed states have left for the
+    next ones (at most four sets of 48 MB and 12 MB)."""
+    check(lib().qvdg_release_cached())
 
 
 def set_device(device: int):

@@ -48,8 +48,9 @@ namespace {
 // word, workspaces, pinned staging and, where they are small, amplitudes.
 // Making and freeing them (above all the pinned memory, one to three
 // milliseconds) cost a statevector() of a few qubits ten times its gates.
-// At most kPoolStates of them wait, each within the limits below; a failing
-// allocation of this library gives them all back first. Nothing uses them any
+// At most kPoolStates of them wait, each within the limits below and with 4 MB
+// of staging chunks; a failing allocation of this library gives them all back
+// first, and qvdg_release_cached does. Nothing uses them any
 // more: where a caller has had the amplitudes' address, destroying the state
 // waits for the whole device. The pool itself is
 // never destroyed: the driver frees what is left at process exit.
@@ -488,6 +489,10 @@ qvdg_status qvdg_state_destroy(qvdg_state* st) {
     free_resources(r);
   delete st;
   return QVDG_OK;
+}
+
+qvdg_status qvdg_release_cached(void) {
+  return guarded([&] { drain_resources(); });
 }
 
 qvdg_status qvdg_state_zero(qvdg_state* st) {

@@ -108,6 +108,7 @@ extern "C" {
     // State vectors (src/state.rs, src/measure.rs).
     pub fn qvdg_state_create(num_qubits: u32, precision_bits: u32, out: *mut *mut qvdg_state) -> qvdg_status;
     pub fn qvdg_state_destroy(state: *mut qvdg_state) -> qvdg_status;
+    pub fn qvdg_release_cached() -> qvdg_status;
     pub fn qvdg_state_zero(state: *mut qvdg_state) -> qvdg_status;
     pub fn qvdg_state_info(state: *const qvdg_state, num_qubits: *mut u32, precision_bits: *mut u32)
         -> qvdg_status;

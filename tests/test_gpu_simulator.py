@@ -401,6 +401,39 @@ def test_states_reuse_what_earlier_ones_left(threads):
     assert before - free_bytes() <= 4 * (16 + 16 + 16 + 2) << 20
 
 
+def test_release_cached_gives_back_what_states_left():
+    """Four states' buffers and workspaces stay on the device when they are
+    closed, until release_cached; new states work after it."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from cuda.bindings import runtime as rt
+
+    from qevedo_simulator_b200 import release_cached
+
+    def free_bytes():
+        return rt.cudaMemGetInfo()[1]
+
+    with DeviceState(3, 32) as st:
+        st.apply(Gate("h").matrix(), [0])
+    release_cached()
+    before = free_bytes()
+    states = [DeviceState(20, 64) for _ in range(4)]  # 16 MB each
+    for st in states:
+        st.apply(Gate("h").matrix(), [0])
+        st.close()
+    assert before - free_bytes() >= 4 << 24
+    release_cached()
+    assert before - free_bytes() < 4 << 20
+    with ThreadPoolExecutor(4) as pool:
+        def work(i):
+            with DeviceState(12, 32) as st:
+                st.apply(Gate("x").matrix(), [i])
+                release_cached()
+                return st.probability_one(i)
+
+        assert list(pool.map(work, range(8))) == [1.0] * 8
+
+
 @pytest.mark.parametrize("pinned", [False, True])
 @pytest.mark.parametrize("n", [16, 17, 18, 20, 23])
 def test_large_copies_through_staging_chunks(n, pinned):
