@@ -789,18 +789,49 @@ def test_swap_passes_of_a_large_state():
     st.close()
 
 
-def test_gates_on_grids_of_many_blocks(oracle):
-    """One gate of each plain kernel on a state that gives every SM more than
-    128 blocks, one after another."""
-    n = 25
+@pytest.mark.parametrize("bits", [32, 64])
+def test_gates_on_grids_of_many_blocks(bits):
+    """One gate of each plain kernel up to three qubits on a state that gives
+    every SM more than 128 blocks of it, one after another, against torch in
+    complex128."""
+    import torch
+
+    n = 27
     rng = np.random.default_rng(n)
-    psi = random_state(rng, n)
     d = lambda k: np.diag(np.exp(1j * rng.uniform(0, 2 * np.pi, 1 << k)))
     ops = [Op([17], [], random_unitary(rng, 1)), Op([9], [(0, True)], random_unitary(rng, 1)),
-           Op([3], [], random_unitary(rng, 1)), Op([4, 1], [], random_unitary(rng, 2)), Op([20, 2], [], d(2)),
+           Op([22, 6], [], random_unitary(rng, 2)), Op([5, 26, 13], [], random_unitary(rng, 3)),
+           Op([0, 24, 3], [], random_unitary(rng, 3)), Op([3], [], random_unitary(rng, 1)),
+           Op([4, 1], [], random_unitary(rng, 2)), Op([2, 4, 0], [], random_unitary(rng, 3)), Op([20, 2], [], d(2)),
            Op([11], [(0, False)], d(1))]
-    with DeviceState(n, 32) as st:
-        st.set_amplitudes(psi)
+    with DeviceState(n, bits) as st:
+        pointer, _ = st.device_buffer()
+
+        class Buffer:
+            __cuda_array_interface__ = {"shape": (1 << n,), "data": (pointer, False), "version": 3,
+                                        "typestr": "<c8" if bits == 32 else "<c16"}
+
+        view = torch.as_tensor(Buffer(), device="cuda")
+        gen = torch.Generator(device="cuda").manual_seed(n)
+        parts = torch.view_as_real(view)
+        parts.copy_(torch.rand(parts.shape, generator=gen, dtype=parts.dtype, device="cuda") - 0.5)
+        expected = view.clone().to(torch.complex128)
+        index = torch.arange(1 << n, device="cuda")
+        torch.cuda.synchronize()
         for op in ops:
             st.apply(op.matrix, op.targets, op.controls)
-        assert max_distance(st.amplitudes(), oracle.naive_statevector(ops, n, initial=psi)) < TOL[32]
+            k = len(op.targets)
+            row = sum(((index >> t) & 1) << j for j, t in enumerate(op.targets))
+            rest = index & ~sum(1 << t for t in op.targets)
+            m = torch.from_numpy(op.matrix).to("cuda")
+            out = torch.zeros_like(expected)
+            for c in range(1 << k):
+                out += m[row, c] * expected[rest | sum(((c >> j) & 1) << t for j, t in enumerate(op.targets))]
+            on = torch.ones_like(index, dtype=torch.bool)
+            for q, v in op.controls:
+                on &= ((index >> q) & 1) == int(v)
+            expected = torch.where(on, out, expected)
+        # A gate on k qubits rounds an amplitude by some 2^k + 2 units of its
+        # group's norm; the ten gates here by 130 units of the largest together.
+        error = (view.to(torch.complex128) - expected).abs().max() / expected.abs().max()
+        assert float(error) < 130 * {32: 2.0 ** -24, 64: 2.0 ** -53}[bits]

@@ -438,9 +438,12 @@ def test_release_cached_gives_back_what_states_left():
 @pytest.mark.parametrize("n", [16, 17, 18, 20, 23])
 def test_large_copies_through_staging_chunks(n, pinned):
     """Amplitudes and probabilities in and out below, at and over the sizes
-    where copies go through two pinned chunks, from ordinary and from pinned
+    where copies go through two pinned chunks, from and to ordinary and pinned
     arrays, also right after one another."""
     import torch
+
+    from qevedo_simulator_b200._abi import as_double_ptr
+    from qevedo_simulator_b200._native import check, lib
 
     rng = np.random.default_rng(n)
     psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
@@ -450,6 +453,10 @@ def test_large_copies_through_staging_chunks(n, pinned):
         for _ in range(2):
             st.set_amplitudes(psi)
             assert np.array_equal(st.amplitudes(), psi)
+            if pinned:
+                out = torch.zeros(1 << n, dtype=torch.complex128).pin_memory().numpy()
+                check(lib().qvdg_state_get_amplitudes(st._h, as_double_ptr(out.view(np.float64)), out.size))
+                assert np.array_equal(out, psi)
             psi[:] = psi[::-1].copy()
         st.set_amplitudes(psi)
         p = st.probabilities()
@@ -470,7 +477,24 @@ def test_outcomes_through_staging_chunks(oracle, shots):
 
 
 @pytest.mark.parametrize("bits", [32, 64])
-@pytest.mark.parametrize("n", [1, 2, 3, 9, 10, 11, 13, 16, 17, 21])
+def test_sampling_more_chunks_than_a_batch_of_checkpoints(bits):
+    """A million shots that land in every chunk of 30 qubits, twice what the
+    checkpoints of one batch cover. Equal amplitudes of 2^-15: every sum is
+    exact, and outcome i is the one whose [i, i + 1) 2^-30 holds the uniform."""
+    import torch
+
+    n = 30
+    rng = np.random.default_rng(bits)
+    u = np.concatenate([rng.random(1_000_000), np.arange(0, 1, 2.0 ** -15), [np.nextafter(1.0, 0.0)]])
+    with DeviceState(n, bits) as st:
+        device_view(st).fill_(2.0 ** -15)
+        torch.cuda.synchronize()
+        got = st.sample_unordered(u)
+    assert np.array_equal(np.sort(got), np.sort(np.floor(u * 2.0 ** n).astype(np.uint64)))
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("n", [1, 2, 3, 9, 10, 11, 13, 16, 17, 21, 22])
 def test_reductions_on_one_and_many_blocks(bits, n):
     """Norm, P(1) of every bit alone and together, and Pauli strings with X/Y
     inside and beyond a 16-byte vector, twice in a row, on states of less than
